@@ -80,7 +80,7 @@ def draw(rng):
     kind = rng.choice(["evaluate", "steps", "steps", "steps", "host_step", "batch", "serve"])
     precision = rng.choice(["fp64", "mixed"])
     if kind == "batch":
-        return dict(kind=kind, members=rng.randint(4, 24), kmin=8, kmax=rng.randint(10, 32),
+        return dict(kind=kind, members=rng.randint(4, 14), kmin=8, kmax=rng.randint(10, 32),
                     sizes=rng.randrange(1 << 20), steps=rng.randint(2, 5), precision=precision)
     if kind == "serve":
         return dict(kind=kind, members=rng.randint(3, 8), nmin=8192, nmax=int(size(16384, 131072)),
