@@ -294,8 +294,10 @@ int sphgpu_pairs_evaluated(sphgpu_problem* p, int64_t* pairs);
 int sphgpu_kernel_launches(sphgpu_problem* p, int64_t* launches);
 /* Kernel schedules (no counterpart in the reference, whose loops are serial).
  * stage "neighbor walk": 0 = automatic (thread per node while the 27-cell
- * candidate set is small, warp per node otherwise), 1 = thread per node,
- * 2 = warp per node.  Every schedule yields the same ConnectivityMap.
+ * candidate set is small, 2 otherwise), 1 = thread per node, 2 = for large
+ * candidate sets: a block per cell that shares its candidates (cells of one
+ * kernel reach), a warp per node (half a reach).  Every schedule yields the
+ * same ConnectivityMap.
  * stage "pair loop": threads per block of the derivative kernels, 64 or 128.
  * stage "neighbor filter": 1 (default) = an FP32 pre-test decides the pairs
  * clearly inside or outside the kernel support and the exact FP64 test the

@@ -25,10 +25,14 @@
 //                                            order) over the 27 neighbouring
 //                                            cells; 64-byte candidate records
 //                                            shared by a warp through L1
-//   nbr_walk<COUNT|FILL>                     warp per node, for large
-//                                            candidate sets
+//   nbr_cell<COUNT|FILL>                     block per cell, for large
+//                                            candidate sets: the window
+//                                            staged and ordered once per cell
+//   nbr_walk<COUNT|FILL>                     warp per node over cells of half
+//                                            a reach, for large sets
 #include <cstdio>
 #include <cstring>
+#include <cfloat>
 #include <climits>
 
 #include "problem.cuh"
@@ -41,6 +45,7 @@ constexpr int kGhostThreads = 256;
 // blocks per member of the streaming passes (member-local grid stride)
 constexpr int64_t kStreamBlocks = 148*4;
 constexpr float kFilterTol = 1.0e-3f;
+constexpr double kFilterTolPerSpread = 2.0e-5;
 // shared memory for the per-thread lists of a 32-thread block (larger lists
 // take the warp schedule)
 constexpr size_t kMaxListSmem = 200*1024;
@@ -587,8 +592,14 @@ __global__ void grid_kernel(const Member* mem, int nmem) {
   s[3] = cell;
   for (int a = 0; a < 3; ++a) setScalI(M.scal, SC_GRID + 4 + a, dim[a]);
   // largest h over smallest h of the problem (>= every node's condition number)
-  const double spread = hmaxAll*M.scal[SC_LMAXALL];
-  s[7] = (M.grid.filterTol > 0.0f && spread > 0.0 && spread <= 100.0) ? (double)M.grid.filterTol : 0.0;
+  // and the cells' edge over the kernel reach where the capacity enlarged them:
+  // the FP32 pre-test's relative error is below 2e-6 times their product (the
+  // offsets are rounded at the size of a cell).  The band is ten times that,
+  // 1e-3 at most, and the pre-test is off beyond a product of 100.
+  const double natural = M.prm.kernelExtent*hmaxAll*1.001/sub;
+  const double spread = hmaxAll*M.scal[SC_LMAXALL]*fmax(1.0, cell/natural);
+  s[7] = (M.grid.filterTol > 0.0f && spread > 0.0 && spread <= 100.0)
+             ? fmin((double)M.grid.filterTol, kFilterTolPerSpread*fmax(spread, 1.0)) : 0.0;
   // the largest kernel reach in cells (<= sub), for the walks' pruning
   M.scal[SC_REACH] = M.prm.kernelExtent*hmaxAll/cell;
   setScalI(M.scal, SC_NCELLS, ncells);
@@ -753,8 +764,8 @@ __device__ __forceinline__ bool exactTest(const Member& M, int32_t i, int32_t j,
 // With tol > 0 a FP32 pre-test decides every pair whose eta^2 lies clearly
 // outside the band kappa^2 (1 -+ tol): eta_i^2 from the FP32 H_i, eta_j^2
 // bounded by min/max eig(H_j)^2 |r_ij|^2, r_ij from the cell offsets.  The
-// pre-test error is below 1e-6 (max h/min h over the problem) relative, and
-// tol (1e-3) is only set when that ratio is <= 100, so it never decides a
+// pre-test error is below 2e-6 (max h/min h over the problem) relative, and
+// tol is ten times that (grid_kernel), so it never decides a
 // pair the exact test would decide otherwise.  Undecided pairs take the
 // exact FP64 test in the reference's operation order.  eta^2 of either node
 // lies in [min eig(H)^2 r^2, max eig(H)^2 r^2]: a candidate beyond the band
@@ -959,29 +970,27 @@ __global__ void __launch_bounds__(256) nbr_compact_warp_kernel(const Member* mem
   for (int t = lane; t < count; t += 32) M.nbr[o + t] = stash[t];
 }
 
-// Warp per internal node (warps dealt over the sorted slots, ghost slots
-// idle): walk the 27 neighbouring cells, apply the ConnectivityMap
-// predicate, count (FILL=false) or collect, sort ascending and store
-// (FILL=true) the neighbor indices.  Used when the candidate sets are large
-// (many nodes per cell), where a warp per node keeps the SMs full.  `cap` is
-// the per-warp list capacity (a power of two >= 32).  A member with a stash
-// (Grid::stashCap > 0) collects and sorts in the COUNT pass and stores the
-// list of node i at stash[i*stashCap]; nbr_compact_warp_kernel moves it to
-// offsets[i].
+// One warp walks the neighbouring cells of the node in sorted slot s (nothing
+// for a ghost slot): apply the ConnectivityMap predicate, count (FILL=false)
+// or collect, sort ascending and store (FILL=true) the neighbor indices.
+// `cap` is the capacity of the warp's list sbuf (a power of two >= 32), R its
+// row table.  A member with a stash (Grid::stashCap > 0) collects and sorts
+// in the COUNT pass and stores the list of node i at stash[i*stashCap];
+// nbr_compact_warp_kernel moves it to offsets[i].
+template<int SUB>
+struct RowTable {
+  static constexpr int NR = (2*SUB + 1)*(2*SUB + 1);
+  static constexpr int RW = 3 + 2*SUB;                // start, first candidate number, x0, cell ends
+  int32_t v[NR*RW];
+};
+
 template<bool FILL, int SUB>
-__global__ void __launch_bounds__(256, SUB == 1 ? 3 : 1) nbr_walk_kernel(const Member* mem, BlockMap bm, int cap, int maxNbr) {
-  extern __shared__ int32_t sbuf_all[];
-  const MemberBlock mb = memberBlock(bm);
-  const Member& M = mem[mb.m];
+__device__ __noinline__ void walkWarp(const Member& M, const Grid& g, int64_t s, int32_t* sbuf, int cap, int maxNbr,
+                                      int32_t* R) {
   const int lane = threadIdx.x & 31;
-  const int wib = threadIdx.x >> 5;
   const int scap = FILL ? 0 : M.grid.stashCap;
   const bool collect = FILL || scap > 0;
-  int32_t* sbuf = sbuf_all + (collect ? wib*cap : 0);
-  const int64_t s = (mb.block*(int64_t)blockDim.x + threadIdx.x) >> 5;
-  if (s >= allNodes(M)) return;
   const NbrArrays a = nbrArrays(M);
-  const Grid g = loadGrid(M);
   const Walker me = makeWalker(M, a, g, (int32_t)s);
   if (me.idx >= M.n) return;
   const int32_t i = me.idx;
@@ -997,10 +1006,7 @@ __global__ void __launch_bounds__(256, SUB == 1 ? 3 : 1) nbr_walk_kernel(const M
   // sequence by a warp scan: the lanes then take 32 consecutive candidates at
   // a time across row ends, so a warp iteration tests 32 candidates however
   // short the rows are.
-  constexpr int NR = (2*SUB + 1)*(2*SUB + 1);
-  constexpr int RW = 3 + 2*SUB;                       // start, first candidate number, x0, cell ends
-  __shared__ int32_t rowTab[256/32][NR*RW];
-  int32_t* R = rowTab[wib];
+  constexpr int NR = RowTable<SUB>::NR, RW = RowTable<SUB>::RW;
   int len = 0;
   if (lane < NR) {
     const int dy = lane % (2*SUB + 1) - SUB, dz = lane/(2*SUB + 1) - SUB;
@@ -1097,6 +1103,415 @@ __global__ void __launch_bounds__(256, SUB == 1 ? 3 : 1) nbr_walk_kernel(const M
   for (int sh = 16; sh > 0; sh >>= 1) above += __shfl_xor_sync(0xffffffffu, above, sh);
   if (lane == 0 && above)
     atomicAdd(reinterpret_cast<unsigned long long*>(M.scal + SC_PAIRS), (unsigned long long)above);
+}
+
+// A warp per sorted slot (walkWarp), cells of half a kernel reach.
+template<bool FILL>
+__global__ void __launch_bounds__(256) nbr_walk_kernel(const Member* mem, BlockMap bm, int cap, int maxNbr) {
+  extern __shared__ int32_t sbuf_all[];
+  __shared__ RowTable<2> rows[256/32];
+  const MemberBlock mb = memberBlock(bm);
+  const Member& M = mem[mb.m];
+  const int wib = threadIdx.x >> 5;
+  const bool collect = FILL || M.grid.stashCap > 0;
+  const int64_t s = (mb.block*(int64_t)blockDim.x + threadIdx.x) >> 5;
+  if (s >= allNodes(M)) return;
+  walkWarp<FILL, 2>(M, loadGrid(M), s, sbuf_all + (collect ? wib*cap : 0), cap, maxNbr, rows[wib].v);
+}
+
+// ---------------------------------------------------------------- cell walk
+// A block per cell of one kernel reach: the candidates of the 27
+// neighbouring cells are staged in shared memory once for all walkers of the
+// cell, in node order, and each warp then tests them for four walkers at a
+// time and appends the ones that pass with a ballot, so every list comes out
+// ascending without a sort of its own.
+//
+// Why this split: a walker of the Sod tube (27 nodes per cell) has 743
+// candidates for 115 neighbors.  With a warp per walker each of the 27
+// walkers of a cell gathered the same candidates from L1/L2 and sorted its
+// own list.  Here the gather and the ordering are shared by the cell, the
+// candidates farther from the cell than the kernel reach are left out first
+// (743 -> 570), and a test is a 16-byte shared-memory read and about twenty
+// instructions for 32 candidates.  The cells' slots are brought into node
+// order once (cell_order_kernel), so that a block only merges 27 sorted runs:
+// along x, then y, then z, each element finding its rank by bisection in the
+// two other runs.
+//
+// Measured (B200): Sod 256x32x32 (262,144 nodes, 115 neighbors) 786 us against
+// 1,939 us with a warp per node; 24 tubes of the ensemble together 3.17 against
+// 8.92 ms.  Bound by instruction issue (about half of the cycles issue, 32
+// warps per SM): a fifth of the instructions are the merges, the rest the
+// tests and the lists' stores.
+constexpr int kCellThreads = 256;
+constexpr int kCellWarps = kCellThreads/32;
+constexpr int kCellCand = 1536;                        // nodes of the 27 cells that can be staged (more: walkWarp)
+constexpr int kCellTest = 1024;                        // of them within the reach of the cell: a ballot word per lane
+constexpr int kCellSort = 128;                         // nodes of a cell kept in node order (more: walkWarp)
+constexpr int kWalkers = 4;                            // walkers a warp tests at a time
+constexpr int64_t kCellBlocks = 148*16;                // blocks of a member, at most
+
+// The slots of one cell into node order (a warp per cell, 32*E >= its nodes).
+template<int E>
+__device__ __forceinline__ void orderCell(const Member& M, int32_t s0, int count) {
+  double* base = static_cast<double*>(M.cand);
+  float4* pre = reinterpret_cast<float4*>(base);
+  float* lmax = reinterpret_cast<float*>(base + 2*M.candcap);
+  const int lane = threadIdx.x & 31;
+  int32_t key[E];
+  float4 p[E];
+  float lm[E];
+  int rank[E];
+#pragma unroll
+  for (int e = 0; e < E; ++e) {
+    const int t = 32*e + lane;
+    key[e] = t < count ? M.sortedIdx[s0 + t] : INT_MAX;
+    if (t < count) { p[e] = pre[s0 + t]; lm[e] = lmax[s0 + t]; }
+    rank[e] = 0;
+  }
+  for (int l = 0; l < 32; ++l) {
+#pragma unroll
+    for (int f = 0; f < E; ++f) {
+      const int32_t o = __shfl_sync(0xffffffffu, key[f], l);
+#pragma unroll
+      for (int e = 0; e < E; ++e) rank[e] += o < key[e];
+    }
+  }
+  __syncwarp();
+#pragma unroll
+  for (int e = 0; e < E; ++e) {
+    if (32*e + lane >= count) continue;
+    M.sortedIdx[s0 + rank[e]] = key[e];
+    pre[s0 + rank[e]] = p[e];
+    lmax[s0 + rank[e]] = lm[e];
+  }
+}
+
+__global__ void __launch_bounds__(256) cell_order_kernel(const Member* mem, BlockMap bm) {
+  const MemberBlock mb = memberBlock(bm);
+  const Member& M = mem[mb.m];
+  const int64_t ncells = scalI(M.scal, SC_NCELLS);
+  const int64_t stride = (int64_t)mb.blocks*(blockDim.x >> 5);
+  for (int64_t c = mb.block*(blockDim.x >> 5) + (threadIdx.x >> 5); c < ncells; c += stride) {
+    const int32_t s0 = (int32_t)M.cellStart[c];
+    const int count = (int)M.cellStart[c + 1] - s0;
+    if (count < 2 || count > kCellSort) continue;
+    if (count <= 32) orderCell<1>(M, s0, count);
+    else if (count <= 64) orderCell<2>(M, s0, count);
+    else orderCell<kCellSort/32>(M, s0, count);
+  }
+}
+
+// Elements of the ascending run key[0 : len) below k.
+__device__ __forceinline__ int runRank(const int32_t* key, int len, int32_t k) {
+  int lo = 0;
+  if (len <= 0) return 0;
+  while (len > 1) {
+    const int half = len >> 1;
+    if (key[lo + half - 1] < k) lo += half;
+    len -= half;
+  }
+  return lo + (key[lo] < k);
+}
+
+// Merge of the ascending runs 3g, 3g + 1, 3g + 2 (run r at [start[r],
+// start[r + 1])) of every g from (key, src) to (keyTo, srcTo), each element at
+// the rank it has among the three.  A warp takes 32 elements of one run at a
+// time, so that the bisections' lengths are the same for its lanes.
+// own (the last merge): the final place of the element staged at ownAt + m
+// goes to own[m], m < ownLen.
+__device__ __forceinline__ void mergeRuns(const int32_t* key, const uint16_t* src, int32_t* keyTo, uint16_t* srcTo,
+                                          const int* start, int runs, uint16_t* own = nullptr, int ownAt = 0,
+                                          int ownLen = 0) {
+  const int lane = threadIdx.x & 31, wib = threadIdx.x >> 5;
+  int task = 0;
+  for (int r = 0; r < runs; ++r) {
+    const int at = start[r], len = start[r + 1] - at, g = r - r % 3;
+    const int o1 = r == g ? g + 1 : g, o2 = r == g + 2 ? g + 1 : g + 2;
+    for (int base = 0; base < len; base += 32, ++task) {
+      if (task % kCellWarps != wib || base + lane >= len) continue;
+      const int32_t k = key[at + base + lane];
+      const int to = start[g] + base + lane + runRank(key + start[o1], start[o1 + 1] - start[o1], k) +
+                     runRank(key + start[o2], start[o2 + 1] - start[o2], k);
+      const uint16_t from = src[at + base + lane];
+      keyTo[to] = k;
+      srcTo[to] = from;
+      if (own != nullptr && (unsigned)(from - ownAt) < (unsigned)ownLen) own[from - ownAt] = (uint16_t)to;
+    }
+  }
+}
+
+// The walker's side of the test.
+struct CellWalker {
+  float x, y, z;
+  float T;             // r^2 above both nodes' T: not neighbors
+  float A;             // r^2 at most either node's A: neighbors
+  int32_t idx;
+};
+
+// A pair between the bounds: the FP32 form of H_i, then the exact test.
+__device__ __noinline__ bool cellUndecided(const Member& M, int32_t i, int32_t j, float fx, float fy, float fz,
+                                           float cT, double k2, float k2lo, float k2hi, bool pretest) {
+  if (pretest) {
+    const Sym H = nodeH(M, i);
+    const float hf[6] = {(float)H.xx, (float)H.xy, (float)H.xz, (float)H.yy, (float)H.yz, (float)H.zz};
+    const float r2 = __fmaf_rn(fx, fx, __fmaf_rn(fy, fy, fz*fz));
+    const float e2i = symEta2F(hf, fx, fy, fz);
+    if (e2i <= k2lo) return true;
+    if (e2i > k2hi && r2 > cT) return false;
+  }
+  return exactTest(M, i, j, k2);
+}
+
+struct CellShared {
+  float4 pre[kCellCand];            // offsets from the cell's corner, T
+  float acc[kCellCand];             // A
+  int32_t key[2][kCellCand];        // node index
+  uint16_t src[2][kCellCand];       // position in pre before the merges
+  uint16_t own[kCellSort];          // place of the cell's own nodes after the merges
+};
+
+template<bool FILL>
+__global__ void __launch_bounds__(kCellThreads, 4) nbr_cell_kernel(const Member* mem, BlockMap bm, int cap, int maxNbr) {
+  extern __shared__ float4 cellSmem[];
+  CellShared& sh = *reinterpret_cast<CellShared*>(cellSmem);
+  __shared__ int32_t cellS0[27];
+  __shared__ int cellLen[27], cellAt[28];       // staged nodes of each cell, their first position
+  __shared__ int rowAt[10], planeAt[4];
+  __shared__ int crowded;
+  const MemberBlock mb = memberBlock(bm);
+  const Member& M = mem[mb.m];
+  const int tid = threadIdx.x, lane = tid & 31, wib = tid >> 5;
+  const int64_t n = M.n;
+  const NbrArrays a = nbrArrays(M);
+  const int ncells = (int)scalI(M.scal, SC_NCELLS);   // at most 2^26 (grid_kernel)
+  const int scap = FILL ? 0 : M.grid.stashCap;
+  const double k2 = M.prm.kernelExtent*M.prm.kernelExtent;
+  const float filterTol = (float)M.scal[SC_GRID + 7];
+  const float k2f = (float)k2;
+  const bool pretest = filterTol > 0.0f;
+  const float k2lo = k2f*(1.0f - filterTol), k2hi = k2f*(1.0f + filterTol);
+  const float cellf = (float)M.scal[SC_GRID + 3];
+  const int dim0 = (int)scalI(M.scal, SC_GRID + 4), dim1 = (int)scalI(M.scal, SC_GRID + 5),
+            dim2 = (int)scalI(M.scal, SC_GRID + 6);
+  // no candidate farther than the largest kernel reach can pass (the margin
+  // covers the FP32 offsets)
+  const float reach = (float)M.scal[SC_REACH]*cellf;
+  const float reach2 = reach*reach*1.0001f;
+  int most = 0;
+  unsigned above = 0;
+  for (int c = (int)mb.block; c < ncells; c += mb.blocks) {
+    const int32_t s0 = (int32_t)M.cellStart[c], s1 = (int32_t)M.cellStart[c + 1];
+    // (also the barrier between the last cell's tests and this one's staging)
+    bool any = false, outside = false;
+    for (int32_t s = s0 + tid; s < s1; s += kCellThreads) {
+      if (M.sortedIdx[s] >= n) continue;
+      any = true;
+      // a node clamped into the grid's outermost cells may lie outside its cell
+      const float4 p = a.pre[s];
+      const float lo = -1.0e-5f*cellf, hi = 1.00001f*cellf;
+      outside = outside || fminf(p.x, fminf(p.y, p.z)) < lo || fmaxf(p.x, fmaxf(p.y, p.z)) > hi;
+    }
+    if (!__syncthreads_or(any)) continue;
+    if (tid == 0) crowded = 0;
+    const float rc2 = __syncthreads_or(outside) ? FLT_MAX : reach2;
+    const int cyz = c/dim0, cx = c - cyz*dim0, cz = cyz/dim1, cy = cyz - cz*dim1;
+    if (wib == 0) {
+      // the 27 cells, x fastest: first slot and nodes, and an upper bound of each run's position
+      int len = 0;
+      if (lane < 27) {
+        const int x = cx + lane % 3 - 1, y = cy + (lane/3) % 3 - 1, z = cz + lane/9 - 1;
+        int32_t first = 0;
+        if (x >= 0 && x < dim0 && y >= 0 && y < dim1 && z >= 0 && z < dim2) {
+          const int64_t* cs = M.cellStart + ((int64_t)z*dim1 + y)*dim0 + x;
+          first = (int32_t)cs[0];
+          len = (int)cs[1] - first;
+        }
+        cellS0[lane] = first;
+        cellLen[lane] = len;
+        if (len > kCellSort) crowded = 1;
+      }
+      int incl = len;
+#pragma unroll
+      for (int o = 1; o < 32; o <<= 1) {
+        const int v = __shfl_up_sync(0xffffffffu, incl, o);
+        if (lane >= o) incl += v;
+      }
+      if (lane < 28) cellAt[lane] = incl - len;
+      if (lane == 31 && incl > kCellCand) crowded = 1;
+    }
+    __syncthreads();
+    // too many to stage or to merge: a warp per walker, its list sorted by itself
+    auto walkAlone = [&]() {
+      int32_t* rows = reinterpret_cast<int32_t*>(cellSmem) + wib*(cap + RowTable<1>::NR*RowTable<1>::RW);
+      const Grid g = loadGrid(M);
+      for (int32_t s = s0 + wib; s < s1; s += kCellWarps) {
+        walkWarp<FILL, 1>(M, g, s, rows + RowTable<1>::NR*RowTable<1>::RW, cap, maxNbr, rows);
+        __syncwarp();
+      }
+    };
+    if (crowded) { walkAlone(); continue; }
+    // stage the cells, a warp each: offsets from this cell's corner; the
+    // nodes beyond the reach of this cell's box left out
+    for (int q = wib; q < 27; q += kCellWarps) {
+      const int len = cellLen[q], at = cellAt[q];
+      const int32_t first = cellS0[q];
+      const float ox = (float)(q % 3 - 1)*cellf, oy = (float)((q/3) % 3 - 1)*cellf, oz = (float)(q/9 - 1)*cellf;
+      int kept = 0;
+      for (int base = 0; base < len; base += 32) {
+        const int t = base + lane;
+        bool keep = false;
+        float4 p = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+        if (t < len) {
+          p = a.pre[first + t];
+          p.x += ox; p.y += oy; p.z += oz;
+          const float gx = fmaxf(fmaxf(-p.x, p.x - cellf), 0.0f), gy = fmaxf(fmaxf(-p.y, p.y - cellf), 0.0f),
+                      gz = fmaxf(fmaxf(-p.z, p.z - cellf), 0.0f);
+          keep = q == 13 || gx*gx + gy*gy + gz*gz <= rc2;   // (the own nodes' places follow their slots)
+        }
+        const unsigned bal = __ballot_sync(0xffffffffu, keep);
+        if (keep) {
+          const int pos = at + kept + __popc(bal & ((1u << lane) - 1u));
+          const float lm = a.lmax[first + t];
+          sh.pre[pos] = p;
+          sh.acc[pos] = pretest ? __fdividef(k2lo, lm*lm) : -1.0f;
+          sh.key[0][pos] = M.sortedIdx[first + t];
+        }
+        kept += __popc(bal);
+      }
+      if (lane == 0) cellLen[q] = kept;
+    }
+    __syncthreads();
+    // rows: three cells along x each, closed up
+    if (tid < 10) {
+      int at = 0;
+      for (int q = 0; q < 3*tid; ++q) at += cellLen[q];
+      rowAt[tid] = at;
+      if (tid % 3 == 0) planeAt[tid/3] = at;
+    }
+    __syncthreads();
+    const int count = rowAt[9];
+    if (count > kCellTest) { walkAlone(); continue; }
+    for (int q = wib; q < 27; q += kCellWarps) {
+      const int len = cellLen[q], at = cellAt[q], r = q/3, o1 = 3*r + (q + 1) % 3, o2 = 3*r + (q + 2) % 3;
+      for (int t = lane; t < len; t += 32) {
+        const int32_t k = sh.key[0][at + t];
+        const int to = rowAt[r] + t + runRank(sh.key[0] + cellAt[o1], cellLen[o1], k) +
+                       runRank(sh.key[0] + cellAt[o2], cellLen[o2], k);
+        sh.key[1][to] = k;
+        sh.src[1][to] = (uint16_t)(at + t);
+      }
+    }
+    __syncthreads();
+    mergeRuns(sh.key[1], sh.src[1], sh.key[0], sh.src[0], rowAt, 9);
+    __syncthreads();
+    mergeRuns(sh.key[0], sh.src[0], sh.key[1], sh.src[1], planeAt, 3, sh.own, cellAt[13], cellLen[13]);
+    __syncthreads();
+    const int32_t* key = sh.key[1];
+    const uint16_t* src = sh.src[1];
+    const unsigned mine = 1u << lane, below = mine - 1u;
+    // kWalkers walkers per warp at a time
+    for (int32_t s = s0 + kWalkers*wib; s < s1; s += kWalkers*kCellWarps) {
+      CellWalker w[kWalkers];
+      int cnt[kWalkers];
+      bool some = false;
+#pragma unroll
+      for (int q = 0; q < kWalkers; ++q) {
+        cnt[q] = 0;
+        const int32_t i = s + q < s1 ? M.sortedIdx[s + q] : -1;
+        const bool on = i >= 0 && i < n;
+        some = some || on;
+        const float4 p = a.pre[on ? s + q : s0];
+        const float lm = a.lmax[on ? s + q : s0];
+        // an empty place tests like any other and is not stored
+        w[q] = CellWalker{p.x, p.y, p.z, pretest ? p.w : FLT_MAX, pretest ? __fdividef(k2lo, lm*lm) : -1.0f, on ? i : -1};
+      }
+      if (!some) continue;
+      const int batches = (count + 31) >> 5;              // at most 32
+      // the batch's ballots, kept by the lane of the batch's number
+      unsigned sure[kWalkers], open[kWalkers];
+#pragma unroll
+      for (int q = 0; q < kWalkers; ++q) { sure[q] = 0; open[q] = 0; }
+      for (int b = 0; b < batches; ++b) {
+        const int t = 32*b + lane;
+        const int at = src[t < count ? t : count - 1];
+        const float4 cnd = sh.pre[at];
+        const float cA = t < count ? sh.acc[at] : -FLT_MAX;
+        const float x = t < count ? cnd.x : FLT_MAX;        // past the end: infinitely far
+#pragma unroll
+        for (int q = 0; q < kWalkers; ++q) {
+          const float fx = w[q].x - x, fy = w[q].y - cnd.y, fz = w[q].z - cnd.z;
+          const float r2 = __fmaf_rn(fx, fx, __fmaf_rn(fy, fy, fz*fz));
+          const unsigned in = __ballot_sync(0xffffffffu, r2 <= fmaxf(w[q].A, cA));
+          const unsigned near = __ballot_sync(0xffffffffu, r2 <= fmaxf(w[q].T, cnd.w));
+          if (lane == b) { sure[q] = in; open[q] = near & ~in; }
+        }
+      }
+#pragma unroll
+      for (int q = 0; q < kWalkers; ++q) {
+        const int32_t i = w[q].idx;
+        if (i < 0) continue;
+        // the walker itself is no neighbor
+        const int self = sh.own[s + q - s0];
+        if (self >> 5 == lane) { sure[q] &= ~(1u << (self & 31)); open[q] &= ~(1u << (self & 31)); }
+        // pairs between the bounds, each lane its own batch's
+        while (open[q]) {
+          const int bit = __ffs(open[q]) - 1;
+          open[q] &= open[q] - 1;
+          const int t = 32*lane + bit, at = src[t];
+          if (cellUndecided(M, i, key[t], w[q].x - sh.pre[at].x, w[q].y - sh.pre[at].y, w[q].z - sh.pre[at].z,
+                            sh.pre[at].w, k2, k2lo, k2hi, pretest))
+            sure[q] |= 1u << bit;
+        }
+        __syncwarp();
+        int32_t* out = nullptr;
+        int lim = 0;
+        if (FILL) {
+          const int64_t o = M.offsets[i];
+          lim = M.counts[i];
+          out = M.nbr + o;
+          if (o + lim > M.ecap) {
+            if (lane == 0) atomicOr(M.err, DERR_ENTRY_CAPACITY);
+            lim = 0;
+          }
+        } else if (scap > 0) {
+          out = reinterpret_cast<int32_t*>(M.pacc) + i*(int64_t)scap;
+          lim = scap;
+        }
+        // neighbors after the walker in node order: its own pairs
+        const int before = 32*lane <= self ? self - 32*lane : 0;
+        above += __popc(before >= 32 ? 0u : sure[q] >> before);
+        if (lim > 0) {
+          for (int b = 0; b < batches; ++b) {
+            const unsigned word = __shfl_sync(0xffffffffu, sure[q], b);
+            const int pos = cnt[q] + __popc(word & below);
+            if ((word & mine) && pos < lim) out[pos] = key[32*b + lane];
+            cnt[q] += __popc(word);
+          }
+        } else {
+          cnt[q] += __reduce_add_sync(0xffffffffu, __popc(sure[q]));
+        }
+      }
+      if (!FILL) {
+#pragma unroll
+        for (int q = 0; q < kWalkers; ++q) {
+          if (w[q].idx < 0) continue;
+          if (lane == 0) {
+            M.counts[w[q].idx] = cnt[q];
+            if (cnt[q] > maxNbr) atomicOr(M.err, DERR_NBR_CAPACITY);
+            if (scap > 0 && cnt[q] > scap) atomicOr(M.err, DERR_LIST_CAPACITY);
+          }
+          most = cnt[q] > most ? cnt[q] : most;
+        }
+      }
+    }
+  }
+  // the pairs of this pass's lists (a counting pass without lists leaves them to the fill pass)
+  unsigned long long pairs = FILL || scap > 0 ? above : 0;
+  for (int o = 16; o > 0; o >>= 1) pairs += __shfl_xor_sync(0xffffffffu, pairs, o);
+  if (lane == 0) {
+    if (!FILL && most > 0) atomicMax(reinterpret_cast<int*>(M.scal + SC_MAXCOUNT), most);
+    if (pairs) atomicAdd(reinterpret_cast<unsigned long long*>(M.scal + SC_PAIRS), pairs);
+  }
 }
 
 int64_t grow(int64_t v) { return v + v/4 + 1024; }
@@ -1328,6 +1743,10 @@ int launch_build(Batch& b) {
   b.lastNbrSchedule = nm ? b.mem[0]->lastNbrSchedule : 0;
   const size_t tsmem = sizeof(int32_t)*(size_t)fthreads*tcap;
   const size_t wsmem = sizeof(int32_t)*(wthreads/32)*(size_t)wcap;
+  // the cell walk's staging area, at least a list and a row table per warp
+  const size_t clists = sizeof(int32_t)*kCellWarps*(size_t)(wcap + RowTable<1>::NR*RowTable<1>::RW);
+  const size_t cstage = sizeof(CellShared);
+  const size_t csmem = clists > cstage ? clists : cstage;
   auto smemAttr = [](auto* kernel, size_t bytes) -> int {
     if (bytes <= 48*1024) return SPHGPU_OK;
     return cuda_status(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes),
@@ -1335,17 +1754,20 @@ int launch_build(Batch& b) {
   };
   SPH_TRY(smemAttr(nbr_thread_kernel<false, 1>, tsmem)); SPH_TRY(smemAttr(nbr_thread_kernel<true, 1>, tsmem));
   SPH_TRY(smemAttr(nbr_thread_kernel<false, 2>, tsmem)); SPH_TRY(smemAttr(nbr_thread_kernel<true, 2>, tsmem));
-  SPH_TRY(smemAttr(nbr_walk_kernel<false, 1>, wsmem)); SPH_TRY(smemAttr(nbr_walk_kernel<true, 1>, wsmem));
-  SPH_TRY(smemAttr(nbr_walk_kernel<false, 2>, wsmem)); SPH_TRY(smemAttr(nbr_walk_kernel<true, 2>, wsmem));
+  SPH_TRY(smemAttr(nbr_cell_kernel<false>, csmem)); SPH_TRY(smemAttr(nbr_cell_kernel<true>, csmem));
+  SPH_TRY(smemAttr(nbr_walk_kernel<false>, wsmem)); SPH_TRY(smemAttr(nbr_walk_kernel<true>, wsmem));
   // One walk launch per (schedule, cell subdivision) present.  pass 0: count
   // (and the lists of members with a stash); pass 1: fill (members without).
   auto walk = [&](bool threadSched, int sub, bool fill) -> int {
     BlockMap map;
     unsigned grid = 0;
-    const int threads = threadSched ? (fill || tstash ? fthreads : 256) : wthreads;
+    const int threads = threadSched ? (fill || tstash ? fthreads : 256) : (sub == 1 ? kCellThreads : wthreads);
     SPH_TRY(batch_map_items(b, [&](const Problem& p) {
       if (thread(p) != threadSched || p.grid.sub != sub || (fill && p.grid.stashCap)) return (int64_t)0;
-      return threadSched ? p.candcap : 32*p.candcap; }, threads, &map, &grid));
+      if (threadSched) return p.candcap;
+      // the cell walk: a block per cell up to kCellBlocks, each striding over the member's cells
+      if (sub == 1) return kCellThreads*(p.cellcap < kCellBlocks ? p.cellcap : kCellBlocks);
+      return 32*p.candcap; }, threads, &map, &grid));
     if (!grid) return SPHGPU_OK;
     if (threadSched) {
       const bool lists = fill || tstash;
@@ -1360,19 +1782,27 @@ int launch_build(Batch& b) {
       }
     } else {
       const bool lists = fill || wstash;
-      const size_t smem = lists ? wsmem : 0;
-      const int c = lists ? wcap : 0;
+      const size_t smem = sub == 1 ? csmem : (lists ? wsmem : 0);
+      const int c = lists || sub == 1 ? wcap : 0;
       if (sub == 1) {
-        if (fill) nbr_walk_kernel<true, 1><<<grid, threads, smem, st>>>(b.d_mem, map, c, maxNbr);
-        else nbr_walk_kernel<false, 1><<<grid, threads, smem, st>>>(b.d_mem, map, c, maxNbr);
+        if (fill) nbr_cell_kernel<true><<<grid, threads, smem, st>>>(b.d_mem, map, c, maxNbr);
+        else nbr_cell_kernel<false><<<grid, threads, smem, st>>>(b.d_mem, map, c, maxNbr);
       } else {
-        if (fill) nbr_walk_kernel<true, 2><<<grid, threads, smem, st>>>(b.d_mem, map, c, maxNbr);
-        else nbr_walk_kernel<false, 2><<<grid, threads, smem, st>>>(b.d_mem, map, c, maxNbr);
+        if (fill) nbr_walk_kernel<true><<<grid, threads, smem, st>>>(b.d_mem, map, c, maxNbr);
+        else nbr_walk_kernel<false><<<grid, threads, smem, st>>>(b.d_mem, map, c, maxNbr);
       }
     }
     batch_count_launch(b);
     return SPHGPU_OK;
   };
+  {
+    // the cell walk reads its cells in node order
+    BlockMap om;
+    unsigned ogrid = 0;
+    SPH_TRY(batch_map_items(b, [&](const Problem& p) {
+      return thread(p) || p.grid.sub != 1 ? (int64_t)0 : fixedItems(32*p.cellcap); }, kGhostThreads, &om, &ogrid));
+    if (ogrid) { cell_order_kernel<<<ogrid, kGhostThreads, 0, st>>>(b.d_mem, om); batch_count_launch(b); }
+  }
   for (int sub = 1; sub <= 2; ++sub) {
     SPH_TRY(walk(true, sub, false));
     SPH_TRY(walk(false, sub, false));

@@ -328,7 +328,7 @@ enum DevError {
 enum NbrSchedule {
   NBR_SCHEDULE_AUTO = 0,     // thread per node for small candidate sets, else warp
   NBR_SCHEDULE_THREAD = 1,   // thread per node, cell-sorted order
-  NBR_SCHEDULE_WARP = 2,     // warp per node
+  NBR_SCHEDULE_WARP = 2,     // block per cell (cells of one reach) or warp per node (half a reach)
 };
 
 // ---- batched launches -------------------------------------------------
