@@ -41,12 +41,9 @@ struct CRec {
   T9 gB;
 };
 
-__device__ __forceinline__ CRec loadCRec(const double* crec, int64_t k) {
-  const double2* q = reinterpret_cast<const double2*>(crec + k*CRECW);
-  double2 a[17];
-#pragma unroll
-  for (int t = 0; t < 17; ++t) a[t] = __ldg(q + t);
-  const double* d = reinterpret_cast<const double*>(a);
+__device__ __forceinline__ CRec loadCRec(const double* crec, int64_t cap, int64_t k) {
+  double d[CRECW];
+  ldPlanes<CRECW/4, true>(crec, cap, k, d);
   CRec R;
   R.r = V3{d[C_X], d[C_Y], d[C_Z]};
   R.v = V3{d[C_VX], d[C_VY], d[C_VZ]};
@@ -92,19 +89,28 @@ __global__ void __launch_bounds__(256) pack_crk_records_kernel(const Member* mem
     }
 #pragma unroll
     for (int c = 0; c < 9; ++c) v[C_GRADB + c] = K[(K_GRADB + c)*n + r];
-    double2* q = reinterpret_cast<double2*>(crec + k*CRECW);
+    const int64_t cap = MB.candcap;
 #pragma unroll
-    for (int t = 0; t < CRECW/2; ++t) q[t] = make_double2(v[2*t], v[2*t + 1]);
+    for (int t = 0; t < CRECW/4; ++t) stPlane(crec + planeAt(cap, k, t), v[4*t], v[4*t + 1], v[4*t + 2], v[4*t + 3]);
+    *reinterpret_cast<double2*>(crec + halfPlaneAt(cap, k, CRECW/4)) = make_double2(v[CRECW - 2], v[CRECW - 1]);
   }
 }
 
-// Record fields shared with the SPH record (positions, H, Hdet).
-__device__ __forceinline__ V3 recPos(const double* rec, int64_t j) {
-  return V3{ldg(rec + j*RECW + R_X), ldg(rec + j*RECW + R_Y), ldg(rec + j*RECW + R_Z)};
+// The fields shared with the SPH record: its first three planes.
+struct PosH {
+  V3 r;
+  Sym H;
+  double m, Hdet;
+};
+__device__ __forceinline__ PosH loadPosH(const double* rec, int64_t cap, int64_t k) {
+  double a[12];
+  ldPlanes<3>(rec, cap, k, a);
+  return PosH{V3{a[R_X], a[R_Y], a[R_Z]},
+              Sym{a[R_H], a[R_H + 1], a[R_H + 2], a[R_H + 3], a[R_H + 4], a[R_H + 5]}, a[R_M], a[R_HDET]};
 }
-__device__ __forceinline__ Sym recH(const double* rec, int64_t j) {
-  const double* h = rec + j*RECW + R_H;
-  return Sym{ldg(h), ldg(h + 1), ldg(h + 2), ldg(h + 3), ldg(h + 4), ldg(h + 5)};
+__device__ __forceinline__ V3 recPos(const double* rec, int64_t cap, int64_t j) {
+  const D4 p = ldPlane(rec + planeAt(cap, j, 0));
+  return V3{p.a, p.b, p.c};
 }
 
 // ---------------------------------------------------------------- volumes
@@ -116,18 +122,20 @@ __global__ void __launch_bounds__(128) crk_sum_volume_kernel(const Member* mem, 
   if (i >= n) return;
   const Params& P = MB.prm;
   const double* rec = MB.rec;
+  const int64_t cap = MB.candcap;
   const int64_t* offsets = MB.offsets;
   const int32_t* nbr = MB.nbr;
   double* S = MB.S;
-  const V3 ri = recPos(rec, i);
-  const Sym Hi = recH(rec, i);
-  const double Hdeti = ldg(rec + i*RECW + R_HDET);
+  const PosH I = loadPosH(rec, cap, i);
+  const V3 ri = I.r;
+  const Sym Hi = I.H;
+  const double Hdeti = I.Hdet;
   const double half = 0.5*P.W.extent;
   const double etaVolMax = half*half*half*(4.0/3.0*3.14159265358979323846);
   double vol = 0.0;
   for (int64_t k = offsets[i]; k < offsets[i + 1]; ++k) {
     const int32_t j = __ldg(nbr + k);
-    const V3 rij = vsub(ri, recPos(rec, j));
+    const V3 rij = vsub(ri, recPos(rec, cap, j));
     vol += tableKernel(P.W, mag(sdot(Hi, rij)), Hdeti);
   }
   vol += tableKernel(P.W, 0.0, Hdeti);
@@ -157,20 +165,23 @@ __global__ void __launch_bounds__(128) crk_sum_density_kernel(const Member* mem,
   if (i >= n) return;
   const Params& P = MB.prm;
   const double* rec = MB.rec;
+  const int64_t cap = MB.candcap;
   const int64_t* offsets = MB.offsets;
   const int32_t* nbr = MB.nbr;
   const int32_t* groot = MB.groot;
   double* S = MB.S;
   const double mi = S[S_M*n + i], Vi = S[S_VOL*n + i];
-  const double Hdeti = ldg(rec + i*RECW + R_HDET);
-  const V3 ri = recPos(rec, i);
+  const PosH I = loadPosH(rec, cap, i);
+  const double Hdeti = I.Hdet;
+  const V3 ri = I.r;
   double wsum = 0.0, rho = 0.0, vol1 = 0.0;
   for (int64_t k = offsets[i]; k < offsets[i + 1]; ++k) {
     const int32_t j = __ldg(nbr + k);
     const int64_t r = j < n ? (int64_t)j : (int64_t)__ldg(groot + (j - n));
     const double mj = ldg(S + S_M*n + r), Vj = ldg(S + S_VOL*n + r);
-    const V3 rij = vsub(ri, recPos(rec, j));
-    const double Wj = tableKernel(P.W, mag(sdot(recH(rec, j), rij)), ldg(rec + (int64_t)j*RECW + R_HDET));
+    const PosH J = loadPosH(rec, cap, j);
+    const V3 rij = vsub(ri, J.r);
+    const double Wj = tableKernel(P.W, mag(sdot(J.H, rij)), J.Hdet);
     wsum += Vj*Wj;
     rho += mj*Vj*Wj;
     vol1 += Vj*Vj*Wj;
@@ -190,14 +201,16 @@ __global__ void __launch_bounds__(128) crk_moments_corrections_kernel(const Memb
   if (i >= n) return;
   const Params& P = MB.prm;
   const double* rec = MB.rec;
+  const int64_t cap = MB.candcap;
   const int64_t* offsets = MB.offsets;
   const int32_t* nbr = MB.nbr;
   const int32_t* groot = MB.groot;
   const double* S = MB.S;
   double* K = MB.K;
-  const V3 ri = recPos(rec, i);
-  const Sym Hi = recH(rec, i);
-  const double Hdeti = ldg(rec + i*RECW + R_HDET);
+  const PosH I = loadPosH(rec, cap, i);
+  const V3 ri = I.r;
+  const Sym Hi = I.H;
+  const double Hdeti = I.Hdet;
   const double wi = S[S_VOL*n + i];
   double m0 = 0.0;
   V3 m1{0, 0, 0}, gm0{0, 0, 0};
@@ -221,9 +234,10 @@ __global__ void __launch_bounds__(128) crk_moments_corrections_kernel(const Memb
     if (k == k1) break;
     const int64_t r = j < n ? (int64_t)j : (int64_t)__ldg(groot + (j - n));
     const double wj = ldg(S + S_VOL*n + r);
-    const V3 rij = vsub(ri, recPos(rec, j));
-    const Sym Hj = recH(rec, j);
-    const double Hdetj = ldg(rec + (int64_t)j*RECW + R_HDET);
+    const PosH J = loadPosH(rec, cap, j);
+    const V3 rij = vsub(ri, J.r);
+    const Sym Hj = J.H;
+    const double Hdetj = J.Hdet;
     const V3 etai = sdot(Hi, rij);
     const V3 etaj = sdot(Hj, rij);
     double Wa, gWa, Wb, gWb;
@@ -388,13 +402,14 @@ __global__ void __launch_bounds__(128) crk_eval_kernel(const Member* mem, BlockM
   if (i >= n) return;
   const Params& P = MB.prm;
   const double* crec = MB.crec;
+  const int64_t cap = MB.candcap;
   const int64_t* offsets = MB.offsets;
   const int32_t* nbr = MB.nbr;
   double* D = MB.D;
   double* K = MB.K;
   double* pacc = MB.pacc;
   const int64_t ecap = MB.ecap;
-  const CRec I = loadCRec(crec, i);
+  const CRec I = loadCRec(crec, cap, i);
   const double Cl = P.Cl*(0.5*(1.0 + 1.0)*1.0);
   const double Cq = P.Cq*(0.5*(1.0 + 1.0)*1.0);
   double wns = 0.0, maxvp = 0.0, effvp = 0.0, viscW = 0.0, DepsDt = 0.0;
@@ -404,7 +419,7 @@ __global__ void __launch_bounds__(128) crk_eval_kernel(const Member* mem, BlockM
   const int64_t k0 = offsets[i], k1 = offsets[i + 1];
   for (int64_t k = k0; k < k1; ++k) {
     const int32_t j = __ldg(nbr + k);
-    const CRec J = loadCRec(crec, j);
+    const CRec J = loadCRec(crec, cap, j);
     const bool own = j > (int32_t)i;
     const V3 rij = vsub(I.r, J.r);
     const V3 etai = sdot(I.H, rij);

@@ -43,21 +43,23 @@ struct CMRec {
   float m, rho, cs, P, Hdet, vol, h[6], A, B[3], gA[3], gB[9];
 };
 
-__device__ __forceinline__ CMRec loadCMRec(const double* rec, int64_t k) {
-  const double2* q = reinterpret_cast<const double2*>(rec + k*CMRECW);
-  const double2 a0 = __ldg(q), a1 = __ldg(q + 1), a2 = __ldg(q + 2);
-  const float4* f = reinterpret_cast<const float4*>(q + 3);
-  const float4 f0 = __ldg(f), f1 = __ldg(f + 1), f2 = __ldg(f + 2), f3 = __ldg(f + 3);
-  const float4 f4 = __ldg(f + 4), f5 = __ldg(f + 5), f6 = __ldg(f + 6);
+__device__ __forceinline__ CMRec loadCMRec(const double* rec, int64_t cap, int64_t k) {
+  double a[CMRECW];
+  ldPlanes<CMRECW/4>(rec, cap, k, a);
+  // 28 floats after the six doubles
+  float f[28];
+#pragma unroll
+  for (int c = 0; c < 14; ++c) { f[2*c] = loF(a[6 + c]); f[2*c + 1] = hiF(a[6 + c]); }
   CMRec R;
-  R.x = a0.x; R.y = a0.y; R.z = a1.x; R.vx = a1.y; R.vy = a2.x; R.vz = a2.y;
-  R.m = f0.x; R.rho = f0.y; R.cs = f0.z; R.P = f0.w;
-  R.Hdet = f1.x; R.vol = f1.y; R.h[0] = f1.z; R.h[1] = f1.w;
-  R.h[2] = f2.x; R.h[3] = f2.y; R.h[4] = f2.z; R.h[5] = f2.w;
-  R.A = f3.x; R.B[0] = f3.y; R.B[1] = f3.z; R.B[2] = f3.w;
-  R.gA[0] = f4.x; R.gA[1] = f4.y; R.gA[2] = f4.z; R.gB[0] = f4.w;
-  R.gB[1] = f5.x; R.gB[2] = f5.y; R.gB[3] = f5.z; R.gB[4] = f5.w;
-  R.gB[5] = f6.x; R.gB[6] = f6.y; R.gB[7] = f6.z; R.gB[8] = f6.w;
+  R.x = a[0]; R.y = a[1]; R.z = a[2]; R.vx = a[3]; R.vy = a[4]; R.vz = a[5];
+  R.m = f[0]; R.rho = f[1]; R.cs = f[2]; R.P = f[3]; R.Hdet = f[4]; R.vol = f[5];
+#pragma unroll
+  for (int c = 0; c < 6; ++c) R.h[c] = f[6 + c];
+  R.A = f[12];
+#pragma unroll
+  for (int c = 0; c < 3; ++c) { R.B[c] = f[13 + c]; R.gA[c] = f[16 + c]; }
+#pragma unroll
+  for (int c = 0; c < 9; ++c) R.gB[c] = f[19 + c];
   return R;
 }
 
@@ -74,19 +76,18 @@ __global__ void __launch_bounds__(256) pack_crk_mixed_kernel(const Member* mem, 
   if (k >= n) x = ghostPosition(MB.prm.bcs, x, MB.gcode[k - n]);
   const Sym H{S[(S_H + 0)*n + r], S[(S_H + 1)*n + r], S[(S_H + 2)*n + r],
               S[(S_H + 3)*n + r], S[(S_H + 4)*n + r], S[(S_H + 5)*n + r]};
-  double2* q = reinterpret_cast<double2*>(MB.mrec + k*CMRECW);
-  q[0] = make_double2(x.x, x.y);
-  q[1] = make_double2(x.z, S[S_VX*n + r]);
-  q[2] = make_double2(S[S_VY*n + r], S[S_VZ*n + r]);
-  float4* f = reinterpret_cast<float4*>(q + 3);
   auto kf = [&](int field) { return (float)K[(int64_t)field*n + r]; };
-  f[0] = make_float4((float)S[S_M*n + r], (float)S[S_RHO*n + r], (float)S[S_CS*n + r], (float)S[S_P*n + r]);
-  f[1] = make_float4((float)sdet(H), (float)S[S_VOL*n + r], (float)H.xx, (float)H.xy);
-  f[2] = make_float4((float)H.xz, (float)H.yy, (float)H.yz, (float)H.zz);
-  f[3] = make_float4(kf(K_A), kf(K_B), kf(K_B + 1), kf(K_B + 2));
-  f[4] = make_float4(kf(K_GRADA), kf(K_GRADA + 1), kf(K_GRADA + 2), kf(K_GRADB));
-  f[5] = make_float4(kf(K_GRADB + 1), kf(K_GRADB + 2), kf(K_GRADB + 3), kf(K_GRADB + 4));
-  f[6] = make_float4(kf(K_GRADB + 5), kf(K_GRADB + 6), kf(K_GRADB + 7), kf(K_GRADB + 8));
+  double* q = MB.mrec;
+  const int64_t cap = MB.candcap;
+  stPlane(q + planeAt(cap, k, 0), x.x, x.y, x.z, S[S_VX*n + r]);
+  stPlane(q + planeAt(cap, k, 1), S[S_VY*n + r], S[S_VZ*n + r], packF((float)S[S_M*n + r], (float)S[S_RHO*n + r]),
+          packF((float)S[S_CS*n + r], (float)S[S_P*n + r]));
+  stPlane(q + planeAt(cap, k, 2), packF((float)sdet(H), (float)S[S_VOL*n + r]), packF((float)H.xx, (float)H.xy),
+          packF((float)H.xz, (float)H.yy), packF((float)H.yz, (float)H.zz));
+  stPlane(q + planeAt(cap, k, 3), packF(kf(K_A), kf(K_B)), packF(kf(K_B + 1), kf(K_B + 2)),
+          packF(kf(K_GRADA), kf(K_GRADA + 1)), packF(kf(K_GRADA + 2), kf(K_GRADB)));
+  stPlane(q + planeAt(cap, k, 4), packF(kf(K_GRADB + 1), kf(K_GRADB + 2)), packF(kf(K_GRADB + 3), kf(K_GRADB + 4)),
+          packF(kf(K_GRADB + 5), kf(K_GRADB + 6)), packF(kf(K_GRADB + 7), kf(K_GRADB + 8)));
 }
 
 __device__ __forceinline__ void tableF(const float* coef, int n, float invStep, float extent, float eta, float Hdet,
@@ -178,6 +179,7 @@ __global__ void __launch_bounds__(128, 3) crk_eval_mixed_kernel(const Member* me
   if (i >= n) return;
   const Params& P = MB.prm;
   const double* rec = MB.mrec;
+  const int64_t cap = MB.candcap;
   const int64_t* offsets = MB.offsets;
   const int32_t* nbr = MB.nbr;
   double* D = MB.D;
@@ -185,7 +187,7 @@ __global__ void __launch_bounds__(128, 3) crk_eval_mixed_kernel(const Member* me
   const int64_t ecap = MB.ecap;
   const TabF T{MB.coefF, P.W.n, (float)(1.0/P.W.stepSize), (float)P.W.extent};
   const float eps2 = (float)P.eps2, Cl = (float)P.Cl, Cq = (float)P.Cq;
-  const CMRec I = loadCMRec(rec, i);
+  const CMRec I = loadCMRec(rec, cap, i);
   KahanF wns, effvp, viscW, DepsDt, DvDt[3], gradRho[3], XSPHdv[3], m2[6], DvDx[9];
   wns.init(); effvp.init(); viscW.init(); DepsDt.init();
 #pragma unroll
@@ -198,7 +200,7 @@ __global__ void __launch_bounds__(128, 3) crk_eval_mixed_kernel(const Member* me
   const int64_t k0 = offsets[i], k1 = offsets[i + 1];
   for (int64_t k = k0; k < k1; ++k) {
     const int32_t j = __ldg(nbr + k);
-    const CMRec J = loadCMRec(rec, j);
+    const CMRec J = loadCMRec(rec, cap, j);
     const bool own = j > (int32_t)i;
     const F3 rij{(float)(I.x - J.x), (float)(I.y - J.y), (float)(I.z - J.z)};
     const F3 vij{(float)(I.vx - J.vx), (float)(I.vy - J.vy), (float)(I.vz - J.vz)};

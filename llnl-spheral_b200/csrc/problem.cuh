@@ -5,7 +5,8 @@
 //   S0   [NSTATE][n]      start-of-step copy (CheapSynchronousRK2 state0)
 //   D    [NDERIV][n]      StateDerivatives of the internal nodes, SoA
 //   rec  [n+G][RECW]      packed pair records (state gathered for a neighbor
-//                         walk; ghosts are images of their root), 160 B each
+//                         walk; ghosts are images of their root), 160 B each,
+//                         stored as planes of 32 bytes per node (ldPlanes)
 //   groot/gcode [G]       ghost -> internal root node, per-axis image code
 //   offsets [n+1] (i64), nbr [E] (i32)   ConnectivityMap as CSR, ascending j
 //   pacc [3][E]           owner-oriented pair acceleration per CSR entry
@@ -30,7 +31,7 @@
 // Blocks of 128 threads per SM the derivative pair kernels are compiled for
 // (the register budget follows: 65,536 / (128 x blocks)).  The FP64 pair
 // kernel keeps node i's record and its two tensor sums in shared memory
-// (SPH_FP64_SHARED_I, SPH_FP64_SHARED_ACC), which brings it to 4 blocks: on
+// (SPH_FP64_SHARED_ACC for the sums), which brings it to 4 blocks: on
 // Kelvin-Helmholtz 128^3 and Sod 256x32x32 that evaluates 15-17% faster than
 // the all-register form at 2 blocks, with the same bits.
 #ifndef SPH_FP64_MIN_BLOCKS
@@ -38,10 +39,6 @@
 #endif
 #ifndef SPH_MIXED_MIN_BLOCKS
 #define SPH_MIXED_MIN_BLOCKS 3
-#endif
-// 1: the FP64 pair kernel keeps node i's record in shared memory
-#ifndef SPH_FP64_SHARED_I
-#define SPH_FP64_SHARED_I 1
 #endif
 // 1: ... and accumulates its two tensor sums there
 #ifndef SPH_FP64_SHARED_ACC
@@ -118,7 +115,7 @@ enum DerivField {
 // Packed pair record: everything one side of a pair needs.
 enum RecField {
   // position, m, det H and H first: the summed density and the CRKSPH
-  // volumes read the first 96 bytes (three sectors) of a neighbor's record
+  // volumes read the first three planes of a neighbor's record
   R_X = 0, R_Y, R_Z, R_M, R_HDET,
   R_H = 5,             // 6
   R_VX = 11, R_VY, R_VZ, R_RHO, R_CS,
@@ -129,41 +126,85 @@ enum RecField {
   RECW = 20
 };
 
+// Pair records are stored as planes: doubles 4q .. 4q+3 of node k's record at
+// ((q*cap + k)*4), cap the node capacity of the buffers (Member::candcap), and
+// a last half plane of two doubles per node where the record's length leaves
+// one.  A pair loop's lanes visit nodes that are mostly consecutive, so one
+// 32-byte load of a warp covers 8 to 12 cache lines; with whole records side
+// by side every lane's load is a line of its own (32 lines for each of the
+// ten 16-byte loads), and those line accesses bound the pair kernels.  A
+// 32-byte piece is a whole sector, so a node order without locality costs no
+// more sectors than whole records do.  Measured (B200, Kelvin-Helmholtz 128^3,
+// whole records -> planes): FP64 pair kernel 807 -> 688 us, summed density
+// 268 -> 184, mid-point update 229 -> 183; mixed 511 -> 488, 203 -> 137,
+// 195 -> 168; CRKSPH 1M volumes and density 202 -> 119.
+struct D4 {
+  double a, b, c, d;
+};
+__device__ __forceinline__ D4 ldPlane(const double* p) {       // read-only data, 32-byte aligned
+  D4 v;
+  asm("ld.global.nc.v4.f64 {%0,%1,%2,%3}, [%4];" : "=d"(v.a), "=d"(v.b), "=d"(v.c), "=d"(v.d) : "l"(p));
+  return v;
+}
+__device__ __forceinline__ D4 ldPlaneW(const double* p) {      // data other threads of the launch write elsewhere
+  D4 v;
+  asm volatile("ld.global.v4.f64 {%0,%1,%2,%3}, [%4];" : "=d"(v.a), "=d"(v.b), "=d"(v.c), "=d"(v.d) : "l"(p) : "memory");
+  return v;
+}
+__device__ __forceinline__ void stPlane(double* p, double a, double b, double c, double d) {
+  asm volatile("st.global.v4.f64 [%0], {%1,%2,%3,%4};" : : "l"(p), "d"(a), "d"(b), "d"(c), "d"(d) : "memory");
+}
+// plane q of node k
+__host__ __device__ __forceinline__ int64_t planeAt(int64_t cap, int64_t k, int q) { return (q*cap + k)*4; }
+// the half plane after Q planes
+__host__ __device__ __forceinline__ int64_t halfPlaneAt(int64_t cap, int64_t k, int Q) { return Q*cap*4 + k*2; }
+
+// a record's first 4*Q doubles (and the half plane after them)
+template<int Q, bool HALF = false>
+__device__ __forceinline__ void ldPlanes(const double* rec, int64_t cap, int64_t k, double* v) {
+#pragma unroll
+  for (int q = 0; q < Q; ++q) {
+    const D4 p = ldPlane(rec + planeAt(cap, k, q));
+    v[4*q] = p.a; v[4*q + 1] = p.b; v[4*q + 2] = p.c; v[4*q + 3] = p.d;
+  }
+  if (HALF) {
+    const double2 h = __ldg(reinterpret_cast<const double2*>(rec + halfPlaneAt(cap, k, Q)));
+    v[4*Q] = h.x; v[4*Q + 1] = h.y;
+  }
+}
+// two floats in the place of a double
+__device__ __forceinline__ double packF(float lo, float hi) {
+  return __hiloint2double(__float_as_int(hi), __float_as_int(lo));
+}
+__device__ __forceinline__ float loF(double v) { return __int_as_float(__double2loint(v)); }
+__device__ __forceinline__ float hiF(double v) { return __int_as_float(__double2hiint(v)); }
+
 // The pair records of one node, from its state.  Written by the record
 // pack kernels and by the update kernel (which packs the internal nodes as
 // it advances them); every writer is compiled in the same translation unit
 // (sph.cu, -fmad=false), so a node's record has the same bits whoever wrote it.
-__device__ __forceinline__ void writeRecord(double* rec, int64_t k, const V3& x, const V3& v, double m, double rho,
-                                            double cs, double P, double omega, const Sym& H) {
+__device__ __forceinline__ void writeRecord(double* rec, int64_t cap, int64_t k, const V3& x, const V3& v, double m,
+                                            double rho, double cs, double P, double omega, const Sym& H) {
   const double somega = safeInv(omega, 1.0e-30);
-  double2* q = reinterpret_cast<double2*>(rec + k*RECW);
-  q[0] = make_double2(x.x, x.y);
-  q[1] = make_double2(x.z, m);
-  q[2] = make_double2(sdet(H), H.xx);
-  q[3] = make_double2(H.xy, H.xz);
-  q[4] = make_double2(H.yy, H.yz);
-  q[5] = make_double2(H.zz, v.x);
-  q[6] = make_double2(v.y, v.z);
-  q[7] = make_double2(rho, cs);
-  q[8] = make_double2(somega*P/(rho*rho), m/rho);
-  q[9] = make_double2(P, somega);
+  stPlane(rec + planeAt(cap, k, 0), x.x, x.y, x.z, m);
+  stPlane(rec + planeAt(cap, k, 1), sdet(H), H.xx, H.xy, H.xz);
+  stPlane(rec + planeAt(cap, k, 2), H.yy, H.yz, H.zz, v.x);
+  stPlane(rec + planeAt(cap, k, 3), v.y, v.z, rho, cs);
+  stPlane(rec + planeAt(cap, k, 4), somega*P/(rho*rho), m/rho, P, somega);
 }
 
 // Mixed-precision record (MRECW doubles): FP64 position and velocity, FP32
 // m, rho, cs, det H, H, P/rho^2 term, m/rho, P, safeOmega, isotropy flag.
-__device__ __forceinline__ void writeMixedRecord(double* mrec, int64_t k, const V3& x, const V3& v, double m,
-                                                 double rho, double cs, double P, double omega, const Sym& H) {
+__device__ __forceinline__ void writeMixedRecord(double* mrec, int64_t cap, int64_t k, const V3& x, const V3& v,
+                                                 double m, double rho, double cs, double P, double omega, const Sym& H) {
   const double somega = safeInv(omega, 1.0e-30);
-  double2* q = reinterpret_cast<double2*>(mrec + k*MRECW);
-  q[0] = make_double2(x.x, x.y);
-  q[1] = make_double2(x.z, v.x);
-  q[2] = make_double2(v.y, v.z);
-  float4* f = reinterpret_cast<float4*>(q + 3);
-  f[0] = make_float4((float)m, (float)rho, (float)cs, (float)sdet(H));
-  f[1] = make_float4((float)H.xx, (float)H.xy, (float)H.xz, (float)H.yy);
-  f[2] = make_float4((float)H.yz, (float)H.zz, (float)(somega*P/(rho*rho)), (float)(m/rho));
+  stPlane(mrec + planeAt(cap, k, 0), x.x, x.y, x.z, v.x);
+  stPlane(mrec + planeAt(cap, k, 1), v.y, v.z, packF((float)m, (float)rho), packF((float)cs, (float)sdet(H)));
+  stPlane(mrec + planeAt(cap, k, 2), packF((float)H.xx, (float)H.xy), packF((float)H.xz, (float)H.yy),
+          packF((float)H.yz, (float)H.zz), packF((float)(somega*P/(rho*rho)), (float)(m/rho)));
   const bool iso = H.xy == 0.0 && H.xz == 0.0 && H.yz == 0.0 && H.xx == H.yy && H.xx == H.zz;
-  f[3] = make_float4((float)P, (float)somega, iso ? 1.0f : 0.0f, 0.0f);
+  *reinterpret_cast<double2*>(mrec + halfPlaneAt(cap, k, 3)) =
+      make_double2(packF((float)P, (float)somega), packF(iso ? 1.0f : 0.0f, 0.0f));
 }
 
 // Read-only physics parameters of one problem (in its Member descriptor).

@@ -12,14 +12,15 @@
 //   hydro_dt             GenericHydro::dt (src/Physics/GenericHydro.cc:114-331)
 //   enforce_boundaries   PeriodicBoundary violation mapping (src/Boundary/PeriodicBoundary.cc:145-203)
 //
-// Pair loops gather: one thread owns node i and walks its ascending CSR row.
-// The reference visits each unordered pair once, from the lower index (the
-// "owner"), and scatters to both nodes.  Here every pair term is formed in
-// owner orientation (r_ij = r_owner - r_other, owner-side Q, owner-side
-// tensile factor) and only node i's side is accumulated.  Node i's sums then
-// receive the same terms in the same order as in the reference: first the
-// pairs owned by lower indices (ascending), then its own (ascending, ghosts
-// last), with self terms inserted where the reference adds them.
+// Pair loops gather over node i's ascending CSR row.  The reference visits
+// each unordered pair once, from the lower index (the "owner"), and scatters
+// to both nodes.  Here every pair term is formed from node i's side, equal to
+// the owner's form up to an exact sign (the owner's order is kept where more
+// than two terms are added), and only node i's side is accumulated.  Node i's
+// sums then receive the same terms in the same order as in the reference:
+// first the pairs owned by lower indices (ascending), then its own
+// (ascending, ghosts last), with self terms inserted where the reference adds
+// them.
 #include <cfloat>
 
 #include "problem.cuh"
@@ -43,26 +44,18 @@ struct Rec {
   double Prho, mrho, P, somega;
 };
 
-__device__ __forceinline__ Rec loadRec(const double* rec, int64_t k) {
-  const double2* q = reinterpret_cast<const double2*>(rec + k*RECW);
-  const double2 a0 = __ldg(q + 0), a1 = __ldg(q + 1), a2 = __ldg(q + 2), a3 = __ldg(q + 3), a4 = __ldg(q + 4);
-  const double2 a5 = __ldg(q + 5), a6 = __ldg(q + 6), a7 = __ldg(q + 7), a8 = __ldg(q + 8), a9 = __ldg(q + 9);
+__device__ __forceinline__ Rec loadRec(const double* rec, int64_t cap, int64_t k) {
+  double a[RECW];
+  ldPlanes<RECW/4>(rec, cap, k, a);
   Rec R;
   // the layout of writeRecord (problem.cuh)
-  R.r = V3{a0.x, a0.y, a1.x};
-  R.m = a1.y; R.Hdet = a2.x;
-  R.H = Sym{a2.y, a3.x, a3.y, a4.x, a4.y, a5.x};
-  R.v = V3{a5.y, a6.x, a6.y};
-  R.rho = a7.x; R.cs = a7.y;
-  R.Prho = a8.x; R.mrho = a8.y; R.P = a9.x; R.somega = a9.y;
+  R.r = V3{a[R_X], a[R_Y], a[R_Z]};
+  R.m = a[R_M]; R.Hdet = a[R_HDET];
+  R.H = Sym{a[R_H], a[R_H + 1], a[R_H + 2], a[R_H + 3], a[R_H + 4], a[R_H + 5]};
+  R.v = V3{a[R_VX], a[R_VY], a[R_VZ]};
+  R.rho = a[R_RHO]; R.cs = a[R_CS];
+  R.Prho = a[R_PRHO]; R.mrho = a[R_MRHO]; R.P = a[R_P]; R.somega = a[R_SOMEGA];
   return R;
-}
-
-__device__ __forceinline__ V3 selv(bool c, const V3& a, const V3& b) {
-  return V3{c ? a.x : b.x, c ? a.y : b.y, c ? a.z : b.z};
-}
-__device__ __forceinline__ Sym sels(bool c, const Sym& a, const Sym& b) {
-  return Sym{c ? a.xx : b.xx, c ? a.xy : b.xy, c ? a.xz : b.xz, c ? a.yy : b.yy, c ? a.yz : b.yz, c ? a.zz : b.zz};
 }
 
 // ---------------------------------------------------------------- records
@@ -88,15 +81,18 @@ __device__ __forceinline__ void nodeRecordState(const Member& M, int64_t k, V3& 
 // root's state.  W doubles per record, position in the first three.
 template<int W>
 __device__ __forceinline__ void ghostFromRoot(const Member& M, double* recs, int64_t k) {
-  const int64_t r = M.groot[k - M.n];
-  const double2* src = reinterpret_cast<const double2*>(recs + r*W);
-  double2* dst = reinterpret_cast<double2*>(recs + k*W);
-  const double2 p01 = src[0], p2v = src[1];
-  const V3 x = ghostPosition(M.prm.bcs, V3{p01.x, p01.y, p2v.x}, M.gcode[k - M.n]);
-  dst[0] = make_double2(x.x, x.y);
-  dst[1] = make_double2(x.z, p2v.y);
+  const int64_t r = M.groot[k - M.n], cap = M.candcap;
+  D4 p = ldPlaneW(recs + planeAt(cap, r, 0));
+  const V3 x = ghostPosition(M.prm.bcs, V3{p.a, p.b, p.c}, M.gcode[k - M.n]);
+  stPlane(recs + planeAt(cap, k, 0), x.x, x.y, x.z, p.d);
 #pragma unroll
-  for (int c = 2; c < W/2; ++c) dst[c] = src[c];
+  for (int q = 1; q < W/4; ++q) {
+    p = ldPlaneW(recs + planeAt(cap, r, q));
+    stPlane(recs + planeAt(cap, k, q), p.a, p.b, p.c, p.d);
+  }
+  if (W % 4)
+    *reinterpret_cast<double2*>(recs + halfPlaneAt(cap, k, W/4)) =
+        *reinterpret_cast<const double2*>(recs + halfPlaneAt(cap, r, W/4));
 }
 
 // ghostsOnly: the update kernel wrote the internal nodes' records (in the
@@ -110,7 +106,7 @@ __global__ void __launch_bounds__(256) pack_records_kernel(const Member* mem, Bl
   if (ghostsOnly) { ghostFromRoot<RECW>(M, M.rec, k); return; }
   V3 x, v; double m, rho, cs, P, omega; Sym H;
   nodeRecordState(M, k, x, v, m, rho, cs, P, omega, H);
-  writeRecord(M.rec, k, x, v, m, rho, cs, P, omega, H);
+  writeRecord(M.rec, M.candcap, k, x, v, m, rho, cs, P, omega, H);
 }
 
 __global__ void __launch_bounds__(256) pack_mixed_kernel(const Member* mem, BlockMap bm, int ghostsOnly) {
@@ -121,17 +117,16 @@ __global__ void __launch_bounds__(256) pack_mixed_kernel(const Member* mem, Bloc
   if (ghostsOnly) { ghostFromRoot<MRECW>(M, M.mrec, k); return; }
   V3 x, v; double m, rho, cs, P, omega; Sym H;
   nodeRecordState(M, k, x, v, m, rho, cs, P, omega, H);
-  writeMixedRecord(M.mrec, k, x, v, m, rho, cs, P, omega, H);
+  writeMixedRecord(M.mrec, M.candcap, k, x, v, m, rho, cs, P, omega, H);
 }
 
 // ---------------------------------------------------------------- derivatives
-// The terms of one directed pair (i, j) that node i's sums take, formed in
-// owner orientation (own: i owns the pair, j > i).  The reference forms every
-// pair term from the owner A and the other node B.  Here each quantity is
-// formed once for node i and once for node j, with the same operands in the
-// same order: with the owner-oriented separation r_ij = r_A - r_B (= r_i -
-// r_j or its exact negation), eta_i = H_i r_ij is eta_A when i owns the pair
-// and eta_B otherwise, and likewise for j.  Sums of two pair terms are
+// The terms of one directed pair (i, j) that node i's sums take (own: i owns
+// the pair, j > i).  The reference forms every pair term from the owner A and
+// the other node B with r_AB = r_A - r_B.  Every term is odd or even under
+// that orientation with exact FP negation, so each is formed once from node
+// i's side (r_ij = r_i - r_j), with the same operands in the same order; the
+// signs cancel where node i's sums take it.  Sums of two pair terms are
 // commutative and keep their bits; where three or more are added the owner's
 // order is selected explicitly.
 struct PairTerms {
@@ -140,29 +135,27 @@ struct PairTerms {
   bool own;
 };
 
-template<bool TENSILE>
-__device__ __forceinline__ PairTerms pairTerms(const Rec& I, bool isoI, const Rec& J, bool own, const Params& P,
+template<bool TENSILE, class RecI>
+__device__ __forceinline__ PairTerms pairTerms(const RecI& I, bool isoI, const Rec& J, bool own, const Params& P,
                                                double Cl, double Cq) {
   PairTerms t;
   t.own = own;
   t.mj = J.m;
   t.mrhoj = J.mrho;
-  const V3 d = vsub(I.r, J.r);
-  const V3 rij = own ? d : V3{-d.x, -d.y, -d.z};
-  const V3 dv = vsub(I.v, J.v);
-  const V3 vij = own ? dv : V3{-dv.x, -dv.y, -dv.z};
+  const V3 rij = vsub(I.r(), J.r);
+  const V3 vij = vsub(I.v(), J.v);
   t.rij = rij;
   t.vij = vij;
   // H = h I (the common case): every H product reduces to a scaling with
   // the same bits (the off-diagonal terms add exact zeros)
   const bool iso = isoI && isoSym(J.H);
-  const V3 etaI = iso ? vmul(rij, I.H.xx) : sdot(I.H, rij);
+  const V3 etaI = iso ? vmul(rij, I.hxx()) : sdot(I.H(), rij);
   const V3 etaJ = iso ? vmul(rij, J.H.xx) : sdot(J.H, rij);
   const V3 uI = unitVector(etaI), uJ = unitVector(etaJ);
-  const V3 HetaI = iso ? vmul(uI, I.H.xx) : sdot(I.H, uI);
+  const V3 HetaI = iso ? vmul(uI, I.hxx()) : sdot(I.H(), uI);
   const V3 HetaJ = iso ? vmul(uJ, J.H.xx) : sdot(J.H, uJ);
   double WI, gWI, WJ, gWJ;
-  tableKernelAndGrad(P.W, mag(etaI), I.Hdet, WI, gWI);
+  tableKernelAndGrad(P.W, mag(etaI), I.Hdet(), WI, gWI);
   tableKernelAndGrad(P.W, mag(etaJ), J.Hdet, WJ, gWJ);
   const V3 gradWI = vmul(HetaI, gWI);    // node i's side of the pair
   const V3 gradWJ = vmul(HetaJ, gWJ);
@@ -174,26 +167,26 @@ __device__ __forceinline__ PairTerms pairTerms(const Rec& I, bool isoI, const Re
   const double muI = dot(vij, etaI)/(mag2(etaI) + P.eps2);
   const double muJ = dot(vij, etaJ)/(mag2(etaJ) + P.eps2);
   const double mI0 = dmin(0.0, muI), mJ0 = dmin(0.0, muJ);
-  const double eI = -Cl*I.cs*(P.linearInExp ? muI : mI0) + Cq*(P.quadInExp ? -sgn(muI)*muI*muI : mI0*mI0);
+  const double eI = -Cl*I.cs()*(P.linearInExp ? muI : mI0) + Cq*(P.quadInExp ? -sgn(muI)*muI*muI : mI0*mI0);
   const double eJ = -Cl*J.cs*(P.linearInExp ? muJ : mJ0) + Cq*(P.quadInExp ? -sgn(muJ)*muJ*muJ : mJ0*mJ0);
-  const double qI = eI/I.rho, qJ = eJ/J.rho;   // (e/rho) * Tensor::one
+  const double qI = eI/I.rho(), qJ = eJ/J.rho;   // (e/rho) * Tensor::one
   // 0.5*(Pi * gradWQ), with WQ = W (same table): the off-diagonal zeros of
   // Pi only add signed zeros.
   const V3 QaccI = vmul(vmul(gradWI, qI), 0.5);
   const V3 QaccJ = vmul(vmul(gradWJ, qJ), 0.5);
   t.workQI = dot(vij, QaccI);
-  t.QI = I.rho*I.rho*fabs(qI);
+  t.QI = I.rho()*I.rho()*fabs(qI);
   // pressure terms (tensile correction uses the owner's W)
   double PrhoI, PrhoJ;
   if (TENSILE) {
-    const double x = own ? WI/(I.Hdet*P.WnPerh) : WJ/(J.Hdet*P.WnPerh);
+    const double x = own ? WI/(I.Hdet()*P.WnPerh) : WJ/(J.Hdet*P.WnPerh);
     const double fij = P.epsTensile*(x*x*x*x);
-    const double RI = fij*(I.P < 0.0 ? -I.P : 0.0);
+    const double RI = fij*(I.P() < 0.0 ? -I.P() : 0.0);
     const double RJ = fij*(J.P < 0.0 ? -J.P : 0.0);
-    PrhoI = I.somega*(I.P + RI)/(I.rho*I.rho);
+    PrhoI = I.somega()*(I.P() + RI)/(I.rho()*I.rho());
     PrhoJ = J.somega*(J.P + RJ)/(J.rho*J.rho);
   } else {
-    PrhoI = I.Prho;
+    PrhoI = I.Prho();
     PrhoJ = J.Prho;
   }
   t.PrhoI = PrhoI;
@@ -201,6 +194,104 @@ __device__ __forceinline__ PairTerms pairTerms(const Rec& I, bool isoI, const Re
   const V3 pp = vadd(vmul(gradWI, PrhoI), vmul(gradWJ, PrhoJ));
   t.dd = vadd(vadd(pp, own ? QaccI : QaccJ), own ? QaccJ : QaccI);
   return t;
+}
+
+// Node i's record in shared memory, field f at d[f*STRIDE]: with a column per
+// thread every read is free of bank conflicts (a record per thread is 160
+// bytes from the next, four threads to a bank).
+template<int STRIDE>
+struct ColumnRec {
+  const double* d;
+  __device__ __forceinline__ double at(int f) const { return d[f*STRIDE]; }
+  __device__ __forceinline__ V3 r() const { return V3{at(R_X), at(R_Y), at(R_Z)}; }
+  __device__ __forceinline__ V3 v() const { return V3{at(R_VX), at(R_VY), at(R_VZ)}; }
+  __device__ __forceinline__ double hxx() const { return at(R_H); }
+  __device__ __forceinline__ Sym H() const {
+    return Sym{at(R_H), at(R_H + 1), at(R_H + 2), at(R_H + 3), at(R_H + 4), at(R_H + 5)};
+  }
+  __device__ __forceinline__ double m() const { return at(R_M); }
+  __device__ __forceinline__ double Hdet() const { return at(R_HDET); }
+  __device__ __forceinline__ double rho() const { return at(R_RHO); }
+  __device__ __forceinline__ double cs() const { return at(R_CS); }
+  __device__ __forceinline__ double Prho() const { return at(R_PRHO); }
+  __device__ __forceinline__ double mrho() const { return at(R_MRHO); }
+  __device__ __forceinline__ double P() const { return at(R_P); }
+  __device__ __forceinline__ double somega() const { return at(R_SOMEGA); }
+};
+
+// The pair sums of one node.
+struct NodeSums {
+  double rhoSum, norm, wns, maxvp, effvp, viscW, DepsDt, XSPHw;
+  V3 DvDt, XSPHdv;
+  Sym m2;
+  T9 DvDx, M;
+};
+
+// The per-node finish (src/SPH/SPHHydroBase.cc:834-902) and the stores of
+// the node's derivatives at d (SoA, coalesced across the warp).
+template<bool XSPH, class RecI>
+__device__ __forceinline__ void finishNode(const Params& P, const RecI& I, const NodeSums& t, int numNeighbors,
+                                           double* d, int64_t n) {
+  const double mi = I.m(), rhoi = I.rho(), Hdeti = I.Hdet();
+  const double rhoSum = t.rhoSum + mi*P.W0*Hdeti;
+  const double norm = t.norm + mi/rhoi*P.W0*Hdeti;
+  T9 Mi = t.M, DvDxi = t.DvDx;
+  if (P.correctVelGrad && fabs(tdet(Mi)) > 1.0e-10 && numNeighbors > 8) {
+    Mi = tinverse(Mi);
+    DvDxi = tdot(DvDxi, Mi);
+  } else {
+    DvDxi = tdiv(DvDxi, rhoi);
+  }
+  const double DrhoDt = -rhoi*ttrace(DvDxi);
+  double wns = dmax(0.0, t.wns/Hdeti);
+  wns = sgn(wns)*pow(fabs(wns), 0.3333333333333333);          // Dim<3>::rootnu
+  const Sym m2 = sdiv(t.m2, Hdeti*Hdeti);
+  double XSPHw = t.XSPHw;
+  V3 DxDt = I.v();
+  if (XSPH) {
+    XSPHw += Hdeti*mi/rhoi*P.W0;
+    DxDt = vadd(I.v(), vdiv(t.XSPHdv, dmax(1.0e-30, XSPHw)));
+  }
+  const Sym DHDt = smul(sdiv(sneg(I.H()), 3.0), ttrace(DvDxi));
+  // SPHSmoothingScale::idealSmoothingScale (src/NodeList/SPHSmoothingScale.cc:118-199)
+  double nPerhCur;
+  if (fuzzyEqual(wns, 0.0)) {
+    nPerhCur = 0.5*P.nPerh;
+  } else {
+    nPerhCur = equivalentNodesPerSmoothingScale(P, wns);
+  }
+  const double s = dmin(4.0, dmax(0.25, P.nPerh/(nPerhCur + 1.0e-30)));
+  const double a = s < 1.0 ? 0.4*(1.0 + s*s) : 0.4*(1.0 + 1.0/(s*s*s));
+  const double hi0 = 1.0/I.hxx();
+  const double hi1 = dmin(P.hmax, dmax(P.hmin, hi0*(1.0 - a + a*s)));
+  const double hinv = 1.0/hi1;
+
+  // ---- stores (SoA, coalesced across the warp)
+  d[(D_DXDT + 0)*n] = DxDt.x; d[(D_DXDT + 1)*n] = DxDt.y; d[(D_DXDT + 2)*n] = DxDt.z;
+  d[(D_DVDT + 0)*n] = t.DvDt.x; d[(D_DVDT + 1)*n] = t.DvDt.y; d[(D_DVDT + 2)*n] = t.DvDt.z;
+  d[D_DRHODT*n] = DrhoDt;
+  d[D_DEPSDT*n] = t.DepsDt;
+  d[(D_DHDT + 0)*n] = DHDt.xx; d[(D_DHDT + 1)*n] = DHDt.xy; d[(D_DHDT + 2)*n] = DHDt.xz;
+  d[(D_DHDT + 3)*n] = DHDt.yy; d[(D_DHDT + 4)*n] = DHDt.yz; d[(D_DHDT + 5)*n] = DHDt.zz;
+  d[(D_HIDEAL + 0)*n] = 1.0*hinv; d[(D_HIDEAL + 1)*n] = 0.0*hinv; d[(D_HIDEAL + 2)*n] = 0.0*hinv;
+  d[(D_HIDEAL + 3)*n] = 1.0*hinv; d[(D_HIDEAL + 4)*n] = 0.0*hinv; d[(D_HIDEAL + 5)*n] = 1.0*hinv;
+  const double* dv = &DvDxi.xx;
+  const double* mm = &Mi.xx;
+#pragma unroll
+  for (int c = 0; c < 9; ++c) {
+    d[(D_DVDX + c)*n] = dv[c];
+    d[(D_M + c)*n] = mm[c];
+  }
+  d[D_RHOSUM*n] = rhoSum;
+  d[D_NORM*n] = norm;
+  d[D_WNS*n] = wns;
+  d[(D_M2 + 0)*n] = m2.xx; d[(D_M2 + 1)*n] = m2.xy; d[(D_M2 + 2)*n] = m2.xz;
+  d[(D_M2 + 3)*n] = m2.yy; d[(D_M2 + 4)*n] = m2.yz; d[(D_M2 + 5)*n] = m2.zz;
+  d[D_XSPHW*n] = XSPHw;
+  d[(D_XSPHDV + 0)*n] = t.XSPHdv.x; d[(D_XSPHDV + 1)*n] = t.XSPHdv.y; d[(D_XSPHDV + 2)*n] = t.XSPHdv.z;
+  d[D_MAXVP*n] = t.maxvp;
+  d[D_EFFVP*n] = t.effvp;
+  d[D_VISCW*n] = t.viscW;
 }
 
 // SPHHydroBase::evaluateDerivatives: one thread per internal node i, its CSR
@@ -215,21 +306,23 @@ __global__ void __launch_bounds__(128, SPH_FP64_MIN_BLOCKS) sph_eval_fp64_kernel
   if (i >= n) return;
   const Params& P = MB.prm;
   const double* rec = MB.rec;
+  const int64_t cap = MB.candcap;
   const int64_t* offsets = MB.offsets;
   const int32_t* nbr = MB.nbr;
   double* D = MB.D;
   double* pacc = MB.pacc;
   const int64_t ecap = MB.ecap;
-#if SPH_FP64_SHARED_I
   // node i's record lives in shared memory: the pair loop reads its fields
-  // from there instead of holding 19 doubles in registers across the loop
-  __shared__ Rec sI[128];
-  sI[threadIdx.x] = loadRec(rec, i);
-  const Rec& I = sI[threadIdx.x];
-#else
-  const Rec I = loadRec(rec, i);
-#endif
-  const bool isoI = isoSym(I.H);
+  // from there instead of holding 20 doubles in registers across the loop
+  __shared__ double sI[RECW][128];
+  {
+    double a[RECW];
+    ldPlanes<RECW/4>(rec, cap, i, a);
+#pragma unroll
+    for (int f = 0; f < RECW; ++f) sI[f][threadIdx.x] = a[f];
+  }
+  const ColumnRec<128> I{&sI[0][threadIdx.x]};
+  const bool isoI = isoSym(I.H());
   double rhoSum = 0.0, norm = 0.0, wns = 0.0, maxvp = 0.0, effvp = 0.0, viscW = 0.0, DepsDt = 0.0;
   double XSPHw = 0.0;
   V3 DvDt{0.0, 0.0, 0.0}, XSPHdv{0.0, 0.0, 0.0};
@@ -259,15 +352,15 @@ __global__ void __launch_bounds__(128, SPH_FP64_MIN_BLOCKS) sph_eval_fp64_kernel
       m2 = sadd(m2, smul(thpt, g2));
     }
     rhoSum += t.mj*t.WI;
-    norm += I.mrho*t.WI;
+    norm += I.mrho()*t.WI;
     maxvp = dmax(maxvp, t.QI);
     effvp += t.mrhoj*t.QI*t.WI;
     viscW += t.mj*t.workQI;
-    DvDt = vadd(DvDt, vmul(t.dd, t.own ? -t.mj : t.mj));
+    DvDt = vadd(DvDt, vmul(t.dd, -t.mj));
     DepsDt += t.mj*(t.PrhoI*dot(t.vij, t.gradWI) + t.workQI);
     if (COMPAT) {
       // the owner's pair acceleration, -m_other*deltaDvDt
-      const V3 pa = vmul(t.dd, t.own ? -t.mj : -I.m);
+      const V3 pa = vmul(t.dd, t.own ? -t.mj : I.m());
       pacc[k] = pa.x;
       pacc[ecap + k] = pa.y;
       pacc[2*ecap + k] = pa.z;
@@ -285,10 +378,9 @@ __global__ void __launch_bounds__(128, SPH_FP64_MIN_BLOCKS) sph_eval_fp64_kernel
     tsubfrom(DvDx, tmul(dyad(t.vij, t.gradWI), t.mj));
 #endif
     if (XSPH) {
-      const double w = 0.5*(I.mrho*t.WI + t.mrhoj*t.WJ);
+      const double w = 0.5*(I.mrho()*t.WI + t.mrhoj*t.WJ);
       XSPHw += w;
-      const V3 dvw = vmul(t.vij, w);
-      XSPHdv = t.own ? vsub(XSPHdv, dvw) : vadd(XSPHdv, dvw);
+      XSPHdv = vsub(XSPHdv, vmul(t.vij, w));
     }
 #if SPH_FP64_SHARED_ACC
     {
@@ -305,82 +397,180 @@ __global__ void __launch_bounds__(128, SPH_FP64_MIN_BLOCKS) sph_eval_fp64_kernel
   for (int64_t k = k0; k < k1; ++k) {
     const int32_t j = __ldg(nbr + k);
     const double fs = BALSARA ? dmax(fsi, MB.fshear[j < n ? (int64_t)j : (int64_t)MB.groot[j - n]]) : 1.0;
-    accumulate(pairTerms<TENSILE>(I, isoI, loadRec(rec, j), j > (int32_t)i, P, P.Cl*(0.5*(1.0 + 1.0)*fs),
+    accumulate(pairTerms<TENSILE>(I, isoI, loadRec(rec, cap, j), j > (int32_t)i, P, P.Cl*(0.5*(1.0 + 1.0)*fs),
                                   P.Cq*(0.5*(1.0 + 1.0)*fs)), k);
   }
 
-  // ---- per-node finish (src/SPH/SPHHydroBase.cc:834-902)
-  const double mi = I.m, rhoi = I.rho, Hdeti = I.Hdet;
-  const int numNeighbors = (int)(k1 - k0);
-  rhoSum += mi*P.W0*Hdeti;
-  norm += mi/rhoi*P.W0*Hdeti;
+  NodeSums t;
+  t.rhoSum = rhoSum; t.norm = norm; t.wns = wns; t.maxvp = maxvp; t.effvp = effvp; t.viscW = viscW; t.DepsDt = DepsDt;
+  t.XSPHw = XSPHw; t.DvDt = DvDt; t.XSPHdv = XSPHdv; t.m2 = m2;
 #if SPH_FP64_SHARED_ACC
-  T9 Mi, DvDxi;
   {
-    double* mi9 = &Mi.xx;
-    double* dv9 = &DvDxi.xx;
+    double* m9 = &t.M.xx;
+    double* dv9 = &t.DvDx.xx;
 #pragma unroll
-    for (int c = 0; c < 9; ++c) { mi9[c] = accM[128*c]; dv9[c] = accDvDx[128*c]; }
+    for (int c = 0; c < 9; ++c) { m9[c] = accM[128*c]; dv9[c] = accDvDx[128*c]; }
   }
 #else
-  T9 Mi = M, DvDxi = DvDx;
+  t.M = M;
+  t.DvDx = DvDx;
 #endif
-  if (P.correctVelGrad && fabs(tdet(Mi)) > 1.0e-10 && numNeighbors > 8) {
-    Mi = tinverse(Mi);
-    DvDxi = tdot(DvDxi, Mi);
-  } else {
-    DvDxi = tdiv(DvDxi, rhoi);
-  }
-  const double DrhoDt = -rhoi*ttrace(DvDxi);
-  wns = dmax(0.0, wns/Hdeti);
-  wns = sgn(wns)*pow(fabs(wns), 0.3333333333333333);          // Dim<3>::rootnu
-  m2 = sdiv(m2, Hdeti*Hdeti);
-  V3 DxDt = I.v;
-  if (XSPH) {
-    XSPHw += Hdeti*mi/rhoi*P.W0;
-    DxDt = vadd(I.v, vdiv(XSPHdv, dmax(1.0e-30, XSPHw)));
-  }
-  const Sym DHDt = smul(sdiv(sneg(I.H), 3.0), ttrace(DvDxi));
-  // SPHSmoothingScale::idealSmoothingScale (src/NodeList/SPHSmoothingScale.cc:118-199)
-  double nPerhCur;
-  if (fuzzyEqual(wns, 0.0)) {
-    nPerhCur = 0.5*P.nPerh;
-  } else {
-    nPerhCur = equivalentNodesPerSmoothingScale(P, wns);
-  }
-  const double s = dmin(4.0, dmax(0.25, P.nPerh/(nPerhCur + 1.0e-30)));
-  const double a = s < 1.0 ? 0.4*(1.0 + s*s) : 0.4*(1.0 + 1.0/(s*s*s));
-  const double hi0 = 1.0/I.H.xx;
-  const double hi1 = dmin(P.hmax, dmax(P.hmin, hi0*(1.0 - a + a*s)));
-  const double hinv = 1.0/hi1;
+  finishNode<XSPH>(P, I, t, (int)(k1 - k0), D + i, n);
+}
 
-  // ---- stores (SoA, coalesced across the warp)
-  double* d = D + i;
-  d[(D_DXDT + 0)*n] = DxDt.x; d[(D_DXDT + 1)*n] = DxDt.y; d[(D_DXDT + 2)*n] = DxDt.z;
-  d[(D_DVDT + 0)*n] = DvDt.x; d[(D_DVDT + 1)*n] = DvDt.y; d[(D_DVDT + 2)*n] = DvDt.z;
-  d[D_DRHODT*n] = DrhoDt;
-  d[D_DEPSDT*n] = DepsDt;
-  d[(D_DHDT + 0)*n] = DHDt.xx; d[(D_DHDT + 1)*n] = DHDt.xy; d[(D_DHDT + 2)*n] = DHDt.xz;
-  d[(D_DHDT + 3)*n] = DHDt.yy; d[(D_DHDT + 4)*n] = DHDt.yz; d[(D_DHDT + 5)*n] = DHDt.zz;
-  d[(D_HIDEAL + 0)*n] = 1.0*hinv; d[(D_HIDEAL + 1)*n] = 0.0*hinv; d[(D_HIDEAL + 2)*n] = 0.0*hinv;
-  d[(D_HIDEAL + 3)*n] = 1.0*hinv; d[(D_HIDEAL + 4)*n] = 0.0*hinv; d[(D_HIDEAL + 5)*n] = 1.0*hinv;
-  const double* dv = &DvDxi.xx;
-  const double* mm = &Mi.xx;
+// The same derivatives with a group of 16 lanes per node, for long rows: the
+// lanes form the terms of 16 consecutive entries, put them into shared memory
+// (a row of 17 doubles per sum), and then each lane adds the 16 terms of its
+// sums (lane l has sums l, l + 16, l + 32) in row order.
+//
+// Why: with a thread per node a row of 115 entries is one serial chain of 115
+// pairs, so a problem of a few thousand nodes takes as long as that chain
+// (300 us) on an almost idle chip, and a large one holds all sums of 32 nodes in
+// a warp's registers and shared memory.  Here the chain is 8 batches of
+// independent pairs, the entries and the stored pair accelerations are read
+// and written coalesced, and the sums take three registers a lane.  Lanes past
+// the end of a row add zeros, which leave every sum's bits (no sum is -0).
+// Measured (B200, Sod, 115 neighbors): 2,048 nodes 298 -> 31 us, 262,144 nodes
+// 1,977 -> 1,817 us; bound by L1 line accesses (63% of their rate) and the
+// latency of the divisions, the FP64 pipe 38% busy.
+constexpr int kRowLanes = 16;
+constexpr int kRowPad = kRowLanes + 1;
+constexpr int kRowGroups = 128/kRowLanes;
+constexpr int kRowMaxNodes = 2;                 // nodes per group of a block, at most
+enum RowSum {
+  RS_WNS = 0, RS_M2 = 1, RS_RHO = 7, RS_NORM = 8, RS_EFFVP = 9, RS_VISCW = 10, RS_DVDT = 11, RS_DEPSDT = 14,
+  RS_DVDX = 15, RS_M = 24, RS_MAXVP = 33, RS_XSPHW = 34, RS_XSPHDV = 35, RS_ALL = 38
+};
+
+template<bool XSPH, bool TENSILE, bool COMPAT, bool SOLO, bool BALSARA>
+__global__ void __launch_bounds__(128, 4) sph_eval_fp64_rows_kernel(const Member* mem, BlockMap bm, const Member single, int nodes) {
+  constexpr int NS = XSPH ? RS_ALL : RS_XSPHW;
+  __shared__ double sT[kRowGroups][NS*kRowPad];
+  __shared__ double sI[kRowGroups][RECW];
+  __shared__ double sF[kRowGroups*kRowMaxNodes][NS + 1];      // (odd stride: the finish reads a node per thread)
+  const MemberBlock mb = memberBlock(bm);
+  const Member& MB = SOLO ? single : mem[mb.m];   // one member: read from the kernel parameters
+  const int64_t n = MB.n;
+  const Params& P = MB.prm;
+  const double* rec = MB.rec;
+  const int64_t cap = MB.candcap;
+  const int32_t* nbr = MB.nbr;
+  double* pacc = MB.pacc;
+  const int64_t ecap = MB.ecap;
+  const int grp = threadIdx.x/kRowLanes, l = threadIdx.x % kRowLanes;
+  const unsigned half = 0xffffu << (threadIdx.x & 16);
+  const int64_t first = mb.block*(int64_t)(kRowGroups*nodes);
+  double* T = sT[grp];
+  for (int q = 0; q < nodes; ++q) {
+    const int64_t i = first + q*kRowGroups + grp;
+    if (i >= n) break;
+    __syncwarp(half);
+    if (l < RECW/2) {
+      const double2 a = __ldg(reinterpret_cast<const double2*>(rec + planeAt(cap, i, l >> 1)) + (l & 1));
+      sI[grp][2*l] = a.x;
+      sI[grp][2*l + 1] = a.y;
+    }
+    __syncwarp(half);
+    const ColumnRec<1> I{sI[grp]};
+    const bool isoI = isoSym(I.H());
+    const double fsi = BALSARA ? MB.fshear[i] : 1.0;
+    double s0 = 0.0, s1 = 0.0, s2 = 0.0;
+    const int64_t k0 = MB.offsets[i], k1 = MB.offsets[i + 1];
+    for (int64_t base = k0; base < k1; base += kRowLanes) {
+      const int64_t k = base + l;
+      double* o = T + l;
+      if (k < k1) {
+        const int32_t j = __ldg(nbr + k);
+        const double fs = BALSARA ? dmax(fsi, MB.fshear[j < n ? (int64_t)j : (int64_t)MB.groot[j - n]]) : 1.0;
+        // Cl *= 0.5*(fCli + fClj)*fshear, as in sph_eval_fp64_kernel
+        const PairTerms t = pairTerms<TENSILE>(I, isoI, loadRec(rec, cap, j), j > (int32_t)i, P,
+                                               P.Cl*(0.5*(1.0 + 1.0)*fs), P.Cq*(0.5*(1.0 + 1.0)*fs));
+        o[RS_WNS*kRowPad] = 1.0*fabs(t.gWI);
+        {
+          const double g2 = 1.0*mag2(t.gradWI);
+          const Sym m2 = smul(smul(selfdyad(t.rij), t.thptS), g2);
+          const double* m = &m2.xx;
 #pragma unroll
-  for (int c = 0; c < 9; ++c) {
-    d[(D_DVDX + c)*n] = dv[c];
-    d[(D_M + c)*n] = mm[c];
+          for (int c = 0; c < 6; ++c) o[(RS_M2 + c)*kRowPad] = m[c];
+        }
+        o[RS_RHO*kRowPad] = t.mj*t.WI;
+        o[RS_NORM*kRowPad] = I.mrho()*t.WI;
+        o[RS_EFFVP*kRowPad] = t.mrhoj*t.QI*t.WI;
+        o[RS_VISCW*kRowPad] = t.mj*t.workQI;
+        o[RS_MAXVP*kRowPad] = t.QI;
+        const V3 a = vmul(t.dd, -t.mj);
+        o[(RS_DVDT + 0)*kRowPad] = a.x; o[(RS_DVDT + 1)*kRowPad] = a.y; o[(RS_DVDT + 2)*kRowPad] = a.z;
+        o[RS_DEPSDT*kRowPad] = t.mj*(t.PrhoI*dot(t.vij, t.gradWI) + t.workQI);
+        if (COMPAT) {
+          // the owner's pair acceleration, -m_other*deltaDvDt
+          const V3 pa = t.own ? a : vmul(t.dd, I.m());
+          pacc[k] = pa.x;
+          pacc[ecap + k] = pa.y;
+          pacc[2*ecap + k] = pa.z;
+        }
+        const double va[3] = {t.vij.x, t.vij.y, t.vij.z}, ra[3] = {t.rij.x, t.rij.y, t.rij.z};
+        const double ga[3] = {t.gradWI.x, t.gradWI.y, t.gradWI.z};
+#pragma unroll
+        for (int r = 0; r < 3; ++r)
+#pragma unroll
+          for (int c = 0; c < 3; ++c) {
+            o[(RS_DVDX + 3*r + c)*kRowPad] = (va[r]*ga[c])*-t.mj;
+            o[(RS_M + 3*r + c)*kRowPad] = (ra[r]*ga[c])*-t.mj;
+          }
+        if (XSPH) {
+          const double w = 0.5*(I.mrho()*t.WI + t.mrhoj*t.WJ);
+          const V3 dv = vmul(t.vij, -w);
+          o[RS_XSPHW*kRowPad] = w;
+          o[(RS_XSPHDV + 0)*kRowPad] = dv.x; o[(RS_XSPHDV + 1)*kRowPad] = dv.y; o[(RS_XSPHDV + 2)*kRowPad] = dv.z;
+        }
+      } else {
+#pragma unroll
+        for (int c = 0; c < NS; ++c) o[c*kRowPad] = 0.0;
+      }
+      __syncwarp(half);
+      const double* t0 = T + l*kRowPad;
+      const double* t1 = t0 + kRowLanes*kRowPad;
+#pragma unroll
+      for (int e = 0; e < kRowLanes; ++e) {
+        s0 += t0[e];
+        s1 += t1[e];
+      }
+      if (l < NS - 2*kRowLanes) {
+        const double* t2 = t1 + kRowLanes*kRowPad;
+        if (l == RS_MAXVP - 2*kRowLanes) {
+#pragma unroll
+          for (int e = 0; e < kRowLanes; ++e) s2 = dmax(s2, t2[e]);
+        } else {
+#pragma unroll
+          for (int e = 0; e < kRowLanes; ++e) s2 += t2[e];
+        }
+      }
+      __syncwarp(half);
+    }
+    double* F = sF[q*kRowGroups + grp];
+    F[l] = s0;
+    F[l + kRowLanes] = s1;
+    if (l < NS - 2*kRowLanes) F[l + 2*kRowLanes] = s2;
   }
-  d[D_RHOSUM*n] = rhoSum;
-  d[D_NORM*n] = norm;
-  d[D_WNS*n] = wns;
-  d[(D_M2 + 0)*n] = m2.xx; d[(D_M2 + 1)*n] = m2.xy; d[(D_M2 + 2)*n] = m2.xz;
-  d[(D_M2 + 3)*n] = m2.yy; d[(D_M2 + 4)*n] = m2.yz; d[(D_M2 + 5)*n] = m2.zz;
-  d[D_XSPHW*n] = XSPHw;
-  d[(D_XSPHDV + 0)*n] = XSPHdv.x; d[(D_XSPHDV + 1)*n] = XSPHdv.y; d[(D_XSPHDV + 2)*n] = XSPHdv.z;
-  d[D_MAXVP*n] = maxvp;
-  d[D_EFFVP*n] = effvp;
-  d[D_VISCW*n] = viscW;
+  __syncthreads();
+  // the finish, a thread per node of the block
+  const int64_t i = first + threadIdx.x;
+  if ((int)threadIdx.x >= kRowGroups*nodes || i >= n) return;
+  const double* F = sF[threadIdx.x];
+  NodeSums t;
+  t.rhoSum = F[RS_RHO]; t.norm = F[RS_NORM]; t.wns = F[RS_WNS]; t.maxvp = F[RS_MAXVP]; t.effvp = F[RS_EFFVP];
+  t.viscW = F[RS_VISCW]; t.DepsDt = F[RS_DEPSDT];
+  t.DvDt = V3{F[RS_DVDT], F[RS_DVDT + 1], F[RS_DVDT + 2]};
+  t.XSPHw = XSPH ? F[RS_XSPHW] : 0.0;
+  t.XSPHdv = XSPH ? V3{F[RS_XSPHDV], F[RS_XSPHDV + 1], F[RS_XSPHDV + 2]} : V3{0.0, 0.0, 0.0};
+  t.m2 = Sym{F[RS_M2], F[RS_M2 + 1], F[RS_M2 + 2], F[RS_M2 + 3], F[RS_M2 + 4], F[RS_M2 + 5]};
+  double* dv9 = &t.DvDx.xx;
+  double* m9 = &t.M.xx;
+#pragma unroll
+  for (int c = 0; c < 9; ++c) { dv9[c] = F[RS_DVDX + c]; m9[c] = F[RS_M + c]; }
+  double own[RECW];
+  ldPlanes<RECW/4>(rec, cap, i, own);
+  finishNode<XSPH>(P, ColumnRec<1>{own}, t, (int)(MB.offsets[i + 1] - MB.offsets[i]), MB.D + i, n);
 }
 
 // ---------------------------------------------------------------- grad-h
@@ -392,18 +582,20 @@ __global__ void __launch_bounds__(128) gradh_kernel(const Member* mem, BlockMap 
   if (i >= n) return;
   const Params& P = MB.prm;
   const double* rec = MB.rec;
+  const int64_t cap = MB.candcap;
   const int32_t* nbr = MB.nbr;
   double* S = MB.S;
   const int64_t k0 = MB.offsets[i], k1 = MB.offsets[i + 1];
   if (k1 == k0) { S[S_OMEGA*n + i] = 1.0; return; }
-  const Rec I = loadRec(rec, i);
+  const Rec I = loadRec(rec, cap, i);
   const double W0 = tableKernel(P.W, 0.0, I.Hdet);
   double omega = 0.0, gradsum = 0.0;
   bool selfDone = false;
   for (int64_t k = k0; k < k1; ++k) {
     const int32_t j = __ldg(nbr + k);
     if (!selfDone && j > (int32_t)i) { omega += W0; selfDone = true; }
-    const V3 rj{ldg(rec + (int64_t)j*RECW + R_X), ldg(rec + (int64_t)j*RECW + R_Y), ldg(rec + (int64_t)j*RECW + R_Z)};
+    const D4 pj = ldPlane(rec + planeAt(cap, j, 0));
+    const V3 rj{pj.a, pj.b, pj.c};
     const V3 rij = vsub(I.r, rj);
     const double eta = mag(sdot(I.H, rij));
     double W, gW;
@@ -455,9 +647,11 @@ __global__ void __launch_bounds__(128) sum_density_kernel(const Member* mem, Blo
   if (i >= n) return;
   const Params& P = MB.prm;
   const double* rec = MB.rec;
+  const int64_t cap = MB.candcap;
   const int32_t* nbr = MB.nbr;
-  const V3 ri{ldg(rec + i*RECW + R_X), ldg(rec + i*RECW + R_Y), ldg(rec + i*RECW + R_Z)};
-  const double mi = ldg(rec + i*RECW + R_M), Hdeti = ldg(rec + i*RECW + R_HDET);
+  const D4 pi = ldPlane(rec + planeAt(cap, i, 0));
+  const V3 ri{pi.a, pi.b, pi.c};
+  const double mi = pi.d, Hdeti = ldg(rec + planeAt(cap, i, 1));
   const double W0 = tableKernel(P.W, 0.0, Hdeti);
   double rho = 0.0;
   bool selfDone = false;
@@ -465,7 +659,7 @@ __global__ void __launch_bounds__(128) sum_density_kernel(const Member* mem, Blo
   for (int64_t k = k0; k < k1; ++k) {
     const int32_t j = __ldg(nbr + k);
     if (!selfDone && j > (int32_t)i) { rho += mi*W0; selfDone = true; }
-    const Rec J = loadRec(rec, j);
+    const Rec J = loadRec(rec, cap, j);
     const V3 rij = vsub(ri, J.r);
     const double eta = mag(isoSym(J.H) ? vmul(rij, J.H.xx) : sdot(J.H, rij));
     rho += J.m*tableKernel(P.W, eta, J.Hdet);
@@ -517,29 +711,27 @@ __global__ void __launch_bounds__(128) sum_density_mixed_kernel(const Member* me
   const double* mrec = MB.mrec;
   const int32_t* nbr = MB.nbr;
   const float invStep = (float)(1.0/P.W.stepSize), extent = (float)P.W.extent;
-  const double2* qi = reinterpret_cast<const double2*>(mrec + i*MRECW);
-  const double2 a0 = __ldg(qi), a1 = __ldg(qi + 1);
-  const float4 bi = __ldg(reinterpret_cast<const float4*>(qi + 3));
-  const float W0 = tableW32(coefF, P.W.n, invStep, extent, 0.0f, bi.w);
+  const int64_t cap = MB.candcap;
+  const D4 pi = ldPlane(mrec + planeAt(cap, i, 0)), vi = ldPlane(mrec + planeAt(cap, i, 1));
+  const float mi = loF(vi.c), Hdeti = hiF(vi.d);
+  const float W0 = tableW32(coefF, P.W.n, invStep, extent, 0.0f, Hdeti);
   KahanSum rho{0.0f, 0.0f};
   bool selfDone = false;
   const int64_t k0 = MB.offsets[i], k1 = MB.offsets[i + 1];
   for (int64_t k = k0; k < k1; ++k) {
     const int32_t j = __ldg(nbr + k);
-    if (!selfDone && j > (int32_t)i) { rho.add(bi.x*W0); selfDone = true; }
-    const double2* q = reinterpret_cast<const double2*>(mrec + (int64_t)j*MRECW);
-    const double2 c0 = __ldg(q), c1 = __ldg(q + 1);
-    const float4* f = reinterpret_cast<const float4*>(q + 3);
-    const float4 f0 = __ldg(f), f1 = __ldg(f + 1);
-    const float2 f2 = __ldg(reinterpret_cast<const float2*>(f + 2));
-    const float rx = (float)(a0.x - c0.x), ry = (float)(a0.y - c0.y), rz = (float)(a1.x - c1.x);
-    const float ex = f1.x*rx + f1.y*ry + f1.z*rz;
-    const float ey = f1.y*rx + f1.w*ry + f2.x*rz;
-    const float ez = f1.z*rx + f2.x*ry + f2.y*rz;
+    if (!selfDone && j > (int32_t)i) { rho.add(mi*W0); selfDone = true; }
+    const D4 p = ldPlane(mrec + planeAt(cap, j, 0)), f0 = ldPlane(mrec + planeAt(cap, j, 1)),
+             h = ldPlane(mrec + planeAt(cap, j, 2));
+    const float rx = (float)(pi.a - p.a), ry = (float)(pi.b - p.b), rz = (float)(pi.c - p.c);
+    const float xx = loF(h.a), xy = hiF(h.a), xz = loF(h.b), yy = hiF(h.b), yz = loF(h.c), zz = hiF(h.c);
+    const float ex = xx*rx + xy*ry + xz*rz;
+    const float ey = xy*rx + yy*ry + yz*rz;
+    const float ez = xz*rx + yz*ry + zz*rz;
     const float eta = sqrtf(ex*ex + ey*ey + ez*ez);
-    rho.add(f0.x*tableW32(coefF, P.W.n, invStep, extent, eta, f0.w));
+    rho.add(loF(f0.c)*tableW32(coefF, P.W.n, invStep, extent, eta, hiF(f0.d)));
   }
-  if (!selfDone) rho.add(bi.x*W0);
+  if (!selfDone) rho.add(mi*W0);
   MB.S[S_RHO*n + i] = rho.value();
   if (enforce) enforceNode(MB, i);
 }
@@ -738,8 +930,8 @@ __global__ void __launch_bounds__(128, SPH_UPDATE_MIN_BLOCKS) update_kernel(cons
                     (packMode == 1 ? !P.gradh : P.densityUpdate == SPHGPU_DENSITY_RIGOROUS_SUM);
   if (pack) {
     const double omega = S[S_OMEGA*n + i];
-    if (P.precision == SPHGPU_PRECISION_MIXED) writeMixedRecord(MB.mrec, i, x, v, m, rho, csn, Pn, omega, Hn);
-    else writeRecord(MB.rec, i, x, v, m, rho, csn, Pn, omega, Hn);
+    if (P.precision == SPHGPU_PRECISION_MIXED) writeMixedRecord(MB.mrec, MB.candcap, i, x, v, m, rho, csn, Pn, omega, Hn);
+    else writeRecord(MB.rec, MB.candcap, i, x, v, m, rho, csn, Pn, omega, Hn);
   }
 }
 
@@ -1115,13 +1307,34 @@ int launch_gradh(Batch& b) {
   return cuda_status(cudaGetLastError(), "gradh");
 }
 
-// One launch of the FP64 pair kernel variant <XSPH, TENSILE, COMPAT, BALSARA>.
-template<bool X, bool T, bool C, bool B>
-void launch_fp64_variant(Batch& b, unsigned grid, BlockMap bm, const Member& one, bool solo) {
-  if (solo) sph_eval_fp64_kernel<X, T, C, true, B><<<grid, b.evalThreads, 0, b.stream>>>(b.d_mem, bm, one);
-  else sph_eval_fp64_kernel<X, T, C, false, B><<<grid, b.evalThreads, 0, b.stream>>>(b.d_mem, bm, one);
+// Members whose rows are long enough for a group of lanes per node: a row
+// of 32 entries fills its batches of 16 to three quarters on average, and
+// below that the thread-per-node kernel's full lanes win (7.8 entries of
+// Kelvin-Helmholtz: two batches would be half empty).
+constexpr int64_t kLongRow = 32;
+bool longRows(const Problem& p) { return p.E >= kLongRow*p.n; }
+
+// Nodes per group of the row kernel: as many as leave two waves of blocks.
+int row_nodes(int64_t nodes) {
+  int q = kRowMaxNodes;
+  while (q > 1 && nodes < (int64_t)kRowGroups*q*148*8) q >>= 1;
+  return q;
 }
-using Fp64Launch = void (*)(Batch&, unsigned, BlockMap, const Member&, bool);
+
+// One launch of the FP64 pair kernel variant <XSPH, TENSILE, COMPAT, BALSARA>;
+// nodes > 0: of the row kernel.
+template<bool X, bool T, bool C, bool B>
+void launch_fp64_variant(Batch& b, unsigned grid, BlockMap bm, const Member& one, bool solo, int nodes) {
+  if (nodes > 0) {
+    if (solo) sph_eval_fp64_rows_kernel<X, T, C, true, B><<<grid, 128, 0, b.stream>>>(b.d_mem, bm, one, nodes);
+    else sph_eval_fp64_rows_kernel<X, T, C, false, B><<<grid, 128, 0, b.stream>>>(b.d_mem, bm, one, nodes);
+  } else if (solo) {
+    sph_eval_fp64_kernel<X, T, C, true, B><<<grid, b.evalThreads, 0, b.stream>>>(b.d_mem, bm, one);
+  } else {
+    sph_eval_fp64_kernel<X, T, C, false, B><<<grid, b.evalThreads, 0, b.stream>>>(b.d_mem, bm, one);
+  }
+}
+using Fp64Launch = void (*)(Batch&, unsigned, BlockMap, const Member&, bool, int);
 // indexed by BALSARA << 3 | XSPH << 2 | TENSILE << 1 | COMPAT
 const Fp64Launch kFp64Launch[16] = {
     &launch_fp64_variant<false, false, false, false>, &launch_fp64_variant<false, false, true, false>,
@@ -1142,14 +1355,20 @@ int launch_eval_sph_fp64(Batch& b) {
   const Member one = solo ? describe_member(*b.mem[0]) : Member{};
   bool present[16] = {};
   for (Problem* p : b.mem) if (isFp64Sph(*p)) present[key(*p)] = true;
-  for (int v = 0; v < 16; ++v) {
-    if (!present[v]) continue;
+  for (int v = 0; v < 32; ++v) {
+    const bool rows = (v & 16) != 0;
+    if (!present[v & 15]) continue;
+    auto mine = [&](const Problem& p) { return isFp64Sph(p) && key(p) == (v & 15) && longRows(p) == rows; };
+    int64_t total = 0;
+    for (Problem* p : b.mem) total += mine(*p) ? p->n : 0;
+    if (total == 0) continue;
+    const int nodes = rows ? row_nodes(total) : 0;
     BlockMap bm;
     unsigned grid = 0;
-    SPH_TRY(batch_map_items(b, [&](const Problem& p) { return isFp64Sph(p) && key(p) == v ? p.n : (int64_t)0; },
-                            b.evalThreads, &bm, &grid));
+    SPH_TRY(batch_map_items(b, [&](const Problem& p) { return mine(p) ? p.n : (int64_t)0; },
+                            rows ? kRowGroups*nodes : b.evalThreads, &bm, &grid));
     if (!grid) continue;
-    kFp64Launch[v](b, grid, bm, one, solo);
+    kFp64Launch[v & 15](b, grid, bm, one, solo, nodes);
     batch_count_launch(b);
   }
   return cuda_status(cudaGetLastError(), "evaluate (FP64)");

@@ -37,17 +37,16 @@ struct MRec {
   float iso;           // 1: H = hxx I (the symmetric products reduce to scalings)
 };
 
-__device__ __forceinline__ MRec loadMRec(const double* mrec, int64_t k) {
-  const double2* q = reinterpret_cast<const double2*>(mrec + k*MRECW);
-  const double2 a0 = __ldg(q), a1 = __ldg(q + 1), a2 = __ldg(q + 2);
-  const float4* f = reinterpret_cast<const float4*>(q + 3);
-  const float4 b0 = __ldg(f), b1 = __ldg(f + 1), b2 = __ldg(f + 2), b3 = __ldg(f + 3);
+__device__ __forceinline__ MRec loadMRec(const double* mrec, int64_t cap, int64_t k) {
+  double a[MRECW];
+  ldPlanes<MRECW/4, true>(mrec, cap, k, a);
   MRec R;
-  R.x = a0.x; R.y = a0.y; R.z = a1.x; R.vx = a1.y; R.vy = a2.x; R.vz = a2.y;
-  R.m = b0.x; R.rho = b0.y; R.cs = b0.z; R.Hdet = b0.w;
-  R.hxx = b1.x; R.hxy = b1.y; R.hxz = b1.z; R.hyy = b1.w;
-  R.hyz = b2.x; R.hzz = b2.y; R.Prho = b2.z; R.mrho = b2.w;
-  R.P = b3.x; R.somega = b3.y; R.iso = b3.z;
+  // the layout of writeMixedRecord (problem.cuh)
+  R.x = a[0]; R.y = a[1]; R.z = a[2]; R.vx = a[3]; R.vy = a[4]; R.vz = a[5];
+  R.m = loF(a[6]); R.rho = hiF(a[6]); R.cs = loF(a[7]); R.Hdet = hiF(a[7]);
+  R.hxx = loF(a[8]); R.hxy = hiF(a[8]); R.hxz = loF(a[9]); R.hyy = hiF(a[9]);
+  R.hyz = loF(a[10]); R.hzz = hiF(a[10]); R.Prho = loF(a[11]); R.mrho = hiF(a[11]);
+  R.P = loF(a[12]); R.somega = hiF(a[12]); R.iso = loF(a[13]);
   return R;
 }
 
@@ -94,13 +93,14 @@ __global__ void __launch_bounds__(128, SPH_MIXED_MIN_BLOCKS) sph_eval_mixed_kern
   const Params& P = MB.prm;
   const float* coefF = MB.coefF;
   const double* mrec = MB.mrec;
+  const int64_t cap = MB.candcap;
   const double* S = MB.S;
   const int64_t* offsets = MB.offsets;
   const int32_t* nbr = MB.nbr;
   double* D = MB.D;
   double* pacc = MB.pacc;
   const int64_t ecap = MB.ecap;
-  const MRec I = loadMRec(mrec, i);
+  const MRec I = loadMRec(mrec, cap, i);
   const float invStep = (float)(1.0/P.W.stepSize), extent = (float)P.W.extent;
   const float eps2 = (float)P.eps2;
   const float Cl = (float)P.Cl, Cq = (float)P.Cq;
@@ -118,7 +118,7 @@ __global__ void __launch_bounds__(128, SPH_MIXED_MIN_BLOCKS) sph_eval_mixed_kern
   const int64_t k0 = offsets[i], k1 = offsets[i + 1];
   for (int64_t k = k0; k < k1; ++k) {
     const int32_t j = __ldg(nbr + k);
-    const MRec J = loadMRec(mrec, j);
+    const MRec J = loadMRec(mrec, cap, j);
     // the Balsara shear correction of the pair (max of the two nodes'), else 1
     const float fs = BALSARA ? fmaxf(fsi, (float)MB.fshear[j < n ? (int64_t)j : (int64_t)MB.groot[j - n]]) : 1.0f;
     const float ClP = Cl*fs, CqP = Cq*fs;

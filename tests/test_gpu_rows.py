@@ -1,0 +1,46 @@
+"""The group-of-lanes FP64 pair kernel (rows of 32 entries and more) at the edges
+of its batches of 16 entries and its blocks of 8 and 16 nodes.  It forms the
+same terms and adds them in the same order as the oracle, so every derivative
+is bit-equal except the cube root of the ideal-H moment (CUDA pow against
+glibc pow, 2 ulp: 1e-12 is the specification's tolerance)."""
+import numpy as np
+import pytest
+
+from conftest import normwise
+
+pytestmark = pytest.mark.gpu
+
+KEYS = ["delta velocity hydro", "delta specific thermal energy", "delta mass density", "new mass density",
+        "normalization", "velocity gradient", "M SPH gradient correction", "mass second moment",
+        "max viscous pressure", "effective viscous pressure", "viscous work rate", "XSPH weight sum",
+        "XSPH delta vi"]
+
+
+# nodes: one block short of its last group, odd counts, one node more than a block of 8 and of 16
+@pytest.mark.parametrize("keep", [512, 505, 497, 449])
+@pytest.mark.parametrize("options", [{}, {"XSPH": 1}, {"epsTensile": 0.3, "compatibleEnergyEvolution": 0},
+                                     {"balsaraShearCorrection": 1}])
+def test_rows(gpu_lib, pkg, oracle_mod, keep, options):
+    gen, abi = pkg.generators, pkg.abi
+    ns = gen.kelvin_helmholtz(nx=8, ny=8, nz=8, jitter=0.2, seed=keep)
+    sel = np.sort(np.random.default_rng(keep).permutation(ns.n)[:keep])
+    # rows of about 30 to 150 entries: smoothing scales spread by 1.7
+    h = np.random.default_rng(keep + 1).uniform(0.13, 0.22, keep)
+    H = np.zeros((keep, 6))
+    H[:, [0, 3, 5]] = 1.0 / h[:, None]
+    ns = gen.NodeSet(ns.pos[sel], ns.vel[sel], ns.mass[sel], ns.rho[sel], ns.eps[sel], H, ns.dx)
+    cfg = gen.kh_config(abi, kernel=abi.KERNEL_BSPLINE, **options)
+    g, o = pkg.SPHHydro(cfg, ns), oracle_mod.OracleProblem(cfg, ns)
+    for p in (g, o):
+        p.build_neighbors()
+    off, _, _ = g.connectivity()
+    rows = np.diff(off)
+    assert rows.mean() >= 32 and len(set((rows % 16).tolist())) == 16      # every remainder of a batch
+    if options.get("balsaraShearCorrection"):
+        # the correction reads the last evaluation's velocity gradient
+        g.initialize(), o.initialize()
+    g.evaluateDerivatives()
+    o.evaluate_derivatives()
+    for k in KEYS:
+        assert np.array_equal(g.field(k), o.field(k)), k
+    assert normwise(g.field("new H"), o.field("new H")) <= 1e-12
