@@ -40,6 +40,13 @@
 #ifndef SPH_MIXED_MIN_BLOCKS
 #define SPH_MIXED_MIN_BLOCKS 3
 #endif
+// the kernels with a group of lanes per node
+#ifndef SPH_ROWS_MIN_BLOCKS
+#define SPH_ROWS_MIN_BLOCKS 4
+#endif
+#ifndef SPH_MIXED_ROWS_MIN_BLOCKS
+#define SPH_MIXED_ROWS_MIN_BLOCKS 4
+#endif
 // 1: ... and accumulates its two tensor sums there
 #ifndef SPH_FP64_SHARED_ACC
 #define SPH_FP64_SHARED_ACC 1
@@ -59,6 +66,9 @@ enum StateField {
 // updates it every full update), and S_EPS holds the specific thermal energy
 // at the start of the last step (the reference's specificThermalEnergy0).
 constexpr int S0_ENTROPY = S_M;
+// ... and the pressure column the compatible energy's rates between its kernel
+// and the full update of the same step.
+constexpr int S0_RATE = S_P;
 
 // CRKSPH corrections and moments of the internal nodes, SoA [NCRK][n].
 enum CrkField {
@@ -684,6 +694,20 @@ int cuda_status(cudaError_t e, const char* where);
     const int rc__ = (expr);                                            \
     if (rc__ != SPHGPU_OK) return rc__;                                 \
   } while (0)
+
+// Members whose rows are long enough for a group of lanes per node in the SPH
+// pair kernels: a row of 32 entries fills its batches of 16 to three quarters
+// on average, and below that the thread-per-node kernels' full lanes win (the
+// 7.8 entries of Kelvin-Helmholtz leave half of two batches empty).
+constexpr int64_t kLongRow = 32;
+inline bool longRows(const Problem& p) { return p.E >= kLongRow*p.n; }
+constexpr int kRowMaxNodes = 2;       // nodes per group of a block, at most
+// Nodes per group: as many as leave two waves of blocks of 8 groups.
+inline int rowNodes(int64_t nodes) {
+  int q = kRowMaxNodes;
+  while (q > 1 && nodes < (int64_t)8*q*148*8) q >>= 1;
+  return q;
+}
 
 // host TableKernel construction (table.cc)
 void build_table_kernel(int kernelType, int numPoints, std::vector<double>& coef6, std::vector<double>& nperh,

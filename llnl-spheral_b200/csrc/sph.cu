@@ -436,14 +436,13 @@ __global__ void __launch_bounds__(128, SPH_FP64_MIN_BLOCKS) sph_eval_fp64_kernel
 constexpr int kRowLanes = 16;
 constexpr int kRowPad = kRowLanes + 1;
 constexpr int kRowGroups = 128/kRowLanes;
-constexpr int kRowMaxNodes = 2;                 // nodes per group of a block, at most
 enum RowSum {
   RS_WNS = 0, RS_M2 = 1, RS_RHO = 7, RS_NORM = 8, RS_EFFVP = 9, RS_VISCW = 10, RS_DVDT = 11, RS_DEPSDT = 14,
   RS_DVDX = 15, RS_M = 24, RS_MAXVP = 33, RS_XSPHW = 34, RS_XSPHDV = 35, RS_ALL = 38
 };
 
 template<bool XSPH, bool TENSILE, bool COMPAT, bool SOLO, bool BALSARA>
-__global__ void __launch_bounds__(128, 4) sph_eval_fp64_rows_kernel(const Member* mem, BlockMap bm, const Member single, int nodes) {
+__global__ void __launch_bounds__(128, SPH_ROWS_MIN_BLOCKS) sph_eval_fp64_rows_kernel(const Member* mem, BlockMap bm, const Member single, int nodes) {
   constexpr int NS = XSPH ? RS_ALL : RS_XSPHW;
   __shared__ double sT[kRowGroups][NS*kRowPad];
   __shared__ double sI[kRowGroups][RECW];
@@ -636,6 +635,83 @@ __device__ __forceinline__ void enforceNode(const Member& MB, int64_t i) {
   S[S_X*n + i] = r.x; S[S_Y*n + i] = r.y; S[S_Z*n + i] = r.z;
 }
 
+// ---------------------------------------------------------------- row sums
+// Loops that add one term per entry (summed density, compatible energy) or take
+// its maximum (the dt vote), for small problems: a warp takes a run of
+// consecutive rows, whose entries are consecutive.  Its lanes form the terms
+// of 32 entries at a time into shared memory, then lane r adds the terms of
+// row r in row order.
+//
+// Why: with a thread per node every entry is a step of a serial chain of
+// dependent loads, 115 of them for a Sod node, and a few thousand nodes leave
+// the chip idle meanwhile.  Here only the addition is serial.  It costs more
+// instructions per entry (finding the row, the stores and loads of the terms,
+// few lanes adding), so the thread-per-node kernels are the faster ones once
+// the nodes fill the chip.  Measured (B200), thread per node -> rows, 4,096
+// Sod nodes: summed density (mixed) 61 -> 20 us, compatible energy 112 -> 16,
+// dt vote 59 -> 14; 262,144 nodes: dt vote 179 -> 391 us, Kelvin-Helmholtz with
+// 124,550 nodes of 7 entries: 16 -> 20.  The lines cross near 40,000 nodes (useRowSums).
+// The rows per warp follow the grid: as many as fill the chunk, fewer while
+// that leaves less than 16 warps per SM.
+constexpr int kSumThreads = 256;
+constexpr int kSumWarps = kSumThreads/32;
+constexpr int kSumChunk = 512;                 // terms of a warp in shared memory
+
+struct RowRun {
+  int64_t i0, e0;       // first node, its first entry
+  int rows, total;      // rows of the run, their entries
+  int rel, next;        // this lane's row: first entry and end, counted from e0
+};
+
+// rows per warp of a member in this launch (at most 32: the host's grids see to it)
+__device__ __forceinline__ int rowsPerWarp(int64_t n, int blocks) {
+  const int64_t warps = (int64_t)blocks*kSumWarps, r = (n + warps - 1)/warps;
+  return r > 32 ? 32 : (int)r;
+}
+
+__device__ __forceinline__ RowRun rowRun(const Member& MB, int64_t i0, int rowsMax) {
+  const int lane = threadIdx.x & 31;
+  RowRun R;
+  R.i0 = i0;
+  R.rows = MB.n - i0 < rowsMax ? (int)(MB.n - i0) : rowsMax;
+  const int64_t at = MB.offsets[i0 + (lane < R.rows ? lane : R.rows)];
+  R.e0 = __shfl_sync(0xffffffffu, at, 0);
+  R.total = (int)(MB.offsets[i0 + R.rows] - R.e0);
+  R.rel = (int)(at - R.e0);
+  const int nx = __shfl_down_sync(0xffffffffu, R.rel, 1);
+  R.next = lane == 31 ? R.total : nx;
+  return R;
+}
+
+// term(t, r, start): the term of the run's entry t, row r (which starts at
+// entry start); begin(): before the chunk's additions; step(t, v): entry t of
+// the lane's row has the term v.
+template<class V, class Term, class Begin, class Step>
+__device__ __forceinline__ void rowSums(const RowRun& R, V* buf, Term term, Begin begin, Step step) {
+  const int lane = threadIdx.x & 31;
+  const int top = R.rows > 1 ? 1 << (31 - __clz(R.rows - 1)) : 0;
+  for (int c0 = 0; c0 < R.total; c0 += kSumChunk) {
+    const int c1 = R.total - c0 < kSumChunk ? R.total : c0 + kSumChunk;
+    for (int b = c0; b < c1; b += 32) {
+      const int t = b + lane < c1 ? b + lane : c1 - 1;
+      int r = 0;                                    // the last row that starts at or before t
+      for (int w = top; w > 0; w >>= 1) {
+        const int s = __shfl_sync(0xffffffffu, R.rel, (r + w) & 31);
+        if (r + w < R.rows && s <= t) r += w;
+      }
+      const int start = __shfl_sync(0xffffffffu, R.rel, r);
+      if (b + lane < c1) buf[t - c0] = term(t, r, start);
+    }
+    __syncwarp();
+    if (lane < R.rows) {
+      begin();
+      const int z = R.next < c1 ? R.next : c1;
+      for (int k = R.rel > c0 ? R.rel : c0; k < z; ++k) step(k, buf[k - c0]);
+    }
+    __syncwarp();
+  }
+}
+
 // enforce: also wrap the node's position through the periodic planes (the
 // step's enforceBoundaries, which follows the summed density; the pair
 // terms read positions from the records, never from the state)
@@ -669,6 +745,55 @@ __global__ void __launch_bounds__(128) sum_density_kernel(const Member* mem, Blo
   if (enforce) enforceNode(MB, i);
 }
 
+// The same with a warp per run of rows (rowSums).
+__global__ void __launch_bounds__(kSumThreads) sum_density_rows_kernel(const Member* mem, BlockMap bm, int enforce) {
+  __shared__ double buf[kSumWarps][kSumChunk];
+  __shared__ int selfAt[kSumWarps][32];           // entry of each row before which the self term is added
+  const MemberBlock mb = memberBlock(bm);
+  const Member& MB = mem[mb.m];
+  const int64_t n = MB.n, cap = MB.candcap;
+  const TableDev W = MB.prm.W;
+  const double* rec = MB.rec;
+  const int32_t* nbr = MB.nbr;
+  const int lane = threadIdx.x & 31, wib = threadIdx.x >> 5;
+  const int rowsMax = rowsPerWarp(n, mb.blocks);
+  const int64_t stride = (int64_t)mb.blocks*kSumWarps*rowsMax;
+  for (int64_t i0 = (mb.block*kSumWarps + wib)*rowsMax; i0 < n; i0 += stride) {
+    const RowRun R = rowRun(MB, i0, rowsMax);
+    selfAt[wib][lane] = R.next;
+    __syncwarp();
+    double self = 0.0;
+    if (lane < R.rows) {
+      const double mi = ldg(rec + planeAt(cap, i0 + lane, 0) + R_M), Hdeti = ldg(rec + planeAt(cap, i0 + lane, 1));
+      self = mi*tableKernel(W, 0.0, Hdeti);
+    }
+    double rho = 0.0;
+    int sa = R.next;
+    rowSums(R, buf[wib],
+            [&](int t, int r, int start) {
+              const int64_t e = R.e0 + t;
+              const int32_t j = __ldg(nbr + e), i = (int32_t)(i0 + r);
+              if (j > i && (t == start || __ldg(nbr + e - 1) < i)) selfAt[wib][r] = t;
+              const D4 pi = ldPlane(rec + planeAt(cap, i, 0));
+              const Rec J = loadRec(rec, cap, j);
+              const V3 rij = vsub(V3{pi.a, pi.b, pi.c}, J.r);
+              const double eta = mag(isoSym(J.H) ? vmul(rij, J.H.xx) : sdot(J.H, rij));
+              return J.m*tableKernel(W, eta, J.Hdet);
+            },
+            [&]() { sa = selfAt[wib][lane]; },
+            [&](int t, double v) {
+              if (t == sa) rho += self;
+              rho += v;
+            });
+    if (lane < R.rows) {
+      if (sa == R.next) rho += self;              // no entry above the node
+      MB.S[S_RHO*n + i0 + lane] = rho;
+      if (enforce) enforceNode(MB, i0 + lane);
+    }
+    __syncwarp();
+  }
+}
+
 // ---------------------------------------------------------------- summed density, mixed form
 struct KahanSum {
   float s, c;
@@ -699,7 +824,7 @@ __device__ __forceinline__ float tableW32(const float* coef, int n, float invSte
 // RigorousSumDensity, mixed form: rho_i = m_i W(0) + sum_j m_j W(|H_j r_ij|)
 // with the pair terms in FP32 (r_ij formed in FP64, rounded once) and a
 // Kahan-compensated FP32 sum, from the mixed records of the end-of-step
-// state.  enforce as for sum_density_kernel.
+// state.  enforce as for sum_density_rows_kernel.
 __global__ void __launch_bounds__(128) sum_density_mixed_kernel(const Member* mem, BlockMap bm, int enforce) {
   const MemberBlock mb = memberBlock(bm);
   const Member& MB = mem[mb.m];
@@ -734,6 +859,63 @@ __global__ void __launch_bounds__(128) sum_density_mixed_kernel(const Member* me
   if (!selfDone) rho.add(mi*W0);
   MB.S[S_RHO*n + i] = rho.value();
   if (enforce) enforceNode(MB, i);
+}
+
+// The same with a warp per run of rows (rowSums).
+__global__ void __launch_bounds__(kSumThreads) sum_density_mixed_rows_kernel(const Member* mem, BlockMap bm, int enforce) {
+  __shared__ float buf[kSumWarps][kSumChunk];
+  __shared__ int selfAt[kSumWarps][32];
+  const MemberBlock mb = memberBlock(bm);
+  const Member& MB = mem[mb.m];
+  const int64_t n = MB.n, cap = MB.candcap;
+  const Params& P = MB.prm;
+  const float* coefF = MB.coefF;
+  const double* mrec = MB.mrec;
+  const int32_t* nbr = MB.nbr;
+  const int nt = P.W.n;
+  const float invStep = (float)(1.0/P.W.stepSize), extent = (float)P.W.extent;
+  const int lane = threadIdx.x & 31, wib = threadIdx.x >> 5;
+  const int rowsMax = rowsPerWarp(n, mb.blocks);
+  const int64_t stride = (int64_t)mb.blocks*kSumWarps*rowsMax;
+  for (int64_t i0 = (mb.block*kSumWarps + wib)*rowsMax; i0 < n; i0 += stride) {
+    const RowRun R = rowRun(MB, i0, rowsMax);
+    selfAt[wib][lane] = R.next;
+    __syncwarp();
+    float self = 0.0f;
+    if (lane < R.rows) {
+      const D4 v = ldPlane(mrec + planeAt(cap, i0 + lane, 1));
+      self = loF(v.c)*tableW32(coefF, nt, invStep, extent, 0.0f, hiF(v.d));
+    }
+    KahanSum rho{0.0f, 0.0f};
+    int sa = R.next;
+    rowSums(R, buf[wib],
+            [&](int t, int r, int start) {
+              const int64_t e = R.e0 + t;
+              const int32_t j = __ldg(nbr + e), i = (int32_t)(i0 + r);
+              if (j > i && (t == start || __ldg(nbr + e - 1) < i)) selfAt[wib][r] = t;
+              const D4 pi = ldPlane(mrec + planeAt(cap, i, 0));
+              const D4 p = ldPlane(mrec + planeAt(cap, j, 0)), f0 = ldPlane(mrec + planeAt(cap, j, 1)),
+                       h = ldPlane(mrec + planeAt(cap, j, 2));
+              const float rx = (float)(pi.a - p.a), ry = (float)(pi.b - p.b), rz = (float)(pi.c - p.c);
+              const float xx = loF(h.a), xy = hiF(h.a), xz = loF(h.b), yy = hiF(h.b), yz = loF(h.c), zz = hiF(h.c);
+              const float ex = xx*rx + xy*ry + xz*rz;
+              const float ey = xy*rx + yy*ry + yz*rz;
+              const float ez = xz*rx + yz*ry + zz*rz;
+              const float eta = sqrtf(ex*ex + ey*ey + ez*ez);
+              return loF(f0.c)*tableW32(coefF, nt, invStep, extent, eta, hiF(f0.d));
+            },
+            [&]() { sa = selfAt[wib][lane]; },
+            [&](int t, float v) {
+              if (t == sa) rho.add(self);
+              rho.add(v);
+            });
+    if (lane < R.rows) {
+      if (sa == R.next) rho.add(self);
+      MB.S[S_RHO*n + i0 + lane] = rho.value();
+      if (enforce) enforceNode(MB, i0 + lane);
+    }
+    __syncwarp();
+  }
 }
 
 // ---------------------------------------------------------------- compatible energy
@@ -784,6 +966,66 @@ __device__ __forceinline__ double compatibleDepsDt(const Member& MB, int64_t i, 
   return DepsDti;
 }
 
+// The same with a warp per run of rows (rowSums): each internal node's rate
+// into S0's rate column, for the full RK2 update that follows.
+__global__ void __launch_bounds__(kSumThreads) compatible_energy_rows_kernel(const Member* mem, BlockMap bm, double scale) {
+  __shared__ double buf[kSumWarps][kSumChunk];
+  __shared__ double sRow[kSumWarps][32][4];        // half-step velocity, weight of the run's nodes
+  const MemberBlock mb = memberBlock(bm);
+  const Member& MB = mem[mb.m];
+  const int64_t n = MB.n;
+  const double* D = MB.D;
+  const double* S = MB.S;
+  const double* S0 = MB.S0;
+  const int32_t* nbr = MB.nbr;
+  const int32_t* groot = MB.groot;
+  const double* pacc = MB.pacc;
+  const float* paccF = reinterpret_cast<const float*>(MB.pacc);
+  const bool mixed = MB.prm.precision == SPHGPU_PRECISION_MIXED;
+  const int64_t ecap = MB.ecap;
+  const double hdt = 0.5*(scale*MB.scal[SC_DT]);
+  const int lane = threadIdx.x & 31, wib = threadIdx.x >> 5;
+  const int rowsMax = rowsPerWarp(n, mb.blocks);
+  const int64_t stride = (int64_t)mb.blocks*kSumWarps*rowsMax;
+  auto half = [&](int64_t r) {
+    const V3 v{S0[S_VX*n + r], S0[S_VY*n + r], S0[S_VZ*n + r]};
+    const V3 a{ldg(D + (D_DVDT + 0)*n + r), ldg(D + (D_DVDT + 1)*n + r), ldg(D + (D_DVDT + 2)*n + r)};
+    return vadd(v, vmul(a, hdt));
+  };
+  for (int64_t i0 = (mb.block*kSumWarps + wib)*rowsMax; i0 < n; i0 += stride) {
+    const RowRun R = rowRun(MB, i0, rowsMax);
+    if (lane < R.rows) {
+      const V3 v = half(i0 + lane);
+      sRow[wib][lane][0] = v.x; sRow[wib][lane][1] = v.y; sRow[wib][lane][2] = v.z;
+      sRow[wib][lane][3] = fabs(ldg(D + D_DEPSDT*n + i0 + lane)) + kDblEps;
+    }
+    __syncwarp();
+    double rate = 0.0;
+    rowSums(R, buf[wib],
+            [&](int t, int row, int) {
+              const int64_t k = R.e0 + t, i = i0 + row;
+              const int32_t j = __ldg(nbr + k);
+              const int64_t r = j < n ? (int64_t)j : (int64_t)__ldg(groot + (j - n));
+              const double weightj = fabs(ldg(D + D_DEPSDT*n + r)) + kDblEps;
+              const V3 vj12 = half(r);
+              const V3 vi12{sRow[wib][row][0], sRow[wib][row][1], sRow[wib][row][2]};
+              const double weighti = sRow[wib][row][3];
+              // owner's pair acceleration (FP32 in the mixed form)
+              const V3 pa = mixed ? V3{(double)__ldg(paccF + k), (double)__ldg(paccF + ecap + k), (double)__ldg(paccF + 2*ecap + k)}
+                                  : V3{ldg(pacc + k), ldg(pacc + ecap + k), ldg(pacc + 2*ecap + k)};
+              const bool own = j > (int32_t)i;
+              const double w = (own ? weighti : weightj)/(weighti + weightj);
+              const double du = dot(own ? vsub(vj12, vi12) : vsub(vi12, vj12), pa);
+              if (own) return w*du;
+              const double mj = ldg(S + S_M*n + r), mi = ldg(S + S_M*n + i);       // mass is constant within the step
+              return (1.0 - w)*du*mj/mi;
+            },
+            []() {}, [&](int, double v) { rate += v; });
+    if (lane < R.rows) MB.S0[S0_RATE*n + i0 + lane] = rate;
+    __syncwarp();
+  }
+}
+
 // ---------------------------------------------------------------- policies
 // The bounded H policies: min(1/hmin, max(1/hmax, H)) with the eigenvalue
 // limiters (boundedSym).  When the Gershgorin discs of H lie inside
@@ -804,7 +1046,8 @@ __device__ __forceinline__ Sym boundH(const Sym& H, double hmin, double hmax) {
 // source is S0 (state.assign(state0) fused into the update); with
 // compatible energy the specific thermal energy comes from
 // compatibleDepsDt (its pair loop reads S0 and the derivatives only, which
-// no thread of this launch writes).  S0 holds only what the rest of the step reads from
+// no thread of this launch writes) or from the rates that
+// compatible_energy_rows_kernel left in S0.  S0 holds only what the rest of the step reads from
 // it: position, velocity, density, energy, H, plus omega with grad-h (the
 // mid-point initialize changes it) and the CRKSPH volume.  Mass is constant
 // and pressure and sound speed are recomputed, so S0 skips them.
@@ -824,13 +1067,14 @@ enum UpdateMode { UPDATE_IN_PLACE = 0, UPDATE_SAVE_START = 1, UPDATE_FROM_START 
 // COMPAT: the launch applies the compatible energy of its compatible members
 // (only from the start-of-step state: mode UPDATE_FROM_START, the full update
 // of the RK2 step); a separate instance keeps the pair loop's registers out of
-// the other updates.
+// the other updates.  useRate: the rates are in S0 already.
 #ifndef SPH_UPDATE_MIN_BLOCKS
 #define SPH_UPDATE_MIN_BLOCKS 6
 #endif
 template<bool COMPAT>
 __global__ void __launch_bounds__(128, SPH_UPDATE_MIN_BLOCKS) update_kernel(const Member* mem, BlockMap bm, double scale,
-                                                     int timeAdvanceOnly, int mode, int packMode, int recordMid) {
+                                                     int timeAdvanceOnly, int mode, int packMode, int recordMid,
+                                                     int useRate) {
   const MemberBlock mb = memberBlock(bm);
   const Member& MB = mem[mb.m];
   const int64_t n = MB.n;
@@ -839,8 +1083,8 @@ __global__ void __launch_bounds__(128, SPH_UPDATE_MIN_BLOCKS) update_kernel(cons
   const Params& P = MB.prm;
   const double mult = scale*MB.scal[SC_DT];
   // the compatible energy's pair loop first, before the node's fields are live
-  const bool compatible = COMPAT && P.compatible;
-  const double compatDeps = compatible ? compatibleDepsDt(MB, i, 0.5*mult) : 0.0;
+  const bool compatible = (COMPAT || useRate) && P.compatible;
+  const double compatDeps = COMPAT && P.compatible ? compatibleDepsDt(MB, i, 0.5*mult) : 0.0;
   double* S = MB.S;
   double* S0 = MB.S0;
   const double* D = MB.D;
@@ -903,7 +1147,7 @@ __global__ void __launch_bounds__(128, SPH_UPDATE_MIN_BLOCKS) update_kernel(cons
   }
   // specific thermal energy: IncrementFieldList, or the compatible policy
   // (from the start-of-step state: only in the full update)
-  const double eps = compatible ? eps0 + compatDeps*mult : eps0 + mult*(D[D_DEPSDT*n + i]);
+  const double eps = compatible ? eps0 + (COMPAT ? compatDeps : S0[S0_RATE*n + i])*mult : eps0 + mult*(D[D_DEPSDT*n + i]);
   // pressure, sound speed (GammaLawGas, no active pressure limits)
   const double g1 = P.gamma - 1.0;
   const double Pn = g1*rho*eps;
@@ -1083,6 +1327,86 @@ __global__ void __launch_bounds__(128) hydro_dt_kernel(const Member* mem, BlockM
     atomicMin(reinterpret_cast<unsigned long long*>(MB.scal + slot), (unsigned long long)__double_as_longlong(minDt));
 }
 
+// The same with a warp per run of rows (rowSums).
+__global__ void __launch_bounds__(kSumThreads) hydro_dt_rows_kernel(const Member* mem, BlockMap bm, int slot, int cachedEig) {
+  __shared__ double buf[kSumWarps][kSumChunk];
+  __shared__ double sRow[kSumWarps][32][3];
+  __shared__ double least[kSumWarps];
+  const MemberBlock mb = memberBlock(bm);
+  const Member& MB = mem[mb.m];
+  const int64_t n = MB.n;
+  const Params& P = MB.prm;
+  const double* S = MB.S;
+  const double* D = MB.D;
+  const int32_t* nbr = MB.nbr;
+  const int lane = threadIdx.x & 31, wib = threadIdx.x >> 5;
+  const int rowsMax = rowsPerWarp(n, mb.blocks);
+  const int64_t stride = (int64_t)mb.blocks*kSumWarps*rowsMax;
+  double minDt = kFltMax;
+  for (int64_t i0 = (mb.block*kSumWarps + wib)*rowsMax; i0 < n; i0 += stride) {
+    const RowRun R = rowRun(MB, i0, rowsMax);
+    const int64_t i = i0 + lane;
+    if (lane < R.rows) {
+#pragma unroll
+      for (int c = 0; c < 3; ++c) sRow[wib][lane][c] = S[(S_VX + c)*n + i];
+    }
+    __syncwarp();
+    // min over the neighbors of nodeScale*safeInvVar(|vi - vj|): sqrt and the
+    // division are correctly rounded and monotone, so it is the term of the
+    // largest |vi - vj|^2, one sqrt and one division per node (bit-identical)
+    double v2max = -1.0;
+    rowSums(R, buf[wib],
+            [&](int t, int row, int) {
+              const int32_t j = __ldg(nbr + R.e0 + t);
+              const int64_t r = j < n ? (int64_t)j : (int64_t)__ldg(MB.groot + (j - n));
+              const V3 d{sRow[wib][row][0] - ldg(S + S_VX*n + r), sRow[wib][row][1] - ldg(S + S_VY*n + r),
+                         sRow[wib][row][2] - ldg(S + S_VZ*n + r)};
+              return d.x*d.x + d.y*d.y + d.z*d.z;
+            },
+            []() {}, [&](int, double v2) { if (v2 > v2max) v2max = v2; });
+    if (lane < R.rows) {
+      double lmax;
+      if (cachedEig) {
+        lmax = MB.hmaxi[n + i];
+      } else {
+        const Sym H{S[(S_H + 0)*n + i], S[(S_H + 1)*n + i], S[(S_H + 2)*n + i],
+                    S[(S_H + 3)*n + i], S[(S_H + 4)*n + i], S[(S_H + 5)*n + i]};
+        lmax = vmax(eigenValues(H));
+      }
+      const double nodeScale = 1.0/lmax/P.nPerh;
+      const double cs = S[S_CS*n + i], rho = S[S_RHO*n + i];
+      const double csDt = nodeScale/(cs + kFltMin);
+      if (csDt < minDt) minDt = csDt;
+      const double csq = sqrt(D[D_MAXVP*n + i]/rho);
+      const double csqDt = nodeScale/(csq + kFltMin);
+      if (csqDt < minDt) minDt = csqDt;
+      const double divv = D[(D_DVDX + 0)*n + i] + D[(D_DVDX + 4)*n + i] + D[(D_DVDX + 8)*n + i];
+      const double divvDt = 1.0/(fabs(divv) + kFltMin);
+      if (divvDt < minDt) minDt = divvDt;
+      if (v2max >= 0.0) {
+        const double dtVelDiff = nodeScale*safeInvVar(sqrt(v2max), 1e-30);
+        if (dtVelDiff < minDt) minDt = dtVelDiff;
+      }
+      const V3 a{D[(D_DVDT + 0)*n + i], D[(D_DVDT + 1)*n + i], D[(D_DVDT + 2)*n + i]};
+      const double dtAcc = sqrt(nodeScale/(mag(a) + kFltMin));
+      if (dtAcc < minDt) minDt = dtAcc;
+      if (P.useVelMagDt) {
+        const V3 vi{sRow[wib][lane][0], sRow[wib][lane][1], sRow[wib][lane][2]};
+        const double velDt = nodeScale/(mag(vi) + 1.0e-10);
+        if (velDt < minDt) minDt = velDt;
+      }
+    }
+    __syncwarp();
+  }
+  for (int o = 16; o > 0; o >>= 1) minDt = dmin(minDt, __shfl_xor_sync(0xffffffffu, minDt, o));
+  if (lane == 0) least[wib] = minDt;
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    for (int w = 1; w < kSumWarps; ++w) minDt = dmin(minDt, least[w]);
+    atomicMin(reinterpret_cast<unsigned long long*>(MB.scal + slot), (unsigned long long)__double_as_longlong(minDt));
+  }
+}
+
 // Integrator::selectDt on the device: dt stays resident for the step kernels.
 __global__ void select_dt_kernel(const Member* mem, int nmem) {
   const int m = blockIdx.x*blockDim.x + threadIdx.x;
@@ -1197,6 +1521,28 @@ namespace {
 bool isSph(const Problem& p) { return p.prm.hydro == SPHGPU_HYDRO_SPH; }
 bool isFp64Sph(const Problem& p) { return isSph(p) && p.cfg.precision == SPHGPU_PRECISION_FP64; }
 
+// Fewer nodes than fill the chip with a thread each: the row-sum kernels (the
+// measured crossing is given there).
+constexpr int64_t kRowSumNodes = 32768;
+bool useRowSums(const Batch& b) {
+  int64_t nodes = 0;
+  for (const Problem* p : b.mem) nodes += p->n;
+  return nodes < kRowSumNodes;
+}
+
+// Blocks of the row-sum kernels: rows per warp by the mean row of the last
+// connectivity (any number is right, it sets the speed only).
+template<class Want>
+int map_row_sums(Batch& b, Want want, BlockMap* bm, unsigned* grid) {
+  return batch_map_items(b, [&](const Problem& p) {
+    if (!want(p)) return (int64_t)0;
+    const int64_t mean = p.E > p.n ? p.E/p.n : 1;
+    int64_t rows = 32;
+    while (rows > 1 && rows*mean > kSumChunk) rows >>= 1;
+    while (rows > 1 && p.n < rows*148*16) rows >>= 1;
+    return kSumThreads*((p.n + rows*kSumWarps - 1)/(rows*kSumWarps)); }, kSumThreads, bm, grid);
+}
+
 int map_nodes(Batch& b, int threads, BlockMap* bm, unsigned* grid) {
   return batch_map_items(b, [](const Problem& p) { return p.n; }, threads, bm, grid);
 }
@@ -1307,20 +1653,6 @@ int launch_gradh(Batch& b) {
   return cuda_status(cudaGetLastError(), "gradh");
 }
 
-// Members whose rows are long enough for a group of lanes per node: a row
-// of 32 entries fills its batches of 16 to three quarters on average, and
-// below that the thread-per-node kernel's full lanes win (7.8 entries of
-// Kelvin-Helmholtz: two batches would be half empty).
-constexpr int64_t kLongRow = 32;
-bool longRows(const Problem& p) { return p.E >= kLongRow*p.n; }
-
-// Nodes per group of the row kernel: as many as leave two waves of blocks.
-int row_nodes(int64_t nodes) {
-  int q = kRowMaxNodes;
-  while (q > 1 && nodes < (int64_t)kRowGroups*q*148*8) q >>= 1;
-  return q;
-}
-
 // One launch of the FP64 pair kernel variant <XSPH, TENSILE, COMPAT, BALSARA>;
 // nodes > 0: of the row kernel.
 template<bool X, bool T, bool C, bool B>
@@ -1362,7 +1694,7 @@ int launch_eval_sph_fp64(Batch& b) {
     int64_t total = 0;
     for (Problem* p : b.mem) total += mine(*p) ? p->n : 0;
     if (total == 0) continue;
-    const int nodes = rows ? row_nodes(total) : 0;
+    const int nodes = rows ? rowNodes(total) : 0;
     BlockMap bm;
     unsigned grid = 0;
     SPH_TRY(batch_map_items(b, [&](const Problem& p) { return mine(p) ? p.n : (int64_t)0; },
@@ -1379,9 +1711,14 @@ bool summedSph(const Problem& p) { return isSph(p) && p.prm.densityUpdate == SPH
 int launch_sum_density(Batch& b, bool enforce) {
   BlockMap bm;
   unsigned grid = 0;
-  SPH_TRY(batch_map_items(b, [](const Problem& p) {
-    return isFp64Sph(p) && summedSph(p) ? p.n : (int64_t)0; }, 128, &bm, &grid));
-  if (grid) { sum_density_kernel<<<grid, 128, 0, b.stream>>>(b.d_mem, bm, enforce ? 1 : 0); batch_count_launch(b); }
+  auto want = [](const Problem& p) { return isFp64Sph(p) && summedSph(p); };
+  if (useRowSums(b)) {
+    SPH_TRY(map_row_sums(b, want, &bm, &grid));
+    if (grid) { sum_density_rows_kernel<<<grid, kSumThreads, 0, b.stream>>>(b.d_mem, bm, enforce ? 1 : 0); batch_count_launch(b); }
+  } else {
+    SPH_TRY(batch_map_items(b, [&](const Problem& p) { return want(p) ? p.n : (int64_t)0; }, 128, &bm, &grid));
+    if (grid) { sum_density_kernel<<<grid, 128, 0, b.stream>>>(b.d_mem, bm, enforce ? 1 : 0); batch_count_launch(b); }
+  }
   return cuda_status(cudaGetLastError(), "sum density");
 }
 
@@ -1390,9 +1727,14 @@ int launch_sum_density_mixed(Batch& b, bool enforce) {
   SPH_TRY(pack_mixed(b, true));
   BlockMap bm;
   unsigned grid = 0;
-  SPH_TRY(batch_map_items(b, [](const Problem& p) {
-    return p.cfg.precision == SPHGPU_PRECISION_MIXED && summedSph(p) ? p.n : (int64_t)0; }, 128, &bm, &grid));
-  if (grid) { sum_density_mixed_kernel<<<grid, 128, 0, b.stream>>>(b.d_mem, bm, enforce ? 1 : 0); batch_count_launch(b); }
+  auto want = [](const Problem& p) { return p.cfg.precision == SPHGPU_PRECISION_MIXED && summedSph(p); };
+  if (useRowSums(b)) {
+    SPH_TRY(map_row_sums(b, want, &bm, &grid));
+    if (grid) { sum_density_mixed_rows_kernel<<<grid, kSumThreads, 0, b.stream>>>(b.d_mem, bm, enforce ? 1 : 0); batch_count_launch(b); }
+  } else {
+    SPH_TRY(batch_map_items(b, [&](const Problem& p) { return want(p) ? p.n : (int64_t)0; }, 128, &bm, &grid));
+    if (grid) { sum_density_mixed_kernel<<<grid, 128, 0, b.stream>>>(b.d_mem, bm, enforce ? 1 : 0); batch_count_launch(b); }
+  }
   return cuda_status(cudaGetLastError(), "sum density (mixed)");
 }
 
@@ -1410,8 +1752,16 @@ int launch_update(Batch& b, double scale, bool timeAdvanceOnly, int mode, int pa
   if (grid) {
     bool compat = false;
     if (!timeAdvanceOnly && mode == UPDATE_FROM_START) for (const Problem* p : b.mem) compat = compat || p->prm.compatible;
-    if (compat) update_kernel<true><<<grid, 128, 0, b.stream>>>(b.d_mem, bm, scale, 0, mode, packMode, rm);
-    else update_kernel<false><<<grid, 128, 0, b.stream>>>(b.d_mem, bm, scale, timeAdvanceOnly ? 1 : 0, mode, packMode, rm);
+    const bool rows = compat && useRowSums(b);
+    if (rows) {
+      BlockMap cm;
+      unsigned cgrid = 0;
+      SPH_TRY(map_row_sums(b, [](const Problem& p) { return p.prm.compatible != 0; }, &cm, &cgrid));
+      compatible_energy_rows_kernel<<<cgrid, kSumThreads, 0, b.stream>>>(b.d_mem, cm, scale);
+      batch_count_launch(b);
+    }
+    if (compat && !rows) update_kernel<true><<<grid, 128, 0, b.stream>>>(b.d_mem, bm, scale, 0, mode, packMode, rm, 0);
+    else update_kernel<false><<<grid, 128, 0, b.stream>>>(b.d_mem, bm, scale, timeAdvanceOnly ? 1 : 0, mode, packMode, rm, rows ? 1 : 0);
     batch_count_launch(b);
   }
   return cuda_status(cudaGetLastError(), "update");
@@ -1450,8 +1800,13 @@ int launch_dt(Batch& b, int slot, bool cachedEig) {
   batch_set_scal(b, slot, kFltMax);
   BlockMap bm;
   unsigned grid = 0;
-  SPH_TRY(map_nodes(b, 128, &bm, &grid));
-  if (grid) { hydro_dt_kernel<<<grid, 128, 0, b.stream>>>(b.d_mem, bm, slot, cachedEig ? 1 : 0); batch_count_launch(b); }
+  if (useRowSums(b)) {
+    SPH_TRY(map_row_sums(b, [](const Problem&) { return true; }, &bm, &grid));
+    if (grid) { hydro_dt_rows_kernel<<<grid, kSumThreads, 0, b.stream>>>(b.d_mem, bm, slot, cachedEig ? 1 : 0); batch_count_launch(b); }
+  } else {
+    SPH_TRY(map_nodes(b, 128, &bm, &grid));
+    if (grid) { hydro_dt_kernel<<<grid, 128, 0, b.stream>>>(b.d_mem, bm, slot, cachedEig ? 1 : 0); batch_count_launch(b); }
+  }
   return cuda_status(cudaGetLastError(), "dt");
 }
 

@@ -44,3 +44,44 @@ def test_rows(gpu_lib, pkg, oracle_mod, keep, options):
     for k in KEYS:
         assert np.array_equal(g.field(k), o.field(k)), k
     assert normwise(g.field("new H"), o.field("new H")) <= 1e-12
+
+
+@pytest.mark.parametrize("keep", [512, 505, 449])
+@pytest.mark.parametrize("options", [{}, {"XSPH": 1, "compatibleEnergyEvolution": 0}, {"epsTensile": 0.3}])
+def test_rows_mixed(gpu_lib, pkg, keep, options):
+    """The mixed form's row kernel at the same edges: within the mixed form's
+    1e-5 (normwise) of the FP64 form."""
+    gen, abi = pkg.generators, pkg.abi
+    ns = gen.kelvin_helmholtz(nx=8, ny=8, nz=8, jitter=0.2, seed=keep)
+    ns = gen.NodeSet(ns.pos[:keep], ns.vel[:keep], ns.mass[:keep], ns.rho[:keep], ns.eps[:keep], ns.H[:keep], ns.dx)
+    ns.H[:, [0, 3, 5]] = 1.0 / np.random.default_rng(keep).uniform(0.13, 0.22, keep)[:, None]
+    out = {}
+    for precision in (abi.PRECISION_FP64, abi.PRECISION_MIXED):
+        g = pkg.SPHHydro(gen.kh_config(abi, kernel=abi.KERNEL_BSPLINE, precision=precision, **options), ns)
+        g.build_neighbors()
+        assert np.diff(g.connectivity()[0]).mean() >= 32
+        g.evaluateDerivatives()
+        out[precision] = {k: g.field(k) for k in KEYS + ["new H"]}
+    for k, want in out[abi.PRECISION_FP64].items():
+        assert normwise(out[abi.PRECISION_MIXED][k], want) <= 1e-5, k
+
+
+@pytest.mark.parametrize("precision", ["PRECISION_FP64", "PRECISION_MIXED"])
+@pytest.mark.parametrize("nx,other", [(15, 40), (9, 40)])
+def test_row_sums_equal_thread_sums(gpu_lib, pkg, precision, nx, other):
+    """Alone, a small problem takes the summed density, compatible energy and
+    dt vote with a warp per run of rows; in a batch of more nodes than fill the
+    chip, a thread per node.  Both add in row order: the states are bit-equal."""
+    gen, abi = pkg.generators, pkg.abi
+
+    def problem(n, seed):
+        ns = gen.kelvin_helmholtz(nx=n, ny=n, nz=n, seed=seed, jitter=0.1)
+        return pkg.SPHHydro(gen.kh_config(abi, precision=getattr(abi, precision)), ns)
+
+    alone, small, large = problem(nx, 3), problem(nx, 3), problem(other, 4)
+    assert nx ** 3 < 32768 <= other ** 3
+    alone.step(4)
+    batch = pkg.SPHBatch([small, large])
+    batch.step(4)
+    for k in ("position", "velocity", "mass density", "specific thermal energy", "H"):
+        assert np.array_equal(alone.field(k), small.field(k)), k
