@@ -35,6 +35,8 @@
 #include <cfloat>
 #include <climits>
 
+#include <cooperative_groups.h>
+
 #include "problem.cuh"
 
 namespace sphgpu {
@@ -303,22 +305,26 @@ __global__ void ghost_advance_kernel(const Member* mem, int nmem) {
 }
 
 // ---------------------------------------------------------------- fused ghost passes
-// The six boundary passes in one cooperative launch, for a batch of a few
-// members: the per-pass hmax, the flags, their prefix sum and the scatter
-// of the new images, separated by grid barriers.  An item's share of a
-// pass's hmax depends on the item alone, so the near-plane nodes give their
-// shares to every pass before the first one, and each new image to the
-// passes after its own as it is made; a pass then needs two barriers (after
-// its block counts, after its scatter).  Block k takes the k-th contiguous
-// chunk of a pass's items and numbers its images in item order, so the
-// images, their order and the error bits are those of the per-pass launches.
+// The six boundary passes in one launch.  A boundary's images follow from its
+// hmax alone, item by item, so a thread keeps the images its near-plane nodes
+// (roots) have so far as a bit set and only the passes' hmax are exchanged:
+// one barrier per pass, and one for the counts at the end.
+//
+// An image is named by the plane it was mapped through on each axis (0 none,
+// 1 or 2): e = x + 3 y + 9 z.  The reference's pass order (x, y, z, each plane 1
+// then 2; in a pass the nodes first, then the images made so far in their
+// order) makes the images come by ascending e, and those of one e by
+// ascending root: their place is the images of smaller e plus the smaller
+// roots that have this one.  Position, order and error bits are those of the
+// per-pass launches.  Measured (B200, whole launch; before, two barriers a pass
+// and every pass re-reading nodes and images): 124,550 nodes 80 -> 57 us,
+// Kelvin-Helmholtz 128^3 121 -> 65 us; bound by the seven grid barriers.
 __device__ __forceinline__ int64_t imin64(int64_t a, int64_t b) { return a < b ? a : b; }
 constexpr int kFusedGhostMembers = 4;
-#ifndef FUSED_GHOST_MIN_BLOCKS
-#define FUSED_GHOST_MIN_BLOCKS 2
-#endif
-constexpr int kFusedGhostBlocks = 148*FUSED_GHOST_MIN_BLOCKS;
-constexpr int kBarrierPolls = 1 << 21;
+constexpr int kGhostCodes = 27;                         // 1 (the root itself) + 26 images
+constexpr int kRootThreads = 1024;
+constexpr int kFusedGhostBlocks = 148;
+constexpr int kBarrierPolls = 1 << 23;
 
 // Grid barrier of a cooperative launch (every block resident).  bar[0]
 // counts arrivals, bar[1] is the generation.  A block that polls more than
@@ -344,7 +350,6 @@ __device__ bool grid_barrier(unsigned int* bar, const Member* mem, int nm) {
           ok = 0;
           break;
         }
-        __nanosleep(100);
       }
     }
     __threadfence();
@@ -353,188 +358,238 @@ __device__ bool grid_barrier(unsigned int* bar, const Member* mem, int nm) {
   return ok != 0;
 }
 
-// position of item node k (ghost positions are written during the launch:
-// read through L2)
-__device__ __forceinline__ V3 fusedPos(const Member& M, int64_t k) {
-  const int64_t n = M.n;
-  if (k < n) return V3{M.S[S_X*n + k], M.S[S_Y*n + k], M.S[S_Z*n + k]};
-  const int64_t g = k - n;
-  return V3{__ldcg(M.gpos + g), __ldcg(M.gpos + M.gcap + g), __ldcg(M.gpos + 2*M.gcap + g)};
-}
-__device__ __forceinline__ int32_t fusedRoot(const Member& M, int64_t k) {
-  return k < M.n ? (int32_t)k : __ldcg(M.groot + (k - M.n));
+
+__device__ __forceinline__ uint32_t imageCode(int e) {
+  return (uint32_t)(e % 3) | (uint32_t)(e/3 % 3) << 2 | (uint32_t)(e/9) << 4;
 }
 
-// an item's shares of the hmax of passes [from, 6) (ghost_hmax_kernel's test)
-__device__ __forceinline__ void hmaxShares(const Member& M, const V3& r, double hmaxi, int from, double* loc) {
-#pragma unroll
-  for (int b = 0; b < 6; ++b) {
-    if (b < from || !M.prm.bcs.periodic[b >> 1]) continue;
-    const PlanarBC& bc = M.prm.bcs.bc[b];
-    if (dmin(minimumDistance(bc.exit, r), minimumDistance(bc.enter, r)) < M.prm.kernelExtent*hmaxi)
-      loc[b] = dmax(loc[b], hmaxi);
-  }
+// image codes with 0 and with 1 on each axis
+__device__ constexpr uint32_t digitMask(int axis, int digit) {
+  uint32_t m = 0;
+  const int step = axis == 0 ? 1 : (axis == 1 ? 3 : 9);
+  for (int e = 0; e < kGhostCodes; ++e) if (e/step % 3 == digit) m |= 1u << e;
+  return m;
 }
 
-// block maxima of the shares into the member's pass hmax words
-__device__ void hmaxFlush(const Member& M, double* loc, int from) {
-  __shared__ double red[6][kGhostThreads/32];
-  const int w = threadIdx.x >> 5, lane = threadIdx.x & 31;
-#pragma unroll
-  for (int b = 0; b < 6; ++b) {
-    double v = loc[b];
-    for (int o = 16; o > 0; o >>= 1) v = dmax(v, __shfl_xor_sync(0xffffffffu, v, o));
-    if (lane == 0) red[b][w] = v;
+// The periodic planes lie across their axis, so a plane's test of an item sees
+// the item's coordinate along that axis only, which mapping along the others
+// leaves as the root's: the root's own position stands for all its images with
+// 0 on the axis, and its image through plane 1 for those with 1.
+
+// largest share of a root's items (itself and its images so far) in the hmax
+// of boundary b (ghost_hmax_kernel's test)
+__device__ __forceinline__ double rootShare(const Member& M, const V3& r, double h, uint32_t items, int b) {
+  const PlanarBC bc = M.prm.bcs.bc[b];
+  const double lim = M.prm.kernelExtent*h;
+  bool f = dmin(minimumDistance(bc.exit, r), minimumDistance(bc.enter, r)) < lim;
+  if ((b & 1) && !f && (items & (b == 1 ? digitMask(0, 1) : (b == 3 ? digitMask(1, 1) : digitMask(2, 1))))) {
+    const PlanarBC& one = M.prm.bcs.bc[b - 1];
+    const V3 x = mapPositionThroughPlanes(r, one.exit, one.enter);
+    f = dmin(minimumDistance(bc.exit, x), minimumDistance(bc.enter, x)) < lim;
   }
+  return f ? h : 0.0;
+}
+
+// the items boundary b images (ghost_flag_kernel's test) join the set
+__device__ __forceinline__ uint32_t rootImages(const Member& M, const V3& r, double hmax, uint32_t items, int b) {
+  if (!(hmax > 0.0)) return items;
+  const PlanarBC bc = M.prm.bcs.bc[b];
+  const int axis = b >> 1, step = axis == 0 ? 1 : (axis == 1 ? 3 : 9);
+  const uint32_t d0 = axis == 0 ? digitMask(0, 0) : (axis == 1 ? digitMask(1, 0) : digitMask(2, 0));
+  const uint32_t d1 = axis == 0 ? digitMask(0, 1) : (axis == 1 ? digitMask(1, 1) : digitMask(2, 1));
+  auto imaged = [&](const V3& x) {
+    const double disti = signedDistance(bc.exit, x)/hmax;
+    return disti >= 0.0 && disti <= M.prm.kernelExtent;
+  };
+  uint32_t all = items;
+  if (imaged(r)) all |= (items & d0) << (((b & 1) + 1)*step);
+  if ((b & 1) && (items & d1)) {
+    const PlanarBC& one = M.prm.bcs.bc[b - 1];
+    if (imaged(mapPositionThroughPlanes(r, one.exit, one.enter))) atomicOr(M.err, DERR_GHOST_CHAIN);
+  }
+  return all;
+}
+
+// roots of the chunk per image code: cnt[e] (shared)
+__device__ __forceinline__ void countImages(const Member& M, int64_t c0, int64_t c1, int* cnt) {
+  if (threadIdx.x < 32) cnt[threadIdx.x] = 0;
   __syncthreads();
-  if (threadIdx.x < 6 && (int)threadIdx.x >= from) {
-    double v = 0.0;
-    for (int k = 0; k < kGhostThreads/32; ++k) v = dmax(v, red[threadIdx.x][k]);
-    if (v > 0.0)
-      atomicMax(reinterpret_cast<unsigned long long*>(M.scal + SC_PHMAX + threadIdx.x),
-                (unsigned long long)__double_as_longlong(v));
-  }
-  __syncthreads();
-}
-
-// ghost_flag_kernel's test of item t for pass b
-__device__ __forceinline__ bool ghostFlag(const Member& M, int b, double hmax, int64_t t, int64_t nnear) {
-  if (!M.prm.bcs.periodic[b >> 1] || !(hmax > 0.0)) return false;
-  const V3 r = fusedPos(M, passNode(M, t, nnear));
-  const double disti = signedDistance(M.prm.bcs.bc[b].exit, r)/hmax;
-  return disti >= 0.0 && disti <= M.prm.kernelExtent;
-}
-
-__global__ void __launch_bounds__(kGhostThreads, FUSED_GHOST_MIN_BLOCKS) ghost_passes_fused_kernel(const Member* mem, int nm, unsigned int* fuse) {
-  unsigned int* bar = fuse;
-  int64_t* blk = reinterpret_cast<int64_t*>(fuse + 2);      // [member][block] counts of a pass
-  const int nb = gridDim.x, kb = blockIdx.x;
-  const int w = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  __shared__ int64_t wsum[kGhostThreads/32];
-  __shared__ int64_t sG[kFusedGhostMembers];
-  __shared__ int64_t sPre, sTot;
-  if (threadIdx.x < kFusedGhostMembers) sG[threadIdx.x] = 0;
-  // the near-plane nodes' shares of every pass's hmax
-  for (int m = 0; m < nm; ++m) {
-    const Member& M = mem[m];
-    const int64_t nnear = scalI(M.scal, SC_NNEAR);
-    double loc[6] = {0.0, 0.0, 0.0, 0.0, 0.0, 0.0};
-    for (int64_t t = kb*(int64_t)blockDim.x + threadIdx.x; t < nnear; t += (int64_t)nb*blockDim.x) {
-      const int64_t k = M.cidx[t];
-      hmaxShares(M, nodePos(M, k), M.hmaxi[k], 0, loc);
+  const int lane = threadIdx.x & 31;
+  for (int64_t base = c0; base < c1; base += kRootThreads) {
+    const int64_t t = base + threadIdx.x;
+    const uint32_t items = t < c1 ? (uint32_t)M.counts[t] : 0u;
+    int mine = 0;
+    for (uint32_t codes = __reduce_or_sync(0xffffffffu, items) & ~1u; codes; codes &= codes - 1) {
+      const int e = __ffs(codes) - 1;
+      const unsigned bal = __ballot_sync(0xffffffffu, items >> e & 1u);
+      if (lane == e) mine = __popc(bal);
     }
-    hmaxFlush(M, loc, 0);
+    if (mine) atomicAdd(cnt + lane, mine);
   }
-  if (!grid_barrier(bar, mem, nm)) return;
+  __syncthreads();
+}
+
+// the images of the chunk's roots; next[e] (shared): ghost index of the
+// chunk's first image of code e
+__device__ __forceinline__ void writeImages(const Member& M, int64_t c0, int64_t c1, int64_t* next, int (*warpCnt)[32]) {
+  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+  for (int64_t base = c0; base < c1; base += kRootThreads) {
+    const int64_t t = base + threadIdx.x;
+    uint32_t items = t < c1 ? (uint32_t)M.counts[t] & ~1u : 0u;
+    const uint32_t codes = __reduce_or_sync(0xffffffffu, items);
+    int mine = 0;
+    for (uint32_t left = codes; left; left &= left - 1) {
+      const int e = __ffs(left) - 1;
+      const unsigned bal = __ballot_sync(0xffffffffu, items >> e & 1u);
+      if (lane == e) mine = __popc(bal);
+    }
+    warpCnt[w][lane] = mine;
+    __syncthreads();
+    // lane e: the first index of this warp's images of code e
+    int64_t at = next[lane];
+    {
+      int pre = 0;
+#pragma unroll 8
+      for (int k = 0; k < kRootThreads/32; ++k) pre += k < w ? warpCnt[k][lane] : 0;
+      at += pre;
+    }
+    if (codes) {
+      int32_t root = 0;
+      V3 r{0.0, 0.0, 0.0};
+      if (items) {
+        root = __ldcg(M.cidx + t);
+        r = nodePos(M, root);
+      }
+      for (uint32_t left = codes; left; left &= left - 1) {
+        const int e = __ffs(left) - 1;
+        const bool has = items >> e & 1u;
+        const unsigned bal = __ballot_sync(0xffffffffu, has);
+        const int64_t first = __shfl_sync(0xffffffffu, at, e);
+        if (!has) continue;
+        const int64_t g = first + __popc(bal & ((1u << lane) - 1u));
+        if (g >= M.gcap) {
+          atomicOr(M.err, DERR_GHOST_CAPACITY);
+          continue;
+        }
+        const uint32_t code = imageCode(e);
+        const V3 gp = ghostPosition(M.prm.bcs, r, code);
+        M.groot[g] = root;
+        M.gcode[g] = code;
+        M.gpos[g] = gp.x; M.gpos[M.gcap + g] = gp.y; M.gpos[2*M.gcap + g] = gp.z;
+      }
+    }
+    __syncthreads();
+    if (w == 0) {
+      int sum = 0;
+#pragma unroll 8
+      for (int k = 0; k < kRootThreads/32; ++k) sum += warpCnt[k][lane];
+      next[lane] += sum;
+    }
+    __syncthreads();
+  }
+}
+
+// sizes after the passes
+__device__ __forceinline__ void endGhosts(const Member& M, int64_t G) {
+  if (G > M.gcap) {
+    atomicOr(M.err, DERR_GHOST_CAPACITY);
+    G = M.gcap;
+  }
+  setScalI(M.scal, SC_NTOT, M.n + G);
+  setScalI(M.scal, SC_G, G);
+  M.scal[SC_HMAX] = 0.0;
+}
+
+__device__ __forceinline__ double blockMax(double x, double* red) {
+  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+  for (int o = 16; o > 0; o >>= 1) x = dmax(x, __shfl_xor_sync(0xffffffffu, x, o));
+  __syncthreads();
+  if (lane == 0) red[w] = x;
+  __syncthreads();
+  x = red[lane];
+  for (int o = 16; o > 0; o >>= 1) x = dmax(x, __shfl_xor_sync(0xffffffffu, x, o));
+  return x;
+}
+
+// A cooperative launch over the near-plane lists of a batch of a few members;
+// fuse: the barrier (2 words), then the per-block counts of each member and code.
+__global__ void __launch_bounds__(kRootThreads, 1) ghost_passes_fused_kernel(const Member* mem, int nm, unsigned int* fuse) {
+  unsigned int* bar = fuse;
+  int* blk = reinterpret_cast<int*>(fuse + 2);            // [member][code][block]
+  const int nb = gridDim.x, kb = blockIdx.x;
+  __shared__ double red[32];
+  __shared__ int cnt[32], warpCnt[kRootThreads/32][32];
+  __shared__ int64_t next[32];
   for (int b = 0; b < 6; ++b) {
     bool any = false;
     for (int m = 0; m < nm; ++m) any = any || mem[m].prm.bcs.periodic[b >> 1];
+    if (!any && b > 0) continue;
+    for (int m = 0; m < nm; ++m) {
+      const Member& M = mem[m];
+      const int64_t nnear = scalI(M.scal, SC_NNEAR), chunk = (nnear + nb - 1)/nb;
+      const int64_t c0 = imin64(nnear, kb*chunk), c1 = imin64(nnear, c0 + chunk);
+      double best = 0.0;
+      for (int64_t t = c0 + threadIdx.x; t < c1; t += kRootThreads) {
+        if (b == 0) M.counts[t] = 1;
+        if (!M.prm.bcs.periodic[b >> 1]) continue;
+        const int64_t k = M.cidx[t];
+        best = dmax(best, rootShare(M, nodePos(M, k), M.hmaxi[k], (uint32_t)M.counts[t], b));
+      }
+      best = blockMax(best, red);
+      if (threadIdx.x == 0 && best > 0.0)
+        atomicMax(reinterpret_cast<unsigned long long*>(M.scal + SC_PHMAX + b), (unsigned long long)__double_as_longlong(best));
+    }
     if (!any) continue;
-    // flags of this block's chunk: the block's count
+    if (!grid_barrier(bar, mem, nm)) return;
     for (int m = 0; m < nm; ++m) {
       const Member& M = mem[m];
-      const int64_t nnear = scalI(M.scal, SC_NNEAR);
-      const int64_t items = nnear + sG[m];
-      const int64_t chunk = (items + nb - 1)/nb;
-      const int64_t c0 = imin64(items, kb*chunk), c1 = imin64(items, c0 + chunk);
+      if (!M.prm.bcs.periodic[b >> 1]) continue;
+      const int64_t nnear = scalI(M.scal, SC_NNEAR), chunk = (nnear + nb - 1)/nb;
+      const int64_t c0 = imin64(nnear, kb*chunk), c1 = imin64(nnear, c0 + chunk);
       const double hmax = __longlong_as_double((long long)__ldcg(reinterpret_cast<const unsigned long long*>(M.scal + SC_PHMAX + b)));
-      int64_t cnt = 0;
-      for (int64_t t = c0 + threadIdx.x; t < c1; t += blockDim.x) cnt += ghostFlag(M, b, hmax, t, nnear) ? 1 : 0;
-      for (int o = 16; o > 0; o >>= 1) cnt += __shfl_xor_sync(0xffffffffu, cnt, o);
-      if (lane == 0) wsum[w] = cnt;
-      __syncthreads();
-      if (threadIdx.x == 0) {
-        int64_t s = 0;
-        for (int k = 0; k < kGhostThreads/32; ++k) s += wsum[k];
-        blk[m*nb + kb] = s;
-      }
-      __syncthreads();
+      for (int64_t t = c0 + threadIdx.x; t < c1; t += kRootThreads)
+        M.counts[t] = (int32_t)rootImages(M, nodePos(M, M.cidx[t]), hmax, (uint32_t)M.counts[t], b);
     }
-    if (!grid_barrier(bar, mem, nm)) return;
-    // the block's offset among the chunks, the pass total, the scatter
-    for (int m = 0; m < nm; ++m) {
-      const Member& M = mem[m];
-      const int64_t n = M.n;
-      const int64_t nnear = scalI(M.scal, SC_NNEAR);
-      const int64_t G = sG[m];
-      const int64_t items = nnear + G;
-      const int64_t chunk = (items + nb - 1)/nb;
-      const int64_t c0 = imin64(items, kb*chunk), c1 = imin64(items, c0 + chunk);
-      const double hmax = __longlong_as_double((long long)__ldcg(reinterpret_cast<const unsigned long long*>(M.scal + SC_PHMAX + b)));
-      int64_t pre = 0, tot = 0;
-      for (int k = threadIdx.x; k < nb; k += blockDim.x) {
-        const int64_t c = __ldcg(blk + m*nb + k);
-        tot += c;
-        if (k < kb) pre += c;
-      }
-      for (int o = 16; o > 0; o >>= 1) {
-        pre += __shfl_xor_sync(0xffffffffu, pre, o);
-        tot += __shfl_xor_sync(0xffffffffu, tot, o);
-      }
-      __shared__ int64_t wpre[kGhostThreads/32];
-      if (lane == 0) { wsum[w] = tot; wpre[w] = pre; }
-      __syncthreads();
-      if (threadIdx.x == 0) {
-        int64_t a = 0, c = 0;
-        for (int k = 0; k < kGhostThreads/32; ++k) { a += wpre[k]; c += wsum[k]; }
-        sPre = a;
-        sTot = c;
-      }
-      __syncthreads();
-      int64_t next = G + sPre;                         // ghost index of this block's first image
-      const PlanarBC& bc = M.prm.bcs.bc[b];
-      const int axis = b >> 1;
-      double loc[6] = {0.0, 0.0, 0.0, 0.0, 0.0, 0.0};
-      for (int64_t base = c0; base < c1; base += blockDim.x) {
-        const int64_t t = base + threadIdx.x;
-        const bool f = t < c1 && ghostFlag(M, b, hmax, t, nnear);
-        const unsigned bal = __ballot_sync(0xffffffffu, f);
-        if (lane == 0) wsum[w] = __popc(bal);
-        __syncthreads();
-        int64_t off = 0, tileTot = 0;
-        for (int k = 0; k < kGhostThreads/32; ++k) {
-          if (k < w) off += wsum[k];
-          tileTot += wsum[k];
-        }
-        off += __popc(bal & ((1u << lane) - 1u));
-        if (f) {
-          const int64_t k = passNode(M, t, nnear);
-          const int64_t g = next + off;
-          if (g >= M.gcap) {
-            atomicOr(M.err, DERR_GHOST_CAPACITY);
-          } else {
-            const V3 gp = mapPositionThroughPlanes(fusedPos(M, k), bc.exit, bc.enter);
-            const int32_t root = fusedRoot(M, k);
-            uint32_t code = k < n ? 0u : __ldcg(M.gcode + (k - n));
-            if ((code >> (2*axis)) & 3u) atomicOr(M.err, DERR_GHOST_CHAIN);
-            code |= (uint32_t)((b & 1) + 1) << (2*axis);
-            M.groot[g] = root;
-            M.gcode[g] = code;
-            M.gpos[g] = gp.x; M.gpos[M.gcap + g] = gp.y; M.gpos[2*M.gcap + g] = gp.z;
-            hmaxShares(M, gp, M.hmaxi[root], b + 1, loc);
-          }
-        }
-        next += tileTot;
-        __syncthreads();
-      }
-      hmaxFlush(M, loc, b + 1);
-      if (threadIdx.x == 0) {
-        int64_t g = G + sTot;
-        if (g > M.gcap) {
-          if (kb == 0) atomicOr(M.err, DERR_GHOST_CAPACITY);
-          g = M.gcap;
-        }
-        sG[m] = g;
-      }
-      __syncthreads();
-    }
-    if (!grid_barrier(bar, mem, nm)) return;
   }
-  if (kb == 0 && threadIdx.x < nm) {
-    const Member& M = mem[threadIdx.x];
-    setScalI(M.scal, SC_NTOT, M.n + sG[threadIdx.x]);
-    setScalI(M.scal, SC_G, sG[threadIdx.x]);
-    M.scal[SC_HMAX] = 0.0;
+  for (int m = 0; m < nm; ++m) {
+    const Member& M = mem[m];
+    const int64_t nnear = scalI(M.scal, SC_NNEAR), chunk = (nnear + nb - 1)/nb;
+    const int64_t c0 = imin64(nnear, kb*chunk), c1 = imin64(nnear, c0 + chunk);
+    countImages(M, c0, c1, cnt);
+    if (threadIdx.x < kGhostCodes) blk[(m*kGhostCodes + threadIdx.x)*nb + kb] = cnt[threadIdx.x];
+    __syncthreads();
+  }
+  if (!grid_barrier(bar, mem, nm)) return;
+  for (int m = 0; m < nm; ++m) {
+    const Member& M = mem[m];
+    const int64_t nnear = scalI(M.scal, SC_NNEAR), chunk = (nnear + nb - 1)/nb;
+    const int64_t c0 = imin64(nnear, kb*chunk), c1 = imin64(nnear, c0 + chunk);
+    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+    // warp e: the images of code e in the blocks before this one, and in all
+    int before = 0, total = 0;
+    if (w < kGhostCodes) {
+      for (int k = lane; k < nb; k += 32) {
+        const int c = __ldcg(blk + (m*kGhostCodes + w)*nb + k);
+        total += c;
+        if (k < kb) before += c;
+      }
+    }
+    before = __reduce_add_sync(0xffffffffu, before);
+    total = __reduce_add_sync(0xffffffffu, total);
+    if (lane == 0) { warpCnt[0][w] = before; warpCnt[1][w] = total; }
+    __syncthreads();
+    if (w == 0) {
+      const int64_t mine = warpCnt[1][lane];
+      int64_t incl = mine;
+      for (int o = 1; o < 32; o <<= 1) {
+        const int64_t v = __shfl_up_sync(0xffffffffu, incl, o);
+        if (lane >= o) incl += v;
+      }
+      next[lane] = incl - mine + warpCnt[0][lane];
+      if (lane == 31 && kb == 0) endGhosts(M, incl);
+    }
+    __syncthreads();
+    writeImages(M, c0, c1, next, warpCnt);
   }
 }
 
@@ -544,10 +599,7 @@ __global__ void __launch_bounds__(kGhostThreads, FUSED_GHOST_MIN_BLOCKS) ghost_p
 // enlarged until the cells fit the cell buffers (larger cells only widen the
 // candidate set).  Also resets the walk's counters and sets the FP32
 // pre-test tolerance: only when max h / min h over the problem is <= 100.
-__global__ void grid_kernel(const Member* mem, int nmem) {
-  const int m = blockIdx.x*blockDim.x + threadIdx.x;
-  if (m >= nmem) return;
-  const Member& M = mem[m];
+__device__ void setGrid(const Member& M) {
   const unsigned long long* bb = reinterpret_cast<const unsigned long long*>(M.scal + SC_BOUNDS);
   double lo[3], hi[3];
   for (int a = 0; a < 3; ++a) { lo[a] = fromOrderedBits(bb[a]); hi[a] = fromOrderedBits(bb[3 + a]); }
@@ -605,6 +657,222 @@ __global__ void grid_kernel(const Member* mem, int nmem) {
   setScalI(M.scal, SC_NCELLS, ncells);
   setScalI(M.scal, SC_MAXCOUNT, 0);
   setScalI(M.scal, SC_PAIRS, 0);
+}
+
+__global__ void grid_kernel(const Member* mem, int nmem) {
+  const int m = blockIdx.x*blockDim.x + threadIdx.x;
+  if (m < nmem) setGrid(mem[m]);
+}
+
+// ---------------------------------------------------------------- small members
+// The build up to the cell grid (hmax, bounds, near-plane list, the six
+// boundary passes, the grid) in one launch with a cluster of 8 blocks per
+// member, for members of at most kClusterNodes nodes.
+//
+// Why: the work is a few thousand items, but as separate launches it was nine
+// kernels with a cooperative one among them.  Measured (B200): 4,096-node Sod
+// tube, the nine launches 100 us, here 45 us.  Beyond kClusterNodes the eight
+// blocks' passes over all nodes take longer than the launches saved (124,550
+// nodes: 262 us against about 85).  The blocks of a cluster exchange their counts and
+// maxima through each other's shared memory and meet at the hardware's cluster
+// barrier.  Block k takes the k-th contiguous chunk of every list, so the
+// near-plane list, the images, their order and the error bits are those of the
+// separate launches.
+namespace cg = cooperative_groups;
+constexpr int kClusterBlocks = 8;
+constexpr int kClusterThreads = kRootThreads;
+#ifndef CLUSTER_NODES
+#define CLUSTER_NODES 32768
+#endif
+constexpr int64_t kClusterNodes = CLUSTER_NODES;
+
+struct ClusterShared {
+  double hmax[6];                 // this block's share of each pass's hmax
+  double bounds[8];               // lo[3], hi[3], largest 1/min(eig(H)), largest max(eig(H))
+  int count;                      // near-plane nodes of this block's chunk
+  int before, total;              // ... of the blocks before, of all
+  double all;                     // the cluster's maximum
+  int images[32];                 // images of this block's chunk, by code
+  int64_t next[32];
+  int warp[32], warpCnt[kClusterThreads/32][32];
+  double red[32][8];
+};
+
+// flagged items of the block's chunk [c0, c1)
+template<class Flag>
+__device__ __forceinline__ int clusterCount(int64_t c0, int64_t c1, Flag flag) {
+  int cnt = 0;
+  for (int64_t base = c0; base < c1; base += kClusterThreads) {
+    const int64_t t = base + threadIdx.x;
+    cnt += __syncthreads_count(t < c1 && flag(t));
+  }
+  return cnt;
+}
+
+// put(t, k): item t is the chunk's k-th flagged one
+template<class Flag, class Put>
+__device__ __forceinline__ void clusterScatter(ClusterShared& sh, int64_t c0, int64_t c1, Flag flag, Put put) {
+  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+  int done = 0;
+  for (int64_t base = c0; base < c1; base += kClusterThreads) {
+    const int64_t t = base + threadIdx.x;
+    const bool f = t < c1 && flag(t);
+    const unsigned bal = __ballot_sync(0xffffffffu, f);
+    __syncthreads();
+    if (lane == 0) sh.warp[w] = __popc(bal);
+    __syncthreads();
+    const int c = sh.warp[lane];
+    const int off = done + __reduce_add_sync(0xffffffffu, lane < w ? c : 0);
+    done += __reduce_add_sync(0xffffffffu, c);
+    if (f) put(t, off + __popc(bal & ((1u << lane) - 1u)));
+  }
+}
+
+__global__ void __cluster_dims__(kClusterBlocks, 1, 1) __launch_bounds__(kClusterThreads, 1) ghost_cluster_kernel(const Member* mem) {
+  __shared__ ClusterShared sh;
+  cg::cluster_group cl = cg::this_cluster();
+  const Member& M = mem[blockIdx.x/kClusterBlocks];
+  const int rank = (int)cl.block_rank();
+  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+  const int64_t n = M.n;
+  // 1/min(eig(H)), max(eig(H)), the bounds (node_hmax_kernel)
+  {
+    double v[8] = {1e300, 1e300, 1e300, -1e300, -1e300, -1e300, 0.0, 0.0};
+    for (int64_t i = rank*(int64_t)kClusterThreads + threadIdx.x; i < n; i += kClusterBlocks*kClusterThreads) {
+      const V3 ev = eigenValues(nodeH(M, i));
+      const double hi1 = 1.0/vmin(ev);
+      M.hmaxi[i] = hi1;
+      v[6] = fmax(v[6], hi1);
+      double l = vmax(ev);
+      M.hmaxi[n + i] = l;
+      if (!(l < 1.0e300)) l = 1.0e300;           // degenerate H: no FP32 pre-test
+      v[7] = dmax(v[7], l);
+      const V3 r = nodePos(M, i);
+      v[0] = fmin(v[0], r.x); v[1] = fmin(v[1], r.y); v[2] = fmin(v[2], r.z);
+      v[3] = fmax(v[3], r.x); v[4] = fmax(v[4], r.y); v[5] = fmax(v[5], r.z);
+    }
+#pragma unroll
+    for (int c = 0; c < 8; ++c) {
+      for (int o = 16; o > 0; o >>= 1) {
+        const double x = __shfl_xor_sync(0xffffffffu, v[c], o);
+        v[c] = c < 3 ? fmin(v[c], x) : (c < 7 ? fmax(v[c], x) : dmax(v[c], x));
+      }
+      if (lane == 0) sh.red[w][c] = v[c];
+    }
+    __syncthreads();
+    if (w < 8) {
+      double x = sh.red[lane][w];
+      for (int o = 16; o > 0; o >>= 1) {
+        const double y = __shfl_xor_sync(0xffffffffu, x, o);
+        x = w < 3 ? fmin(x, y) : fmax(x, y);
+      }
+      if (lane == 0) sh.bounds[w] = x;
+    }
+  }
+  cl.sync();
+  if (w == 0) {
+    // one warp reads the other blocks' shared memory
+    double b[8];
+#pragma unroll
+    for (int c = 0; c < 8; ++c) {
+      double x = cl.map_shared_rank(&sh, lane % kClusterBlocks)->bounds[c];
+      for (int o = kClusterBlocks/2; o > 0; o >>= 1) {
+        const double y = __shfl_xor_sync(0xffffffffu, x, o);
+        x = c < 3 ? fmin(x, y) : fmax(x, y);
+      }
+      b[c] = x;
+    }
+    if (lane == 0) sh.all = b[6];
+    if (rank == 0 && lane == 0) {
+    unsigned long long* out = reinterpret_cast<unsigned long long*>(M.scal + SC_BOUNDS);
+    for (int a = 0; a < 3; ++a) {
+      out[a] = b[6] > 0.0 ? orderedBits(b[a]) : ~0ULL;
+      out[3 + a] = b[6] > 0.0 ? orderedBits(b[3 + a]) : 0ULL;
+    }
+    out[6] = b[6] > 0.0 ? orderedBits(b[6]) : 0ULL;
+    M.scal[SC_LMAXALL] = b[7];
+    }
+  }
+  __syncthreads();
+  const double hAll = sh.all;
+  // the near-plane list, ascending (near_flag_kernel, near_list_kernel)
+  const double nearReach = M.prm.kernelExtent*fromOrderedBits(hAll > 0.0 ? orderedBits(hAll) : 0ULL)*(1.0 + 1.0e-6);
+  auto isNear = [&](int64_t i) {
+    const V3 r = nodePos(M, i);
+    bool f = false;
+    for (int a = 0; a < 3; ++a) {
+      if (!M.prm.bcs.periodic[a]) continue;
+      const PlanarBC& bc = M.prm.bcs.bc[2*a];
+      if (dmin(minimumDistance(bc.exit, r), minimumDistance(bc.enter, r)) <= nearReach) f = true;
+    }
+    return f;
+  };
+  int64_t before = 0, nnear = 0;
+  {
+    const int64_t chunk = (n + kClusterBlocks - 1)/kClusterBlocks;
+    const int64_t c0 = imin64(n, rank*chunk), c1 = imin64(n, c0 + chunk);
+    const int cnt = clusterCount(c0, c1, isNear);
+    if (threadIdx.x == 0) sh.count = cnt;
+    cl.sync();
+    if (w == 0) {
+      const int c = lane < kClusterBlocks ? cl.map_shared_rank(&sh, lane)->count : 0;
+      const int pre = __reduce_add_sync(0xffffffffu, lane < rank ? c : 0), all = __reduce_add_sync(0xffffffffu, c);
+      if (lane == 0) { sh.before = pre; sh.total = all; }
+    }
+    __syncthreads();
+    before = sh.before;
+    nnear = sh.total;
+    clusterScatter(sh, c0, c1, isNear, [&](int64_t i, int64_t k) { M.cidx[before + k] = (int32_t)i; });
+    cl.sync();
+  }
+  // the boundary passes (ghost_passes_fused_kernel)
+  const int64_t chunk = (nnear + kClusterBlocks - 1)/kClusterBlocks;
+  const int64_t c0 = imin64(nnear, rank*chunk), c1 = imin64(nnear, c0 + chunk);
+  for (int64_t t = c0 + threadIdx.x; t < c1; t += kRootThreads) M.counts[t] = 1;
+  for (int b = 0; b < 6; ++b) {
+    if (!M.prm.bcs.periodic[b >> 1]) continue;
+    double best = 0.0;
+    for (int64_t t = c0 + threadIdx.x; t < c1; t += kRootThreads) {
+      const int64_t k = __ldcg(M.cidx + t);
+      best = dmax(best, rootShare(M, nodePos(M, k), __ldcg(M.hmaxi + k), (uint32_t)M.counts[t], b));
+    }
+    best = blockMax(best, &sh.red[0][0]);
+    if (threadIdx.x == 0) sh.hmax[b] = best;
+    cl.sync();
+    if (w == 0) {
+      double x = cl.map_shared_rank(&sh, lane % kClusterBlocks)->hmax[b];
+      for (int o = kClusterBlocks/2; o > 0; o >>= 1) x = dmax(x, __shfl_xor_sync(0xffffffffu, x, o));
+      if (lane == 0) sh.all = x;
+    }
+    __syncthreads();
+    const double hmax = sh.all;
+    for (int64_t t = c0 + threadIdx.x; t < c1; t += kRootThreads)
+      M.counts[t] = (int32_t)rootImages(M, nodePos(M, __ldcg(M.cidx + t)), hmax, (uint32_t)M.counts[t], b);
+  }
+  countImages(M, c0, c1, sh.images);
+  cl.sync();
+  if (w == 0) {
+    int64_t mine = 0, pre = 0;
+    for (int k = 0; k < kClusterBlocks; ++k) {
+      const int c = cl.map_shared_rank(&sh, k)->images[lane];
+      if (k < rank) pre += c;
+      mine += c;
+    }
+    int64_t incl = mine;
+    for (int o = 1; o < 32; o <<= 1) {
+      const int64_t v = __shfl_up_sync(0xffffffffu, incl, o);
+      if (lane >= o) incl += v;
+    }
+    sh.next[lane] = incl - mine + pre;
+    if (lane == 31 && rank == 0) {
+      setScalI(M.scal, SC_NNEAR, nnear);
+      endGhosts(M, incl);
+    }
+  }
+  __syncthreads();
+  writeImages(M, c0, c1, sh.next, sh.warpCnt);
+  if (rank == 0 && threadIdx.x == 0) setGrid(M);
+  cl.sync();                      // no block leaves while another may read its shared memory
 }
 
 __device__ __forceinline__ int cellCoord(double x, double lo, double cell, int dim) {
@@ -1622,7 +1890,7 @@ int fused_ghost_grid() {
     int dev = 0, sms = 0, occ = 0;
     if (cudaGetDevice(&dev) != cudaSuccess ||
         cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess ||
-        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, ghost_passes_fused_kernel, kGhostThreads, 0) != cudaSuccess) {
+        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, ghost_passes_fused_kernel, kRootThreads, 0) != cudaSuccess) {
       cudaGetLastError();
       grid = 0;
     } else {
@@ -1640,7 +1908,7 @@ bool use_fused_ghost_passes(Batch& b) {
   if (b.ghostPasses == 1 || nm > kFusedGhostMembers || fused_ghost_grid() <= 0) return false;
   if (b.d_fuse == nullptr) {
     if (b.capturing) return false;
-    const size_t bytes = 2*sizeof(unsigned int) + sizeof(int64_t)*(size_t)kFusedGhostMembers*kFusedGhostBlocks + 8;
+    const size_t bytes = 2*sizeof(unsigned int) + sizeof(int)*(size_t)kFusedGhostMembers*kGhostCodes*kFusedGhostBlocks;
     if (dev_alloc(reinterpret_cast<void**>(&b.d_fuse), bytes) != cudaSuccess) { cudaGetLastError(); return false; }
     if (cudaMemset(b.d_fuse, 0, bytes) != cudaSuccess) { cudaGetLastError(); return false; }
   }
@@ -1650,7 +1918,7 @@ bool use_fused_ghost_passes(Batch& b) {
 int launch_fused_ghost_passes(Batch& b) {
   cudaLaunchConfig_t lc = {};
   lc.gridDim = dim3((unsigned)fused_ghost_grid());
-  lc.blockDim = dim3(kGhostThreads);
+  lc.blockDim = dim3(kRootThreads);
   lc.dynamicSmemBytes = 0;
   lc.stream = b.stream;
   cudaLaunchAttribute attr[1];
@@ -1671,42 +1939,50 @@ int launch_build(Batch& b) {
   if (!b.capturing && !b.buildPlanned) SPH_TRY(batch_upload(b));
   b.buildPlanned = false;
   // ---- ghosts: six planar boundaries in order, sizes kept on the device
-  build_init_kernel<<<(nm + 127)/128, 128, 0, st>>>(b.d_mem, nm); batch_count_launch(b);
   // fixed grids: at most kStreamBlocks blocks per member, member-local stride
   auto fixedItems = [](int64_t cap) { return cap < kStreamBlocks*kGhostThreads ? cap : kStreamBlocks*kGhostThreads; };
   BlockMap nmap, cap;
   unsigned ngrid = 0, capGrid = 0;
   SPH_TRY(batch_map_items(b, [&](const Problem& p) { return fixedItems(p.n); }, kGhostThreads, &nmap, &ngrid));
   SPH_TRY(batch_map_items(b, [&](const Problem& p) { return fixedItems(p.candcap); }, kGhostThreads, &cap, &capGrid));
-  if (ngrid) { node_hmax_kernel<<<ngrid, kGhostThreads, 0, st>>>(b.d_mem, nmap); batch_count_launch(b); }
   bool anyPeriodic = false;
   for (Problem* p : b.mem) for (int a = 0; a < 3; ++a) anyPeriodic = anyPeriodic || p->prm.bcs.periodic[a];
-  if (anyPeriodic) {
-    // the boundary passes visit only the internal nodes near a periodic plane
-    near_flag_kernel<<<ngrid, kGhostThreads, 0, st>>>(b.d_mem, nmap); batch_count_launch(b);
-    SPH_TRY(batch_scan(b, SCAN_COUNTS));
-    near_list_kernel<<<ngrid, kGhostThreads, 0, st>>>(b.d_mem, nmap); batch_count_launch(b);
+  bool small = b.ghostPasses == 0;
+  for (Problem* p : b.mem) small = small && p->n <= kClusterNodes;
+  if (small) {
+    // (the first pass's schedule value: all six passes in one launch)
+    if (anyPeriodic) b.lastGhostPasses = 2;
+    ghost_cluster_kernel<<<nm*kClusterBlocks, kClusterThreads, 0, st>>>(b.d_mem); batch_count_launch(b);
+  } else {
+    build_init_kernel<<<(nm + 127)/128, 128, 0, st>>>(b.d_mem, nm); batch_count_launch(b);
+    if (ngrid) { node_hmax_kernel<<<ngrid, kGhostThreads, 0, st>>>(b.d_mem, nmap); batch_count_launch(b); }
+    if (anyPeriodic) {
+      // the boundary passes visit only the internal nodes near a periodic plane
+      near_flag_kernel<<<ngrid, kGhostThreads, 0, st>>>(b.d_mem, nmap); batch_count_launch(b);
+      SPH_TRY(batch_scan(b, SCAN_COUNTS));
+      near_list_kernel<<<ngrid, kGhostThreads, 0, st>>>(b.d_mem, nmap); batch_count_launch(b);
+    }
+    const bool fused = anyPeriodic && use_fused_ghost_passes(b);
+    if (anyPeriodic) b.lastGhostPasses = fused ? 2 : 1;
+    if (fused) {
+      // (the barrier's arrival counter is back at zero after every completed
+      // barrier; a build that reported a timed-out barrier clears it)
+      SPH_TRY(launch_fused_ghost_passes(b));
+      batch_count_launch(b);
+    }
+    for (int bnd = 0; bnd < 6 && !fused; ++bnd) {
+      bool any = false;
+      for (Problem* p : b.mem) any = any || p->prm.bcs.periodic[bnd >> 1];
+      if (!any) continue;
+      ghost_hmax_kernel<<<capGrid, kGhostThreads, 0, st>>>(b.d_mem, cap, bnd); batch_count_launch(b);
+      ghost_flag_kernel<<<capGrid, kGhostThreads, 0, st>>>(b.d_mem, cap, bnd); batch_count_launch(b);
+      SPH_TRY(batch_scan(b, SCAN_FLAGS));
+      ghost_scatter_kernel<<<capGrid, kGhostThreads, 0, st>>>(b.d_mem, cap, bnd); batch_count_launch(b);
+      ghost_advance_kernel<<<(nm + 127)/128, 128, 0, st>>>(b.d_mem, nm); batch_count_launch(b);
+    }
+    grid_kernel<<<(nm + 127)/128, 128, 0, st>>>(b.d_mem, nm); batch_count_launch(b);
   }
-  const bool fused = anyPeriodic && use_fused_ghost_passes(b);
-  if (anyPeriodic) b.lastGhostPasses = fused ? 2 : 1;
-  if (fused) {
-    // (the barrier's arrival counter is back at zero after every completed
-    // barrier; a build that reported a timed-out barrier clears it)
-    SPH_TRY(launch_fused_ghost_passes(b));
-    batch_count_launch(b);
-  }
-  for (int bnd = 0; bnd < 6 && !fused; ++bnd) {
-    bool any = false;
-    for (Problem* p : b.mem) any = any || p->prm.bcs.periodic[bnd >> 1];
-    if (!any) continue;
-    ghost_hmax_kernel<<<capGrid, kGhostThreads, 0, st>>>(b.d_mem, cap, bnd); batch_count_launch(b);
-    ghost_flag_kernel<<<capGrid, kGhostThreads, 0, st>>>(b.d_mem, cap, bnd); batch_count_launch(b);
-    SPH_TRY(batch_scan(b, SCAN_FLAGS));
-    ghost_scatter_kernel<<<capGrid, kGhostThreads, 0, st>>>(b.d_mem, cap, bnd); batch_count_launch(b);
-    ghost_advance_kernel<<<(nm + 127)/128, 128, 0, st>>>(b.d_mem, nm); batch_count_launch(b);
-  }
-  // ---- cell grid and counting sort of all nodes by cell
-  grid_kernel<<<(nm + 127)/128, 128, 0, st>>>(b.d_mem, nm); batch_count_launch(b);
+  // ---- counting sort of all nodes by cell
   BlockMap cm;
   unsigned cgrid = 0;
   SPH_TRY(batch_map_items(b, [&](const Problem& p) { return fixedItems(p.cellcap); }, kGhostThreads, &cm, &cgrid));
