@@ -637,78 +637,48 @@ __device__ __forceinline__ void enforceNode(const Member& MB, int64_t i) {
 
 // ---------------------------------------------------------------- row sums
 // Loops that add one term per entry (summed density, compatible energy) or take
-// its maximum (the dt vote), for small problems: a warp takes a run of
-// consecutive rows, whose entries are consecutive.  Its lanes form the terms
-// of 32 entries at a time into shared memory, then lane r adds the terms of
-// row r in row order.
+// its maximum (the dt vote), for long rows: 16 lanes per node form the terms
+// of 16 consecutive entries into shared memory and add them in row order (every
+// lane the same sum).
 //
-// Why: with a thread per node every entry is a step of a serial chain of
-// dependent loads, 115 of them for a Sod node, and a few thousand nodes leave
-// the chip idle meanwhile.  Here only the addition is serial.  It costs more
-// instructions per entry (finding the row, the stores and loads of the terms,
-// few lanes adding), so the thread-per-node kernels are the faster ones once
-// the nodes fill the chip.  Measured (B200), thread per node -> rows, 4,096
-// Sod nodes: summed density (mixed) 61 -> 20 us, compatible energy 112 -> 16,
-// dt vote 59 -> 14; 262,144 nodes: dt vote 179 -> 391 us, Kelvin-Helmholtz with
-// 124,550 nodes of 7 entries: 16 -> 20.  The lines cross near 40,000 nodes (useRowSums).
-// The rows per warp follow the grid: as many as fill the chunk, fewer while
-// that leaves less than 16 warps per SM.
+// Why: with a thread per node a row of 115 entries is a serial chain of
+// dependent loads, and the index and pair-acceleration loads of a warp lie a
+// row apart, a sector fetched for each and lost from L1 before its next entry
+// is read.  Here the entries are read coalesced.  The 16 additions of a batch
+// are repeated by its lanes, which short rows would not pay back (longRows).
+// Measured (B200, Sod, thread per node -> 16 lanes): 4,096 nodes, mixed: summed
+// density 61 -> 17 us, compatible energy 112 -> 13, dt vote 59 -> 10; 262,144
+// nodes, FP64: compatible energy 700 -> 522 us (it reads 28 bytes an entry), but
+// summed density about 400 -> 684 and dt vote 179 -> 259, which read little per
+// entry and have threads enough there: those two take the lanes only while the
+// nodes are fewer than kRowSumNodes (the lines cross near 38,000 and 98,000).
 constexpr int kSumThreads = 256;
-constexpr int kSumWarps = kSumThreads/32;
-constexpr int kSumChunk = 512;                 // terms of a warp in shared memory
+constexpr int kSumLanes = 16;
+constexpr int kSumNodes = kSumThreads/kSumLanes;      // nodes of a block
 
-struct RowRun {
-  int64_t i0, e0;       // first node, its first entry
-  int rows, total;      // rows of the run, their entries
-  int rel, next;        // this lane's row: first entry and end, counted from e0
-};
-
-// rows per warp of a member in this launch (at most 32: the host's grids see to it)
-__device__ __forceinline__ int rowsPerWarp(int64_t n, int blocks) {
-  const int64_t warps = (int64_t)blocks*kSumWarps, r = (n + warps - 1)/warps;
-  return r > 32 ? 32 : (int)r;
-}
-
-__device__ __forceinline__ RowRun rowRun(const Member& MB, int64_t i0, int rowsMax) {
-  const int lane = threadIdx.x & 31;
-  RowRun R;
-  R.i0 = i0;
-  R.rows = MB.n - i0 < rowsMax ? (int)(MB.n - i0) : rowsMax;
-  const int64_t at = MB.offsets[i0 + (lane < R.rows ? lane : R.rows)];
-  R.e0 = __shfl_sync(0xffffffffu, at, 0);
-  R.total = (int)(MB.offsets[i0 + R.rows] - R.e0);
-  R.rel = (int)(at - R.e0);
-  const int nx = __shfl_down_sync(0xffffffffu, R.rel, 1);
-  R.next = lane == 31 ? R.total : nx;
-  return R;
-}
-
-// term(t, r, start): the term of the run's entry t, row r (which starts at
-// entry start); begin(): before the chunk's additions; step(t, v): entry t of
-// the lane's row has the term v.
-template<class V, class Term, class Begin, class Step>
-__device__ __forceinline__ void rowSums(const RowRun& R, V* buf, Term term, Begin begin, Step step) {
-  const int lane = threadIdx.x & 31;
-  const int top = R.rows > 1 ? 1 << (31 - __clz(R.rows - 1)) : 0;
-  for (int c0 = 0; c0 < R.total; c0 += kSumChunk) {
-    const int c1 = R.total - c0 < kSumChunk ? R.total : c0 + kSumChunk;
-    for (int b = c0; b < c1; b += 32) {
-      const int t = b + lane < c1 ? b + lane : c1 - 1;
-      int r = 0;                                    // the last row that starts at or before t
-      for (int w = top; w > 0; w >>= 1) {
-        const int s = __shfl_sync(0xffffffffu, R.rel, (r + w) & 31);
-        if (r + w < R.rows && s <= t) r += w;
-      }
-      const int start = __shfl_sync(0xffffffffu, R.rel, r);
-      if (b + lane < c1) buf[t - c0] = term(t, r, start);
+// term(k, j) of every entry k (neighbor j) of the group's row [k0, k1), then
+// step(v, j) in row order.
+template<class V, class Term, class Step>
+__device__ __forceinline__ void groupRow(const int32_t* nbr, int64_t k0, int64_t k1, V* terms, int32_t* js, Term term,
+                                         Step step) {
+  const int l = threadIdx.x % kSumLanes;
+  const unsigned half = 0xffffu << (threadIdx.x & 16);
+  for (int64_t base = k0; base < k1; base += kSumLanes) {
+    const int64_t k = base + l;
+    if (k < k1) {
+      const int32_t j = __ldg(nbr + k);
+      js[l] = j;
+      terms[l] = term(k, j);
     }
-    __syncwarp();
-    if (lane < R.rows) {
-      begin();
-      const int z = R.next < c1 ? R.next : c1;
-      for (int k = R.rel > c0 ? R.rel : c0; k < z; ++k) step(k, buf[k - c0]);
+    __syncwarp(half);
+    if (k1 - base >= kSumLanes) {
+#pragma unroll
+      for (int e = 0; e < kSumLanes; ++e) step(terms[e], js[e]);
+    } else {
+      const int valid = (int)(k1 - base);
+      for (int e = 0; e < valid; ++e) step(terms[e], js[e]);
     }
-    __syncwarp();
+    __syncwarp(half);
   }
 }
 
@@ -745,53 +715,37 @@ __global__ void __launch_bounds__(128) sum_density_kernel(const Member* mem, Blo
   if (enforce) enforceNode(MB, i);
 }
 
-// The same with a warp per run of rows (rowSums).
+// The same for long rows (groupRow).
 __global__ void __launch_bounds__(kSumThreads) sum_density_rows_kernel(const Member* mem, BlockMap bm, int enforce) {
-  __shared__ double buf[kSumWarps][kSumChunk];
-  __shared__ int selfAt[kSumWarps][32];           // entry of each row before which the self term is added
+  __shared__ double terms[kSumNodes][kSumLanes];
+  __shared__ int32_t js[kSumNodes][kSumLanes];
   const MemberBlock mb = memberBlock(bm);
   const Member& MB = mem[mb.m];
   const int64_t n = MB.n, cap = MB.candcap;
   const TableDev W = MB.prm.W;
   const double* rec = MB.rec;
-  const int32_t* nbr = MB.nbr;
-  const int lane = threadIdx.x & 31, wib = threadIdx.x >> 5;
-  const int rowsMax = rowsPerWarp(n, mb.blocks);
-  const int64_t stride = (int64_t)mb.blocks*kSumWarps*rowsMax;
-  for (int64_t i0 = (mb.block*kSumWarps + wib)*rowsMax; i0 < n; i0 += stride) {
-    const RowRun R = rowRun(MB, i0, rowsMax);
-    selfAt[wib][lane] = R.next;
-    __syncwarp();
-    double self = 0.0;
-    if (lane < R.rows) {
-      const double mi = ldg(rec + planeAt(cap, i0 + lane, 0) + R_M), Hdeti = ldg(rec + planeAt(cap, i0 + lane, 1));
-      self = mi*tableKernel(W, 0.0, Hdeti);
-    }
-    double rho = 0.0;
-    int sa = R.next;
-    rowSums(R, buf[wib],
-            [&](int t, int r, int start) {
-              const int64_t e = R.e0 + t;
-              const int32_t j = __ldg(nbr + e), i = (int32_t)(i0 + r);
-              if (j > i && (t == start || __ldg(nbr + e - 1) < i)) selfAt[wib][r] = t;
-              const D4 pi = ldPlane(rec + planeAt(cap, i, 0));
-              const Rec J = loadRec(rec, cap, j);
-              const V3 rij = vsub(V3{pi.a, pi.b, pi.c}, J.r);
-              const double eta = mag(isoSym(J.H) ? vmul(rij, J.H.xx) : sdot(J.H, rij));
-              return J.m*tableKernel(W, eta, J.Hdet);
-            },
-            [&]() { sa = selfAt[wib][lane]; },
-            [&](int t, double v) {
-              if (t == sa) rho += self;
-              rho += v;
-            });
-    if (lane < R.rows) {
-      if (sa == R.next) rho += self;              // no entry above the node
-      MB.S[S_RHO*n + i0 + lane] = rho;
-      if (enforce) enforceNode(MB, i0 + lane);
-    }
-    __syncwarp();
-  }
+  const int g = threadIdx.x/kSumLanes;
+  const int64_t i = mb.block*kSumNodes + g;
+  if (i >= n) return;
+  const D4 pi = ldPlane(rec + planeAt(cap, i, 0));
+  const double self = pi.d*tableKernel(W, 0.0, ldg(rec + planeAt(cap, i, 1)));
+  double rho = 0.0;
+  bool selfDone = false;
+  groupRow(MB.nbr, MB.offsets[i], MB.offsets[i + 1], terms[g], js[g],
+           [&](int64_t, int32_t j) {
+             const Rec J = loadRec(rec, cap, j);
+             const V3 rij = vsub(V3{pi.a, pi.b, pi.c}, J.r);
+             const double eta = mag(isoSym(J.H) ? vmul(rij, J.H.xx) : sdot(J.H, rij));
+             return J.m*tableKernel(W, eta, J.Hdet);
+           },
+           [&](double v, int32_t j) {
+             if (!selfDone && j > (int32_t)i) { rho += self; selfDone = true; }
+             rho += v;
+           });
+  if (threadIdx.x % kSumLanes) return;
+  if (!selfDone) rho += self;
+  MB.S[S_RHO*n + i] = rho;
+  if (enforce) enforceNode(MB, i);
 }
 
 // ---------------------------------------------------------------- summed density, mixed form
@@ -861,61 +815,45 @@ __global__ void __launch_bounds__(128) sum_density_mixed_kernel(const Member* me
   if (enforce) enforceNode(MB, i);
 }
 
-// The same with a warp per run of rows (rowSums).
+// The same for long rows (groupRow).
 __global__ void __launch_bounds__(kSumThreads) sum_density_mixed_rows_kernel(const Member* mem, BlockMap bm, int enforce) {
-  __shared__ float buf[kSumWarps][kSumChunk];
-  __shared__ int selfAt[kSumWarps][32];
+  __shared__ float terms[kSumNodes][kSumLanes];
+  __shared__ int32_t js[kSumNodes][kSumLanes];
   const MemberBlock mb = memberBlock(bm);
   const Member& MB = mem[mb.m];
   const int64_t n = MB.n, cap = MB.candcap;
   const Params& P = MB.prm;
   const float* coefF = MB.coefF;
   const double* mrec = MB.mrec;
-  const int32_t* nbr = MB.nbr;
   const int nt = P.W.n;
   const float invStep = (float)(1.0/P.W.stepSize), extent = (float)P.W.extent;
-  const int lane = threadIdx.x & 31, wib = threadIdx.x >> 5;
-  const int rowsMax = rowsPerWarp(n, mb.blocks);
-  const int64_t stride = (int64_t)mb.blocks*kSumWarps*rowsMax;
-  for (int64_t i0 = (mb.block*kSumWarps + wib)*rowsMax; i0 < n; i0 += stride) {
-    const RowRun R = rowRun(MB, i0, rowsMax);
-    selfAt[wib][lane] = R.next;
-    __syncwarp();
-    float self = 0.0f;
-    if (lane < R.rows) {
-      const D4 v = ldPlane(mrec + planeAt(cap, i0 + lane, 1));
-      self = loF(v.c)*tableW32(coefF, nt, invStep, extent, 0.0f, hiF(v.d));
-    }
-    KahanSum rho{0.0f, 0.0f};
-    int sa = R.next;
-    rowSums(R, buf[wib],
-            [&](int t, int r, int start) {
-              const int64_t e = R.e0 + t;
-              const int32_t j = __ldg(nbr + e), i = (int32_t)(i0 + r);
-              if (j > i && (t == start || __ldg(nbr + e - 1) < i)) selfAt[wib][r] = t;
-              const D4 pi = ldPlane(mrec + planeAt(cap, i, 0));
-              const D4 p = ldPlane(mrec + planeAt(cap, j, 0)), f0 = ldPlane(mrec + planeAt(cap, j, 1)),
-                       h = ldPlane(mrec + planeAt(cap, j, 2));
-              const float rx = (float)(pi.a - p.a), ry = (float)(pi.b - p.b), rz = (float)(pi.c - p.c);
-              const float xx = loF(h.a), xy = hiF(h.a), xz = loF(h.b), yy = hiF(h.b), yz = loF(h.c), zz = hiF(h.c);
-              const float ex = xx*rx + xy*ry + xz*rz;
-              const float ey = xy*rx + yy*ry + yz*rz;
-              const float ez = xz*rx + yz*ry + zz*rz;
-              const float eta = sqrtf(ex*ex + ey*ey + ez*ez);
-              return loF(f0.c)*tableW32(coefF, nt, invStep, extent, eta, hiF(f0.d));
-            },
-            [&]() { sa = selfAt[wib][lane]; },
-            [&](int t, float v) {
-              if (t == sa) rho.add(self);
-              rho.add(v);
-            });
-    if (lane < R.rows) {
-      if (sa == R.next) rho.add(self);
-      MB.S[S_RHO*n + i0 + lane] = rho.value();
-      if (enforce) enforceNode(MB, i0 + lane);
-    }
-    __syncwarp();
-  }
+  const int g = threadIdx.x/kSumLanes;
+  const int64_t i = mb.block*kSumNodes + g;
+  if (i >= n) return;
+  const D4 pi = ldPlane(mrec + planeAt(cap, i, 0)), vi = ldPlane(mrec + planeAt(cap, i, 1));
+  const float self = loF(vi.c)*tableW32(coefF, nt, invStep, extent, 0.0f, hiF(vi.d));
+  KahanSum rho{0.0f, 0.0f};
+  bool selfDone = false;
+  groupRow(MB.nbr, MB.offsets[i], MB.offsets[i + 1], terms[g], js[g],
+           [&](int64_t, int32_t j) {
+             const D4 p = ldPlane(mrec + planeAt(cap, j, 0)), f0 = ldPlane(mrec + planeAt(cap, j, 1)),
+                      h = ldPlane(mrec + planeAt(cap, j, 2));
+             const float rx = (float)(pi.a - p.a), ry = (float)(pi.b - p.b), rz = (float)(pi.c - p.c);
+             const float xx = loF(h.a), xy = hiF(h.a), xz = loF(h.b), yy = hiF(h.b), yz = loF(h.c), zz = hiF(h.c);
+             const float ex = xx*rx + xy*ry + xz*rz;
+             const float ey = xy*rx + yy*ry + yz*rz;
+             const float ez = xz*rx + yz*ry + zz*rz;
+             const float eta = sqrtf(ex*ex + ey*ey + ez*ez);
+             return loF(f0.c)*tableW32(coefF, nt, invStep, extent, eta, hiF(f0.d));
+           },
+           [&](float v, int32_t j) {
+             if (!selfDone && j > (int32_t)i) { rho.add(self); selfDone = true; }
+             rho.add(v);
+           });
+  if (threadIdx.x % kSumLanes) return;
+  if (!selfDone) rho.add(self);
+  MB.S[S_RHO*n + i] = rho.value();
+  if (enforce) enforceNode(MB, i);
 }
 
 // ---------------------------------------------------------------- compatible energy
@@ -966,64 +904,51 @@ __device__ __forceinline__ double compatibleDepsDt(const Member& MB, int64_t i, 
   return DepsDti;
 }
 
-// The same with a warp per run of rows (rowSums): each internal node's rate
-// into S0's rate column, for the full RK2 update that follows.
+// The same for long rows (groupRow): each internal node's rate into S0's rate
+// column, for the full RK2 update that follows.
 __global__ void __launch_bounds__(kSumThreads) compatible_energy_rows_kernel(const Member* mem, BlockMap bm, double scale) {
-  __shared__ double buf[kSumWarps][kSumChunk];
-  __shared__ double sRow[kSumWarps][32][4];        // half-step velocity, weight of the run's nodes
+  __shared__ double terms[kSumNodes][kSumLanes];
+  __shared__ int32_t js[kSumNodes][kSumLanes];
   const MemberBlock mb = memberBlock(bm);
   const Member& MB = mem[mb.m];
   const int64_t n = MB.n;
   const double* D = MB.D;
   const double* S = MB.S;
   const double* S0 = MB.S0;
-  const int32_t* nbr = MB.nbr;
   const int32_t* groot = MB.groot;
   const double* pacc = MB.pacc;
   const float* paccF = reinterpret_cast<const float*>(MB.pacc);
   const bool mixed = MB.prm.precision == SPHGPU_PRECISION_MIXED;
   const int64_t ecap = MB.ecap;
   const double hdt = 0.5*(scale*MB.scal[SC_DT]);
-  const int lane = threadIdx.x & 31, wib = threadIdx.x >> 5;
-  const int rowsMax = rowsPerWarp(n, mb.blocks);
-  const int64_t stride = (int64_t)mb.blocks*kSumWarps*rowsMax;
+  const int g = threadIdx.x/kSumLanes;
+  const int64_t i = mb.block*kSumNodes + g;
+  if (i >= n) return;
   auto half = [&](int64_t r) {
     const V3 v{S0[S_VX*n + r], S0[S_VY*n + r], S0[S_VZ*n + r]};
     const V3 a{ldg(D + (D_DVDT + 0)*n + r), ldg(D + (D_DVDT + 1)*n + r), ldg(D + (D_DVDT + 2)*n + r)};
     return vadd(v, vmul(a, hdt));
   };
-  for (int64_t i0 = (mb.block*kSumWarps + wib)*rowsMax; i0 < n; i0 += stride) {
-    const RowRun R = rowRun(MB, i0, rowsMax);
-    if (lane < R.rows) {
-      const V3 v = half(i0 + lane);
-      sRow[wib][lane][0] = v.x; sRow[wib][lane][1] = v.y; sRow[wib][lane][2] = v.z;
-      sRow[wib][lane][3] = fabs(ldg(D + D_DEPSDT*n + i0 + lane)) + kDblEps;
-    }
-    __syncwarp();
-    double rate = 0.0;
-    rowSums(R, buf[wib],
-            [&](int t, int row, int) {
-              const int64_t k = R.e0 + t, i = i0 + row;
-              const int32_t j = __ldg(nbr + k);
-              const int64_t r = j < n ? (int64_t)j : (int64_t)__ldg(groot + (j - n));
-              const double weightj = fabs(ldg(D + D_DEPSDT*n + r)) + kDblEps;
-              const V3 vj12 = half(r);
-              const V3 vi12{sRow[wib][row][0], sRow[wib][row][1], sRow[wib][row][2]};
-              const double weighti = sRow[wib][row][3];
-              // owner's pair acceleration (FP32 in the mixed form)
-              const V3 pa = mixed ? V3{(double)__ldg(paccF + k), (double)__ldg(paccF + ecap + k), (double)__ldg(paccF + 2*ecap + k)}
-                                  : V3{ldg(pacc + k), ldg(pacc + ecap + k), ldg(pacc + 2*ecap + k)};
-              const bool own = j > (int32_t)i;
-              const double w = (own ? weighti : weightj)/(weighti + weightj);
-              const double du = dot(own ? vsub(vj12, vi12) : vsub(vi12, vj12), pa);
-              if (own) return w*du;
-              const double mj = ldg(S + S_M*n + r), mi = ldg(S + S_M*n + i);       // mass is constant within the step
-              return (1.0 - w)*du*mj/mi;
-            },
-            []() {}, [&](int, double v) { rate += v; });
-    if (lane < R.rows) MB.S0[S0_RATE*n + i0 + lane] = rate;
-    __syncwarp();
-  }
+  const V3 vi12 = half(i);
+  const double weighti = fabs(ldg(D + D_DEPSDT*n + i)) + kDblEps;
+  const double mi = ldg(S + S_M*n + i);          // mass is constant within the step
+  double rate = 0.0;
+  groupRow(MB.nbr, MB.offsets[i], MB.offsets[i + 1], terms[g], js[g],
+           [&](int64_t k, int32_t j) {
+             const int64_t r = j < n ? (int64_t)j : (int64_t)__ldg(groot + (j - n));
+             const double weightj = fabs(ldg(D + D_DEPSDT*n + r)) + kDblEps;
+             const V3 vj12 = half(r);
+             // owner's pair acceleration (FP32 in the mixed form)
+             const V3 pa = mixed ? V3{(double)__ldg(paccF + k), (double)__ldg(paccF + ecap + k), (double)__ldg(paccF + 2*ecap + k)}
+                                 : V3{ldg(pacc + k), ldg(pacc + ecap + k), ldg(pacc + 2*ecap + k)};
+             const bool own = j > (int32_t)i;
+             const double w = (own ? weighti : weightj)/(weighti + weightj);
+             const double du = dot(own ? vsub(vj12, vi12) : vsub(vi12, vj12), pa);
+             if (own) return w*du;
+             return (1.0 - w)*du*ldg(S + S_M*n + r)/mi;
+           },
+           [&](double v, int32_t) { rate += v; });
+  if (threadIdx.x % kSumLanes == 0) MB.S0[S0_RATE*n + i] = rate;
 }
 
 // ---------------------------------------------------------------- policies
@@ -1269,38 +1194,58 @@ __global__ void __launch_bounds__(128) ideal_h_iter_kernel(const Member* mem, Bl
 // cachedEig: max eig(H) of each node is the one the neighbor build stored
 // (hmaxi[n + i]), valid when H has not changed since that build (the step's
 // selectDt, which follows the build); otherwise it is solved here.
+// The dt vote of node i; v2max: its neighbors' largest |vi - vj|^2 (-1: none).
+// min over the neighbors of nodeScale*safeInvVar(|vi - vj|): sqrt and the
+// division are correctly rounded and monotone, so it is the term of the
+// largest |vi - vj|^2, one sqrt and one division per node (bit-identical).
+__device__ __forceinline__ double nodeDt(const Member& MB, int64_t i, double v2max, int cachedEig) {
+  const int64_t n = MB.n;
+  const Params& P = MB.prm;
+  const double* S = MB.S;
+  const double* D = MB.D;
+  double minDt = kFltMax;
+  double lmax;
+  if (cachedEig) {
+    lmax = MB.hmaxi[n + i];
+  } else {
+    const Sym H{S[(S_H + 0)*n + i], S[(S_H + 1)*n + i], S[(S_H + 2)*n + i],
+                S[(S_H + 3)*n + i], S[(S_H + 4)*n + i], S[(S_H + 5)*n + i]};
+    lmax = vmax(eigenValues(H));
+  }
+  const double nodeScale = 1.0/lmax/P.nPerh;
+  const double cs = S[S_CS*n + i], rho = S[S_RHO*n + i];
+  const double csDt = nodeScale/(cs + kFltMin);
+  if (csDt < minDt) minDt = csDt;
+  const double csq = sqrt(D[D_MAXVP*n + i]/rho);
+  const double csqDt = nodeScale/(csq + kFltMin);
+  if (csqDt < minDt) minDt = csqDt;
+  const double divv = D[(D_DVDX + 0)*n + i] + D[(D_DVDX + 4)*n + i] + D[(D_DVDX + 8)*n + i];
+  const double divvDt = 1.0/(fabs(divv) + kFltMin);
+  if (divvDt < minDt) minDt = divvDt;
+  if (v2max >= 0.0) {
+    const double dtVelDiff = nodeScale*safeInvVar(sqrt(v2max), 1e-30);
+    if (dtVelDiff < minDt) minDt = dtVelDiff;
+  }
+  const V3 a{D[(D_DVDT + 0)*n + i], D[(D_DVDT + 1)*n + i], D[(D_DVDT + 2)*n + i]};
+  const double dtAcc = sqrt(nodeScale/(mag(a) + kFltMin));
+  if (dtAcc < minDt) minDt = dtAcc;
+  if (P.useVelMagDt) {
+    const V3 vi{S[S_VX*n + i], S[S_VY*n + i], S[S_VZ*n + i]};
+    const double velDt = nodeScale/(mag(vi) + 1.0e-10);
+    if (velDt < minDt) minDt = velDt;
+  }
+  return minDt;
+}
+
 __global__ void __launch_bounds__(128) hydro_dt_kernel(const Member* mem, BlockMap bm, int slot, int cachedEig) {
   const MemberBlock mb = memberBlock(bm);
   const Member& MB = mem[mb.m];
   const int64_t n = MB.n;
   const int64_t i = mb.block*blockDim.x + threadIdx.x;
-  const Params& P = MB.prm;
   const double* S = MB.S;
-  const double* D = MB.D;
   double minDt = kFltMax;
   if (i < n) {
-    double lmax;
-    if (cachedEig) {
-      lmax = MB.hmaxi[n + i];
-    } else {
-      const Sym H{S[(S_H + 0)*n + i], S[(S_H + 1)*n + i], S[(S_H + 2)*n + i],
-                  S[(S_H + 3)*n + i], S[(S_H + 4)*n + i], S[(S_H + 5)*n + i]};
-      lmax = vmax(eigenValues(H));
-    }
-    const double nodeScale = 1.0/lmax/P.nPerh;
-    const double cs = S[S_CS*n + i], rho = S[S_RHO*n + i];
-    const double csDt = nodeScale/(cs + kFltMin);
-    if (csDt < minDt) minDt = csDt;
-    const double csq = sqrt(D[D_MAXVP*n + i]/rho);
-    const double csqDt = nodeScale/(csq + kFltMin);
-    if (csqDt < minDt) minDt = csqDt;
-    const double divv = D[(D_DVDX + 0)*n + i] + D[(D_DVDX + 4)*n + i] + D[(D_DVDX + 8)*n + i];
-    const double divvDt = 1.0/(fabs(divv) + kFltMin);
-    if (divvDt < minDt) minDt = divvDt;
     const V3 vi{S[S_VX*n + i], S[S_VY*n + i], S[S_VZ*n + i]};
-    // min over the neighbors of nodeScale*safeInvVar(|vi - vj|): sqrt and the
-    // division are correctly rounded and monotone, so it is the term of the
-    // largest |vi - vj|^2, one sqrt and one division per node (bit-identical)
     double v2max = -1.0;
     for (int64_t k = MB.offsets[i]; k < MB.offsets[i + 1]; ++k) {
       const int32_t j = __ldg(MB.nbr + k);
@@ -1310,101 +1255,47 @@ __global__ void __launch_bounds__(128) hydro_dt_kernel(const Member* mem, BlockM
       const double v2 = d.x*d.x + d.y*d.y + d.z*d.z;
       if (v2 > v2max) v2max = v2;
     }
-    if (v2max >= 0.0) {
-      const double dtVelDiff = nodeScale*safeInvVar(sqrt(v2max), 1e-30);
-      if (dtVelDiff < minDt) minDt = dtVelDiff;
-    }
-    const V3 a{D[(D_DVDT + 0)*n + i], D[(D_DVDT + 1)*n + i], D[(D_DVDT + 2)*n + i]};
-    const double dtAcc = sqrt(nodeScale/(mag(a) + kFltMin));
-    if (dtAcc < minDt) minDt = dtAcc;
-    if (P.useVelMagDt) {
-      const double velDt = nodeScale/(mag(vi) + 1.0e-10);
-      if (velDt < minDt) minDt = velDt;
-    }
+    minDt = nodeDt(MB, i, v2max, cachedEig);
   }
   for (int o = 16; o > 0; o >>= 1) minDt = dmin(minDt, __shfl_xor_sync(0xffffffffu, minDt, o));
   if ((threadIdx.x & 31) == 0)
     atomicMin(reinterpret_cast<unsigned long long*>(MB.scal + slot), (unsigned long long)__double_as_longlong(minDt));
 }
 
-// The same with a warp per run of rows (rowSums).
+// The same for long rows: 16 lanes per node (a maximum needs no order).
 __global__ void __launch_bounds__(kSumThreads) hydro_dt_rows_kernel(const Member* mem, BlockMap bm, int slot, int cachedEig) {
-  __shared__ double buf[kSumWarps][kSumChunk];
-  __shared__ double sRow[kSumWarps][32][3];
-  __shared__ double least[kSumWarps];
+  __shared__ double v2[kSumNodes];
   const MemberBlock mb = memberBlock(bm);
   const Member& MB = mem[mb.m];
   const int64_t n = MB.n;
-  const Params& P = MB.prm;
   const double* S = MB.S;
-  const double* D = MB.D;
-  const int32_t* nbr = MB.nbr;
-  const int lane = threadIdx.x & 31, wib = threadIdx.x >> 5;
-  const int rowsMax = rowsPerWarp(n, mb.blocks);
-  const int64_t stride = (int64_t)mb.blocks*kSumWarps*rowsMax;
-  double minDt = kFltMax;
-  for (int64_t i0 = (mb.block*kSumWarps + wib)*rowsMax; i0 < n; i0 += stride) {
-    const RowRun R = rowRun(MB, i0, rowsMax);
-    const int64_t i = i0 + lane;
-    if (lane < R.rows) {
-#pragma unroll
-      for (int c = 0; c < 3; ++c) sRow[wib][lane][c] = S[(S_VX + c)*n + i];
-    }
-    __syncwarp();
-    // min over the neighbors of nodeScale*safeInvVar(|vi - vj|): sqrt and the
-    // division are correctly rounded and monotone, so it is the term of the
-    // largest |vi - vj|^2, one sqrt and one division per node (bit-identical)
+  const int g = threadIdx.x/kSumLanes, l = threadIdx.x % kSumLanes;
+  const unsigned half = 0xffffu << (threadIdx.x & 16);
+  const int64_t first = mb.block*kSumNodes, i = first + g;
+  if (i < n) {
+    const V3 vi{S[S_VX*n + i], S[S_VY*n + i], S[S_VZ*n + i]};
     double v2max = -1.0;
-    rowSums(R, buf[wib],
-            [&](int t, int row, int) {
-              const int32_t j = __ldg(nbr + R.e0 + t);
-              const int64_t r = j < n ? (int64_t)j : (int64_t)__ldg(MB.groot + (j - n));
-              const V3 d{sRow[wib][row][0] - ldg(S + S_VX*n + r), sRow[wib][row][1] - ldg(S + S_VY*n + r),
-                         sRow[wib][row][2] - ldg(S + S_VZ*n + r)};
-              return d.x*d.x + d.y*d.y + d.z*d.z;
-            },
-            []() {}, [&](int, double v2) { if (v2 > v2max) v2max = v2; });
-    if (lane < R.rows) {
-      double lmax;
-      if (cachedEig) {
-        lmax = MB.hmaxi[n + i];
-      } else {
-        const Sym H{S[(S_H + 0)*n + i], S[(S_H + 1)*n + i], S[(S_H + 2)*n + i],
-                    S[(S_H + 3)*n + i], S[(S_H + 4)*n + i], S[(S_H + 5)*n + i]};
-        lmax = vmax(eigenValues(H));
-      }
-      const double nodeScale = 1.0/lmax/P.nPerh;
-      const double cs = S[S_CS*n + i], rho = S[S_RHO*n + i];
-      const double csDt = nodeScale/(cs + kFltMin);
-      if (csDt < minDt) minDt = csDt;
-      const double csq = sqrt(D[D_MAXVP*n + i]/rho);
-      const double csqDt = nodeScale/(csq + kFltMin);
-      if (csqDt < minDt) minDt = csqDt;
-      const double divv = D[(D_DVDX + 0)*n + i] + D[(D_DVDX + 4)*n + i] + D[(D_DVDX + 8)*n + i];
-      const double divvDt = 1.0/(fabs(divv) + kFltMin);
-      if (divvDt < minDt) minDt = divvDt;
-      if (v2max >= 0.0) {
-        const double dtVelDiff = nodeScale*safeInvVar(sqrt(v2max), 1e-30);
-        if (dtVelDiff < minDt) minDt = dtVelDiff;
-      }
-      const V3 a{D[(D_DVDT + 0)*n + i], D[(D_DVDT + 1)*n + i], D[(D_DVDT + 2)*n + i]};
-      const double dtAcc = sqrt(nodeScale/(mag(a) + kFltMin));
-      if (dtAcc < minDt) minDt = dtAcc;
-      if (P.useVelMagDt) {
-        const V3 vi{sRow[wib][lane][0], sRow[wib][lane][1], sRow[wib][lane][2]};
-        const double velDt = nodeScale/(mag(vi) + 1.0e-10);
-        if (velDt < minDt) minDt = velDt;
-      }
+    const int64_t k1 = MB.offsets[i + 1];
+    for (int64_t k = MB.offsets[i] + l; k < k1; k += kSumLanes) {
+      const int32_t j = __ldg(MB.nbr + k);
+      const int64_t r = j < n ? (int64_t)j : (int64_t)__ldg(MB.groot + (j - n));
+      const V3 d = vsub(vi, V3{ldg(S + S_VX*n + r), ldg(S + S_VY*n + r), ldg(S + S_VZ*n + r)});
+      const double x = d.x*d.x + d.y*d.y + d.z*d.z;
+      if (x > v2max) v2max = x;
     }
-    __syncwarp();
+    for (int o = kSumLanes/2; o > 0; o >>= 1) {
+      const double x = __shfl_xor_sync(half, v2max, o);
+      if (x > v2max) v2max = x;
+    }
+    if (l == 0) v2[g] = v2max;
   }
-  for (int o = 16; o > 0; o >>= 1) minDt = dmin(minDt, __shfl_xor_sync(0xffffffffu, minDt, o));
-  if (lane == 0) least[wib] = minDt;
   __syncthreads();
-  if (threadIdx.x == 0) {
-    for (int w = 1; w < kSumWarps; ++w) minDt = dmin(minDt, least[w]);
+  if (threadIdx.x >= 32) return;
+  double minDt = kFltMax;
+  if (threadIdx.x < kSumNodes && first + threadIdx.x < n) minDt = nodeDt(MB, first + threadIdx.x, v2[threadIdx.x], cachedEig);
+  for (int o = 16; o > 0; o >>= 1) minDt = dmin(minDt, __shfl_xor_sync(0xffffffffu, minDt, o));
+  if (threadIdx.x == 0)
     atomicMin(reinterpret_cast<unsigned long long*>(MB.scal + slot), (unsigned long long)__double_as_longlong(minDt));
-  }
 }
 
 // Integrator::selectDt on the device: dt stays resident for the step kernels.
@@ -1521,26 +1412,20 @@ namespace {
 bool isSph(const Problem& p) { return p.prm.hydro == SPHGPU_HYDRO_SPH; }
 bool isFp64Sph(const Problem& p) { return isSph(p) && p.cfg.precision == SPHGPU_PRECISION_FP64; }
 
-// Fewer nodes than fill the chip with a thread each: the row-sum kernels (the
-// measured crossing is given there).
+// Nodes of a launch below which the summed density and the dt vote take 16
+// lanes per node of a long row (measured at groupRow).
 constexpr int64_t kRowSumNodes = 32768;
-bool useRowSums(const Batch& b) {
+bool fewNodes(const Batch& b) {
   int64_t nodes = 0;
   for (const Problem* p : b.mem) nodes += p->n;
   return nodes < kRowSumNodes;
 }
 
-// Blocks of the row-sum kernels: rows per warp by the mean row of the last
-// connectivity (any number is right, it sets the speed only).
+// The members of `want` with long rows (16 nodes a block) or without (128).
 template<class Want>
-int map_row_sums(Batch& b, Want want, BlockMap* bm, unsigned* grid) {
-  return batch_map_items(b, [&](const Problem& p) {
-    if (!want(p)) return (int64_t)0;
-    const int64_t mean = p.E > p.n ? p.E/p.n : 1;
-    int64_t rows = 32;
-    while (rows > 1 && rows*mean > kSumChunk) rows >>= 1;
-    while (rows > 1 && p.n < rows*148*16) rows >>= 1;
-    return kSumThreads*((p.n + rows*kSumWarps - 1)/(rows*kSumWarps)); }, kSumThreads, bm, grid);
+int map_sums(Batch& b, Want want, bool rows, BlockMap* bm, unsigned* grid) {
+  return batch_map_items(b, [&](const Problem& p) { return want(p) && longRows(p) == rows ? p.n : (int64_t)0; },
+                         rows ? kSumNodes : 128, bm, grid);
 }
 
 int map_nodes(Batch& b, int threads, BlockMap* bm, unsigned* grid) {
@@ -1712,13 +1597,12 @@ int launch_sum_density(Batch& b, bool enforce) {
   BlockMap bm;
   unsigned grid = 0;
   auto want = [](const Problem& p) { return isFp64Sph(p) && summedSph(p); };
-  if (useRowSums(b)) {
-    SPH_TRY(map_row_sums(b, want, &bm, &grid));
-    if (grid) { sum_density_rows_kernel<<<grid, kSumThreads, 0, b.stream>>>(b.d_mem, bm, enforce ? 1 : 0); batch_count_launch(b); }
-  } else {
-    SPH_TRY(batch_map_items(b, [&](const Problem& p) { return want(p) ? p.n : (int64_t)0; }, 128, &bm, &grid));
-    if (grid) { sum_density_kernel<<<grid, 128, 0, b.stream>>>(b.d_mem, bm, enforce ? 1 : 0); batch_count_launch(b); }
-  }
+  const bool lanes = fewNodes(b);
+  if (lanes) SPH_TRY(map_sums(b, want, true, &bm, &grid));
+  if (grid) { sum_density_rows_kernel<<<grid, kSumThreads, 0, b.stream>>>(b.d_mem, bm, enforce ? 1 : 0); batch_count_launch(b); }
+  if (lanes) SPH_TRY(map_sums(b, want, false, &bm, &grid));
+  else SPH_TRY(batch_map_items(b, [&](const Problem& p) { return want(p) ? p.n : (int64_t)0; }, 128, &bm, &grid));
+  if (grid) { sum_density_kernel<<<grid, 128, 0, b.stream>>>(b.d_mem, bm, enforce ? 1 : 0); batch_count_launch(b); }
   return cuda_status(cudaGetLastError(), "sum density");
 }
 
@@ -1728,13 +1612,12 @@ int launch_sum_density_mixed(Batch& b, bool enforce) {
   BlockMap bm;
   unsigned grid = 0;
   auto want = [](const Problem& p) { return p.cfg.precision == SPHGPU_PRECISION_MIXED && summedSph(p); };
-  if (useRowSums(b)) {
-    SPH_TRY(map_row_sums(b, want, &bm, &grid));
-    if (grid) { sum_density_mixed_rows_kernel<<<grid, kSumThreads, 0, b.stream>>>(b.d_mem, bm, enforce ? 1 : 0); batch_count_launch(b); }
-  } else {
-    SPH_TRY(batch_map_items(b, [&](const Problem& p) { return want(p) ? p.n : (int64_t)0; }, 128, &bm, &grid));
-    if (grid) { sum_density_mixed_kernel<<<grid, 128, 0, b.stream>>>(b.d_mem, bm, enforce ? 1 : 0); batch_count_launch(b); }
-  }
+  const bool lanes = fewNodes(b);
+  if (lanes) SPH_TRY(map_sums(b, want, true, &bm, &grid));
+  if (grid) { sum_density_mixed_rows_kernel<<<grid, kSumThreads, 0, b.stream>>>(b.d_mem, bm, enforce ? 1 : 0); batch_count_launch(b); }
+  if (lanes) SPH_TRY(map_sums(b, want, false, &bm, &grid));
+  else SPH_TRY(batch_map_items(b, [&](const Problem& p) { return want(p) ? p.n : (int64_t)0; }, 128, &bm, &grid));
+  if (grid) { sum_density_mixed_kernel<<<grid, 128, 0, b.stream>>>(b.d_mem, bm, enforce ? 1 : 0); batch_count_launch(b); }
   return cuda_status(cudaGetLastError(), "sum density (mixed)");
 }
 
@@ -1743,25 +1626,35 @@ int launch_update(Batch& b, double scale, bool timeAdvanceOnly, int mode, int pa
     set_error("a record-only mid-point update packs the mid-point records");
     return SPHGPU_ERR_ARG;
   }
-  BlockMap bm;
-  unsigned grid = 0;
-  SPH_TRY(map_nodes(b, 128, &bm, &grid));
   b.packedByUpdate = packMode;
   b.midInS0 = recordMid && mode == UPDATE_SAVE_START;
   const int rm = recordMid ? 1 : 0;
-  if (grid) {
-    bool compat = false;
-    if (!timeAdvanceOnly && mode == UPDATE_FROM_START) for (const Problem* p : b.mem) compat = compat || p->prm.compatible;
-    const bool rows = compat && useRowSums(b);
-    if (rows) {
-      BlockMap cm;
-      unsigned cgrid = 0;
-      SPH_TRY(map_row_sums(b, [](const Problem& p) { return p.prm.compatible != 0; }, &cm, &cgrid));
-      compatible_energy_rows_kernel<<<cgrid, kSumThreads, 0, b.stream>>>(b.d_mem, cm, scale);
+  bool compat = false;
+  if (!timeAdvanceOnly && mode == UPDATE_FROM_START) for (const Problem* p : b.mem) compat = compat || p->prm.compatible;
+  BlockMap bm;
+  unsigned grid = 0;
+  if (!compat) {
+    SPH_TRY(map_nodes(b, 128, &bm, &grid));
+    if (grid) {
+      update_kernel<false><<<grid, 128, 0, b.stream>>>(b.d_mem, bm, scale, timeAdvanceOnly ? 1 : 0, mode, packMode, rm, 0);
       batch_count_launch(b);
     }
-    if (compat && !rows) update_kernel<true><<<grid, 128, 0, b.stream>>>(b.d_mem, bm, scale, 0, mode, packMode, rm, 0);
-    else update_kernel<false><<<grid, 128, 0, b.stream>>>(b.d_mem, bm, scale, timeAdvanceOnly ? 1 : 0, mode, packMode, rm, rows ? 1 : 0);
+    return cuda_status(cudaGetLastError(), "update");
+  }
+  // the compatible energy of the members with long rows by its own kernel, of
+  // the others inside their update
+  auto byRate = [](const Problem& p) { return p.prm.compatible && longRows(p); };
+  SPH_TRY(map_sums(b, byRate, true, &bm, &grid));
+  if (grid) {
+    compatible_energy_rows_kernel<<<grid, kSumThreads, 0, b.stream>>>(b.d_mem, bm, scale);
+    batch_count_launch(b);
+    SPH_TRY(batch_map_items(b, [&](const Problem& p) { return byRate(p) ? p.n : (int64_t)0; }, 128, &bm, &grid));
+    update_kernel<false><<<grid, 128, 0, b.stream>>>(b.d_mem, bm, scale, 0, mode, packMode, rm, 1);
+    batch_count_launch(b);
+  }
+  SPH_TRY(batch_map_items(b, [&](const Problem& p) { return byRate(p) ? (int64_t)0 : p.n; }, 128, &bm, &grid));
+  if (grid) {
+    update_kernel<true><<<grid, 128, 0, b.stream>>>(b.d_mem, bm, scale, 0, mode, packMode, rm, 0);
     batch_count_launch(b);
   }
   return cuda_status(cudaGetLastError(), "update");
@@ -1800,13 +1693,13 @@ int launch_dt(Batch& b, int slot, bool cachedEig) {
   batch_set_scal(b, slot, kFltMax);
   BlockMap bm;
   unsigned grid = 0;
-  if (useRowSums(b)) {
-    SPH_TRY(map_row_sums(b, [](const Problem&) { return true; }, &bm, &grid));
-    if (grid) { hydro_dt_rows_kernel<<<grid, kSumThreads, 0, b.stream>>>(b.d_mem, bm, slot, cachedEig ? 1 : 0); batch_count_launch(b); }
-  } else {
-    SPH_TRY(map_nodes(b, 128, &bm, &grid));
-    if (grid) { hydro_dt_kernel<<<grid, 128, 0, b.stream>>>(b.d_mem, bm, slot, cachedEig ? 1 : 0); batch_count_launch(b); }
-  }
+  auto all = [](const Problem&) { return true; };
+  const bool lanes = fewNodes(b);
+  if (lanes) SPH_TRY(map_sums(b, all, true, &bm, &grid));
+  if (grid) { hydro_dt_rows_kernel<<<grid, kSumThreads, 0, b.stream>>>(b.d_mem, bm, slot, cachedEig ? 1 : 0); batch_count_launch(b); }
+  if (lanes) SPH_TRY(map_sums(b, all, false, &bm, &grid));
+  else SPH_TRY(map_nodes(b, 128, &bm, &grid));
+  if (grid) { hydro_dt_kernel<<<grid, 128, 0, b.stream>>>(b.d_mem, bm, slot, cachedEig ? 1 : 0); batch_count_launch(b); }
   return cuda_status(cudaGetLastError(), "dt");
 }
 
