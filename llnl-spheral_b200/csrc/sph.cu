@@ -648,7 +648,7 @@ __device__ __forceinline__ void enforceNode(const Member& MB, int64_t i) {
 // are repeated by its lanes, which short rows would not pay back (longRows).
 // Measured (B200, Sod, thread per node -> 16 lanes): 4,096 nodes, mixed: summed
 // density 61 -> 17 us, compatible energy 112 -> 13, dt vote 59 -> 10; 262,144
-// nodes, FP64: compatible energy 700 -> 522 us (it reads 28 bytes an entry), but
+// nodes, FP64: compatible energy 700 -> 522 us (28 bytes of pair data an entry), but
 // summed density about 400 -> 684 and dt vote 179 -> 259, which read little per
 // entry and have threads enough there: those two take the lanes only while the
 // nodes are fewer than kRowSumNodes (the lines cross near 38,000 and 98,000).
@@ -904,45 +904,64 @@ __device__ __forceinline__ double compatibleDepsDt(const Member& MB, int64_t i, 
   return DepsDti;
 }
 
+// What the compatible energy of long rows reads of a neighbor, in one 32-byte
+// plane per internal node: the half-step velocity v + a dt/2 of the start-of-step state
+// S0 and the weight |DepsDt| + eps.  The planes lie in the cell-ordered
+// candidate arrays, which hold nothing between the walk and the next build
+// (CAND_DOUBLES for each of at least 1.5 n slots).  One streaming pass in place
+// of seven 8-byte gathers per entry.  Measured (B200): Sod 262,144 nodes 522 ->
+// 476 + 6 us, the ensemble's 24 tubes (mixed) 2,260 -> 2,009 + 20 us.  With the
+// 8 entries of a Kelvin-Helmholtz row in lattice order the pass costs more than
+// it saves (327 -> 315 + 31 us of the update), so short rows gather the fields.
+__device__ __forceinline__ double* halfStepPlanes(const Member& MB) { return static_cast<double*>(MB.cand); }
+
+__global__ void __launch_bounds__(256) half_step_kernel(const Member* mem, BlockMap bm, double scale) {
+  const MemberBlock mb = memberBlock(bm);
+  const Member& MB = mem[mb.m];
+  const int64_t n = MB.n;
+  const int64_t i = mb.block*blockDim.x + threadIdx.x;
+  if (i >= n) return;
+  const double* D = MB.D;
+  const double* S0 = MB.S0;
+  const double hdt = 0.5*(scale*MB.scal[SC_DT]);
+  const V3 v{S0[S_VX*n + i], S0[S_VY*n + i], S0[S_VZ*n + i]};
+  const V3 a{D[(D_DVDT + 0)*n + i], D[(D_DVDT + 1)*n + i], D[(D_DVDT + 2)*n + i]};
+  const V3 h = vadd(v, vmul(a, hdt));
+  stPlane(halfStepPlanes(MB) + 4*i, h.x, h.y, h.z, fabs(D[D_DEPSDT*n + i]) + kDblEps);
+}
+
 // The same for long rows (groupRow): each internal node's rate into S0's rate
 // column, for the full RK2 update that follows.
-__global__ void __launch_bounds__(kSumThreads) compatible_energy_rows_kernel(const Member* mem, BlockMap bm, double scale) {
+__global__ void __launch_bounds__(kSumThreads) compatible_energy_rows_kernel(const Member* mem, BlockMap bm) {
   __shared__ double terms[kSumNodes][kSumLanes];
   __shared__ int32_t js[kSumNodes][kSumLanes];
   const MemberBlock mb = memberBlock(bm);
   const Member& MB = mem[mb.m];
   const int64_t n = MB.n;
-  const double* D = MB.D;
   const double* S = MB.S;
-  const double* S0 = MB.S0;
+  const double* H = halfStepPlanes(MB);
   const int32_t* groot = MB.groot;
   const double* pacc = MB.pacc;
   const float* paccF = reinterpret_cast<const float*>(MB.pacc);
   const bool mixed = MB.prm.precision == SPHGPU_PRECISION_MIXED;
   const int64_t ecap = MB.ecap;
-  const double hdt = 0.5*(scale*MB.scal[SC_DT]);
   const int g = threadIdx.x/kSumLanes;
   const int64_t i = mb.block*kSumNodes + g;
   if (i >= n) return;
-  auto half = [&](int64_t r) {
-    const V3 v{S0[S_VX*n + r], S0[S_VY*n + r], S0[S_VZ*n + r]};
-    const V3 a{ldg(D + (D_DVDT + 0)*n + r), ldg(D + (D_DVDT + 1)*n + r), ldg(D + (D_DVDT + 2)*n + r)};
-    return vadd(v, vmul(a, hdt));
-  };
-  const V3 vi12 = half(i);
-  const double weighti = fabs(ldg(D + D_DEPSDT*n + i)) + kDblEps;
+  const D4 pi = ldPlane(H + 4*i);
+  const V3 vi12{pi.a, pi.b, pi.c};
   const double mi = ldg(S + S_M*n + i);          // mass is constant within the step
   double rate = 0.0;
   groupRow(MB.nbr, MB.offsets[i], MB.offsets[i + 1], terms[g], js[g],
            [&](int64_t k, int32_t j) {
              const int64_t r = j < n ? (int64_t)j : (int64_t)__ldg(groot + (j - n));
-             const double weightj = fabs(ldg(D + D_DEPSDT*n + r)) + kDblEps;
-             const V3 vj12 = half(r);
+             const D4 pj = ldPlane(H + 4*r);
+             const V3 vj12{pj.a, pj.b, pj.c};
              // owner's pair acceleration (FP32 in the mixed form)
              const V3 pa = mixed ? V3{(double)__ldg(paccF + k), (double)__ldg(paccF + ecap + k), (double)__ldg(paccF + 2*ecap + k)}
                                  : V3{ldg(pacc + k), ldg(pacc + ecap + k), ldg(pacc + 2*ecap + k)};
              const bool own = j > (int32_t)i;
-             const double w = (own ? weighti : weightj)/(weighti + weightj);
+             const double w = (own ? pi.d : pj.d)/(pi.d + pj.d);
              const double du = dot(own ? vsub(vj12, vi12) : vsub(vi12, vj12), pa);
              if (own) return w*du;
              return (1.0 - w)*du*ldg(S + S_M*n + r)/mi;
@@ -1644,9 +1663,12 @@ int launch_update(Batch& b, double scale, bool timeAdvanceOnly, int mode, int pa
   // the compatible energy of the members with long rows by its own kernel, of
   // the others inside their update
   auto byRate = [](const Problem& p) { return p.prm.compatible && longRows(p); };
-  SPH_TRY(map_sums(b, byRate, true, &bm, &grid));
+  SPH_TRY(batch_map_items(b, [&](const Problem& p) { return byRate(p) ? p.n : (int64_t)0; }, 256, &bm, &grid));
   if (grid) {
-    compatible_energy_rows_kernel<<<grid, kSumThreads, 0, b.stream>>>(b.d_mem, bm, scale);
+    half_step_kernel<<<grid, 256, 0, b.stream>>>(b.d_mem, bm, scale);
+    batch_count_launch(b);
+    SPH_TRY(map_sums(b, byRate, true, &bm, &grid));
+    compatible_energy_rows_kernel<<<grid, kSumThreads, 0, b.stream>>>(b.d_mem, bm);
     batch_count_launch(b);
     SPH_TRY(batch_map_items(b, [&](const Problem& p) { return byRate(p) ? p.n : (int64_t)0; }, 128, &bm, &grid));
     update_kernel<false><<<grid, 128, 0, b.stream>>>(b.d_mem, bm, scale, 0, mode, packMode, rm, 1);
