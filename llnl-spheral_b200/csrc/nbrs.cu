@@ -1406,10 +1406,14 @@ __global__ void __launch_bounds__(256) nbr_walk_kernel(const Member* mem, BlockM
 // two other runs.
 //
 // Measured (B200): Sod 256x32x32 (262,144 nodes, 115 neighbors) 786 us against
-// 1,939 us with a warp per node; 24 tubes of the ensemble together 3.17 against
-// 8.92 ms.  Bound by instruction issue (about half of the cycles issue, 32
-// warps per SM): a fifth of the instructions are the merges, the rest the
-// tests and the lists' stores.
+// 1,939 us with a warp per node; 24 tubes of the ensemble together 2.83 against
+// 8.92 ms.  Bound by the latency of its steps between barriers (32 warps per
+// SM, about half of the cycles issue): the merges' bisections, then the tests
+// and the lists' stores.  With the bisections in the two other runs one after
+// the other and a warp per 32 elements of one run the merges took 23,000 of a
+// cell's 60,000 cycles, and the walk 786 us.  Loading the 27 cells ahead of
+// the first test: 786 us again (the registers spill); a list's places from a
+// scan of its words' counts instead of one after the other: 702 us.
 constexpr int kCellThreads = 256;
 constexpr int kCellWarps = kCellThreads/32;
 constexpr int kCellCand = 1536;                        // nodes of the 27 cells that can be staged (more: walkWarp)
@@ -1469,42 +1473,42 @@ __global__ void __launch_bounds__(256) cell_order_kernel(const Member* mem, Bloc
   }
 }
 
-// Elements of the ascending run key[0 : len) below k.
-__device__ __forceinline__ int runRank(const int32_t* key, int len, int32_t k) {
-  int lo = 0;
-  if (len <= 0) return 0;
-  while (len > 1) {
-    const int half = len >> 1;
-    if (key[lo + half - 1] < k) lo += half;
-    len -= half;
+// Elements below k of the ascending runs a[0 : la) and b[0 : lb), summed (the
+// two bisections' reads overlap).
+__device__ __forceinline__ int rankInTwo(const int32_t* a, int la, const int32_t* b, int lb, int32_t k) {
+  int x = 0, y = 0;
+  const int most = la > lb ? la : lb;
+  for (int w = most > 0 ? 1 << (31 - __clz(most)) : 0; w > 0; w >>= 1) {
+    const bool ga = x + w <= la && a[x + w - 1] < k, gb = y + w <= lb && b[y + w - 1] < k;
+    x += ga ? w : 0;
+    y += gb ? w : 0;
   }
-  return lo + (key[lo] < k);
+  return x + y;
 }
 
 // Merge of the ascending runs 3g, 3g + 1, 3g + 2 (run r at [start[r],
 // start[r + 1])) of every g from (key, src) to (keyTo, srcTo), each element at
-// the rank it has among the three.  A warp takes 32 elements of one run at a
-// time, so that the bisections' lengths are the same for its lanes.
+// the rank it has among the three.
 // own (the last merge): the final place of the element staged at ownAt + m
 // goes to own[m], m < ownLen.
+template<int RUNS>
 __device__ __forceinline__ void mergeRuns(const int32_t* key, const uint16_t* src, int32_t* keyTo, uint16_t* srcTo,
-                                          const int* start, int runs, uint16_t* own = nullptr, int ownAt = 0,
-                                          int ownLen = 0) {
-  const int lane = threadIdx.x & 31, wib = threadIdx.x >> 5;
-  int task = 0;
-  for (int r = 0; r < runs; ++r) {
-    const int at = start[r], len = start[r + 1] - at, g = r - r % 3;
+                                          const int* start, uint16_t* own = nullptr, int ownAt = 0, int ownLen = 0) {
+  const int count = start[RUNS];
+  for (int t = threadIdx.x; t < count; t += kCellThreads) {
+    int r = 0;
+#pragma unroll
+    for (int q = 1; q < RUNS; ++q) r += start[q] <= t;
+    const int g = r - r % 3;
     const int o1 = r == g ? g + 1 : g, o2 = r == g + 2 ? g + 1 : g + 2;
-    for (int base = 0; base < len; base += 32, ++task) {
-      if (task % kCellWarps != wib || base + lane >= len) continue;
-      const int32_t k = key[at + base + lane];
-      const int to = start[g] + base + lane + runRank(key + start[o1], start[o1 + 1] - start[o1], k) +
-                     runRank(key + start[o2], start[o2 + 1] - start[o2], k);
-      const uint16_t from = src[at + base + lane];
-      keyTo[to] = k;
-      srcTo[to] = from;
-      if (own != nullptr && (unsigned)(from - ownAt) < (unsigned)ownLen) own[from - ownAt] = (uint16_t)to;
-    }
+    const int a1 = start[o1], a2 = start[o2];
+    const int32_t k = key[t];
+    const uint16_t from = src[t];
+    const int to = start[g] + (t - start[r]) +
+                   rankInTwo(key + a1, start[o1 + 1] - a1, key + a2, start[o2 + 1] - a2, k);
+    keyTo[to] = k;
+    srcTo[to] = from;
+    if (own != nullptr && (unsigned)(from - ownAt) < (unsigned)ownLen) own[from - ownAt] = (uint16_t)to;
   }
 }
 
@@ -1663,16 +1667,15 @@ __global__ void __launch_bounds__(kCellThreads, 4) nbr_cell_kernel(const Member*
       const int len = cellLen[q], at = cellAt[q], r = q/3, o1 = 3*r + (q + 1) % 3, o2 = 3*r + (q + 2) % 3;
       for (int t = lane; t < len; t += 32) {
         const int32_t k = sh.key[0][at + t];
-        const int to = rowAt[r] + t + runRank(sh.key[0] + cellAt[o1], cellLen[o1], k) +
-                       runRank(sh.key[0] + cellAt[o2], cellLen[o2], k);
+        const int to = rowAt[r] + t + rankInTwo(sh.key[0] + cellAt[o1], cellLen[o1], sh.key[0] + cellAt[o2], cellLen[o2], k);
         sh.key[1][to] = k;
         sh.src[1][to] = (uint16_t)(at + t);
       }
     }
     __syncthreads();
-    mergeRuns(sh.key[1], sh.src[1], sh.key[0], sh.src[0], rowAt, 9);
+    mergeRuns<9>(sh.key[1], sh.src[1], sh.key[0], sh.src[0], rowAt);
     __syncthreads();
-    mergeRuns(sh.key[0], sh.src[0], sh.key[1], sh.src[1], planeAt, 3, sh.own, cellAt[13], cellLen[13]);
+    mergeRuns<3>(sh.key[0], sh.src[0], sh.key[1], sh.src[1], planeAt, sh.own, cellAt[13], cellLen[13]);
     __syncthreads();
     const int32_t* key = sh.key[1];
     const uint16_t* src = sh.src[1];
