@@ -323,15 +323,17 @@ int sphgpu_kernel_launches(sphgpu_problem* p, int64_t* launches);
  * 1 = cells of one reach (27-cell window), 2 = cells of half a reach
  * (125-cell window, rows and cells beyond the reach skipped).  Same
  * ConnectivityMap either way.  stage "ghost passes": the six periodic
- * boundary passes of the ghost build, 0 = automatic (2 for a problem or a
- * batch of at most 4 members, else 1), 1 = four launches and a prefix sum
- * per pass, 2 = all six passes in one cooperative launch with grid
- * barriers.  Same ghosts in the same order either way.
+ * boundary passes of the ghost build, 0 = automatic (while every member has
+ * at most 32,768 nodes: one launch with a thread-block cluster per member;
+ * otherwise 2 for a problem or a batch of at most 4 members, else 1), 1 =
+ * four launches and a prefix sum per pass, 2 = all six passes in one
+ * cooperative launch with grid barriers.  Same ghosts in the same order
+ * either way.
  * sphgpu_get_schedule reports what the last call used. */
 int sphgpu_set_schedule(sphgpu_problem* p, const char* stage, int32_t schedule);
 int sphgpu_get_schedule(sphgpu_problem* p, const char* stage, int32_t* schedule);
-/* Autotuner: times every schedule of the neighbor walk (thread or warp per
- * node, then cells of one or half a kernel reach) and of the pair loop on
+/* Autotuner: times every schedule of the neighbor walk (thread per node, or 2
+ * above, then cells of one or half a kernel reach) and of the pair loop on
  * the problem's own data (CUDA events, median of three) and keeps the
  * fastest.  Results do not depend on the schedule; the call leaves the
  * connectivity rebuilt and the derivatives evaluated at the current state (as

@@ -18,12 +18,16 @@
 // launches every stage, and reads the sizes back once at the end; a capacity
 // overflow sets an error bit and the build is redone with larger buffers.
 //
-// Kernels and their bounds (see the roofline notes in the design document):
+// Kernels and their bounds:
+//   ghost_cluster                            all ghost passes of a small member
+//                                            by one cluster: barrier latency
+//   ghost_passes_fused                       ... of a large one by one
+//                                            cooperative launch: the same
 //   ghost_hmax / ghost_flag / ghost_scatter  O(N+G) streaming, HBM bound
 //   node_bounds / cell_index / cell_scatter  O(N+G) streaming + atomics
 //   nbr_thread<COUNT|FILL>                   thread per node (cell-sorted
 //                                            order) over the 27 neighbouring
-//                                            cells; 64-byte candidate records
+//                                            cells; 16-byte candidate records
 //                                            shared by a warp through L1
 //   nbr_cell<COUNT|FILL>                     block per cell, for large
 //                                            candidate sets: the window
@@ -1199,7 +1203,9 @@ __global__ void __launch_bounds__(256, SUB == 1 ? NBR_THREAD_MIN_BLOCKS : 1) nbr
   }
 }
 
-// Stashed lists (thread schedule) to the CSR: thread per sorted slot.
+// Stashed lists (thread schedule) to the CSR: thread per sorted slot, eight
+// entries loaded before the first is stored (one after the other the loads'
+// latency bound it; Kelvin-Helmholtz 128^3 60 -> 42 us).
 __global__ void __launch_bounds__(256) nbr_compact_thread_kernel(const Member* mem, BlockMap bm) {
   const MemberBlock mb = memberBlock(bm);
   const Member& M = mem[mb.m];
@@ -1216,11 +1222,21 @@ __global__ void __launch_bounds__(256) nbr_compact_thread_kernel(const Member* m
     return;
   }
   const int32_t* stash = reinterpret_cast<const int32_t*>(M.pacc);
-  for (int c = 0; c < count; ++c) M.nbr[o + c] = stash[c*stride + s];
+  int32_t* to = M.nbr + o;
+  for (int base = 0; base < count; base += 8) {
+    int32_t v[8];
+#pragma unroll
+    for (int u = 0; u < 8; ++u)
+      if (base + u < count) v[u] = __ldg(stash + (base + u)*stride + s);
+#pragma unroll
+    for (int u = 0; u < 8; ++u)
+      if (base + u < count) to[base + u] = v[u];
+  }
 }
 
 // Stashed lists (warp schedule) to the CSR: warp per internal node, the list
-// of node i at stash[i*stashCap : i*stashCap + count].
+// of node i at stash[i*stashCap : i*stashCap + count].  Four loads per lane in
+// flight: Sod 256x32x32 121 -> 82 us (3 TB/s), 24 tubes 570 -> 410 us.
 __global__ void __launch_bounds__(256) nbr_compact_warp_kernel(const Member* mem, BlockMap bm) {
   const MemberBlock mb = memberBlock(bm);
   const Member& M = mem[mb.m];
@@ -1235,7 +1251,20 @@ __global__ void __launch_bounds__(256) nbr_compact_warp_kernel(const Member* mem
     return;
   }
   const int32_t* stash = reinterpret_cast<const int32_t*>(M.pacc) + i*(int64_t)M.grid.stashCap;
-  for (int t = lane; t < count; t += 32) M.nbr[o + t] = stash[t];
+  int32_t* to = M.nbr + o;
+  for (int base = 0; base < count; base += 128) {
+    int32_t v[4];
+#pragma unroll
+    for (int u = 0; u < 4; ++u) {
+      const int t = base + 32*u + lane;
+      if (t < count) v[u] = __ldg(stash + t);
+    }
+#pragma unroll
+    for (int u = 0; u < 4; ++u) {
+      const int t = base + 32*u + lane;
+      if (t < count) to[t] = v[u];
+    }
+  }
 }
 
 // One warp walks the neighbouring cells of the node in sorted slot s (nothing
