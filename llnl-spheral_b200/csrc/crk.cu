@@ -51,7 +51,7 @@ struct CRec {
 
 __device__ __forceinline__ CRec loadCRec(const double* crec, int64_t cap, int64_t k) {
   double d[CRECW];
-  ldPlanes<CRECW/4, true>(crec, cap, k, d);
+  ldPlanes<CRECW/4, true, false>(crec, cap, k, d);
   CRec R;
   R.r = V3{d[C_X], d[C_Y], d[C_Z]};
   R.v = V3{d[C_VX], d[C_VY], d[C_VZ]};
@@ -99,7 +99,7 @@ __global__ void __launch_bounds__(256) pack_crk_records_kernel(const Member* mem
     for (int c = 0; c < 9; ++c) v[C_GRADB + c] = K[(K_GRADB + c)*n + r];
     const int64_t cap = MB.candcap;
 #pragma unroll
-    for (int t = 0; t < CRECW/4; ++t) stPlane(crec + planeAt(cap, k, t), v[4*t], v[4*t + 1], v[4*t + 2], v[4*t + 3]);
+    for (int t = 0; t < CRECW/4; ++t) stPlane(crec + planeAt<false>(cap, k, t), v[4*t], v[4*t + 1], v[4*t + 2], v[4*t + 3]);
     *reinterpret_cast<double2*>(crec + halfPlaneAt(cap, k, CRECW/4)) = make_double2(v[CRECW - 2], v[CRECW - 1]);
   }
 }

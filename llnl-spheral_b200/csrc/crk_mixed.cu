@@ -45,7 +45,7 @@ struct CMRec {
 
 __device__ __forceinline__ CMRec loadCMRec(const double* rec, int64_t cap, int64_t k) {
   double a[CMRECW];
-  ldPlanes<CMRECW/4>(rec, cap, k, a);
+  ldPlanes<CMRECW/4, false, false>(rec, cap, k, a);
   // 28 floats after the six doubles
   float f[28];
 #pragma unroll
@@ -79,14 +79,14 @@ __global__ void __launch_bounds__(256) pack_crk_mixed_kernel(const Member* mem, 
   auto kf = [&](int field) { return (float)K[(int64_t)field*n + r]; };
   double* q = MB.mrec;
   const int64_t cap = MB.candcap;
-  stPlane(q + planeAt(cap, k, 0), x.x, x.y, x.z, S[S_VX*n + r]);
-  stPlane(q + planeAt(cap, k, 1), S[S_VY*n + r], S[S_VZ*n + r], packF((float)S[S_M*n + r], (float)S[S_RHO*n + r]),
+  stPlane(q + planeAt<false>(cap, k, 0), x.x, x.y, x.z, S[S_VX*n + r]);
+  stPlane(q + planeAt<false>(cap, k, 1), S[S_VY*n + r], S[S_VZ*n + r], packF((float)S[S_M*n + r], (float)S[S_RHO*n + r]),
           packF((float)S[S_CS*n + r], (float)S[S_P*n + r]));
-  stPlane(q + planeAt(cap, k, 2), packF((float)sdet(H), (float)S[S_VOL*n + r]), packF((float)H.xx, (float)H.xy),
+  stPlane(q + planeAt<false>(cap, k, 2), packF((float)sdet(H), (float)S[S_VOL*n + r]), packF((float)H.xx, (float)H.xy),
           packF((float)H.xz, (float)H.yy), packF((float)H.yz, (float)H.zz));
-  stPlane(q + planeAt(cap, k, 3), packF(kf(K_A), kf(K_B)), packF(kf(K_B + 1), kf(K_B + 2)),
+  stPlane(q + planeAt<false>(cap, k, 3), packF(kf(K_A), kf(K_B)), packF(kf(K_B + 1), kf(K_B + 2)),
           packF(kf(K_GRADA), kf(K_GRADA + 1)), packF(kf(K_GRADA + 2), kf(K_GRADB)));
-  stPlane(q + planeAt(cap, k, 4), packF(kf(K_GRADB + 1), kf(K_GRADB + 2)), packF(kf(K_GRADB + 3), kf(K_GRADB + 4)),
+  stPlane(q + planeAt<false>(cap, k, 4), packF(kf(K_GRADB + 1), kf(K_GRADB + 2)), packF(kf(K_GRADB + 3), kf(K_GRADB + 4)),
           packF(kf(K_GRADB + 5), kf(K_GRADB + 6)), packF(kf(K_GRADB + 7), kf(K_GRADB + 8)));
 }
 

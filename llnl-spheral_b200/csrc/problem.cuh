@@ -142,9 +142,7 @@ enum RecField {
 // one.  A pair loop's lanes visit nodes that are mostly consecutive, so one
 // 32-byte load of a warp covers 8 to 12 cache lines; with whole records side
 // by side every lane's load is a line of its own (32 lines for each of the
-// ten 16-byte loads), and those line accesses bound the pair kernels.  A
-// 32-byte piece is a whole sector, so a node order without locality costs no
-// more sectors than whole records do.  Measured (B200, Kelvin-Helmholtz 128^3,
+// ten 16-byte loads), and those line accesses bound the pair kernels.  Measured (B200, Kelvin-Helmholtz 128^3,
 // whole records -> planes): FP64 pair kernel 807 -> 688 us, summed density
 // 268 -> 184, mid-point update 229 -> 183; mixed 511 -> 488, 203 -> 137,
 // 195 -> 168; CRKSPH 1M volumes and density 202 -> 119.
@@ -164,17 +162,34 @@ __device__ __forceinline__ D4 ldPlaneW(const double* p) {      // data other thr
 __device__ __forceinline__ void stPlane(double* p, double a, double b, double c, double d) {
   asm volatile("st.global.v4.f64 [%0], {%1,%2,%3,%4};" : : "l"(p), "d"(a), "d"(b), "d"(c), "d"(d) : "memory");
 }
-// plane q of node k
-__host__ __device__ __forceinline__ int64_t planeAt(int64_t cap, int64_t k, int q) { return (q*cap + k)*4; }
+// plane q of node k.  Above a capacity of kPairedPlanes nodes (a problem of 1.08M
+// nodes) the SPH records keep planes 1 and 2, and 3 and 4, of a node side by
+// side: the records are then well beyond the L2 cache, and where the node order
+// has no locality every 32-byte piece fetched from HBM brings its 64-byte
+// neighborhood with it.  Measured (B200, Kelvin-Helmholtz in a random node order,
+// one step; whole records / planes / paired planes): 128^3 FP64 4.54 / 4.92 /
+// 4.46 ms, mixed 4.06 / 4.38 / 4.12; 112^3 2.88 / 2.97 / 2.76, 2.50 / 2.58 /
+// 2.48; 96^3 1.78 / 1.74 / 1.65, 1.56 / 1.54 / 1.50.  In lattice order a pair
+// covers twice the lines of a plane (128^3 FP64 pair kernel 687 -> 724 us, mixed
+// 510 -> 522, Sod 1,817 -> 1,860), so problems whose single planes are no slower
+// than whole records in either order keep them.  CRKSPH's longer records (PAIRED
+// false) gain from planes in either order (96^3 random 3.21 / 2.86 / 2.89 ms; 1M
+// in order, pair kernel 520 against 548 us).
+constexpr int64_t kPairedPlanes = 1900000;
+template<bool PAIRED = true>
+__host__ __device__ __forceinline__ int64_t planeAt(int64_t cap, int64_t k, int q) {
+  if (PAIRED && q > 0 && cap > kPairedPlanes) return (((q - 1) | 1)*cap + 2*k)*4 + (q & 1 ? 0 : 4);
+  return (q*cap + k)*4;
+}
 // the half plane after Q planes
 __host__ __device__ __forceinline__ int64_t halfPlaneAt(int64_t cap, int64_t k, int Q) { return Q*cap*4 + k*2; }
 
 // a record's first 4*Q doubles (and the half plane after them)
-template<int Q, bool HALF = false>
+template<int Q, bool HALF = false, bool PAIRED = true>
 __device__ __forceinline__ void ldPlanes(const double* rec, int64_t cap, int64_t k, double* v) {
 #pragma unroll
   for (int q = 0; q < Q; ++q) {
-    const D4 p = ldPlane(rec + planeAt(cap, k, q));
+    const D4 p = ldPlane(rec + planeAt<PAIRED>(cap, k, q));
     v[4*q] = p.a; v[4*q + 1] = p.b; v[4*q + 2] = p.c; v[4*q + 3] = p.d;
   }
   if (HALF) {

@@ -104,3 +104,26 @@ def test_long_and_short_rows_in_one_batch(gpu_lib, pkg, precision):
     for a, b in zip(alone, together):
         for k in ("position", "velocity", "mass density", "specific thermal energy", "H"):
             assert np.array_equal(a.field(k), b.field(k)), k
+
+
+@pytest.mark.parametrize("precision", ["PRECISION_FP64", "PRECISION_MIXED"])
+def test_paired_planes_of_large_problems(gpu_lib, pkg, precision):
+    """The record layout of problems above 1.08M nodes: one step of the nodes of a
+    cube far from the periodic planes equals the step of that cube alone, which
+    keeps the small layout, bit for bit where the cube's surface (four kernel
+    reaches) has no influence: neighbors, their order and every term are the same."""
+    gen, abi = pkg.generators, pkg.abi
+    cfg = gen.kh_config(abi, precision=getattr(abi, precision), dtMin=1.0e-4, dtMax=1.0e-4)
+    whole = gen.kelvin_helmholtz(nx=104, ny=104, nz=104)
+    assert 1.75 * whole.n > 1.9e6
+    sel = np.flatnonzero((np.abs(whole.pos - 0.5) < 0.17).all(axis=1))
+    cube = gen.NodeSet(whole.pos[sel], whole.vel[sel], whole.mass[sel], whole.rho[sel], whole.eps[sel],
+                       whole.H[sel], whole.dx)
+    # a reach is at most 2.7 spacings of 1/104
+    inner = np.flatnonzero((np.abs(cube.pos - 0.5) < 0.17 - 4 * 2.7 / 104).all(axis=1))
+    assert inner.size > 1000
+    large, small = pkg.SPHHydro(cfg, whole), pkg.SPHHydro(cfg, cube)
+    large.step(1)
+    small.step(1)
+    for k in ("position", "velocity", "mass density", "specific thermal energy", "H"):
+        assert np.array_equal(large.field(k)[sel][inner], small.field(k)[inner]), k
