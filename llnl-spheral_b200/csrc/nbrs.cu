@@ -36,10 +36,10 @@
 //                                            a reach, for large sets
 #include <cstdio>
 #include <cstring>
-#include <cfloat>
 #include <climits>
 
 #include <cooperative_groups.h>
+#include <math_constants.h>
 
 #include "problem.cuh"
 
@@ -626,6 +626,7 @@ __device__ void setGrid(const Member& M) {
   }
   const int64_t maxCells = M.cellcap < ((int64_t)1 << 26) ? M.cellcap : ((int64_t)1 << 26);
   int64_t dim[3] = {1, 1, 1}, ncells = 1;
+  bool covered = true;
   {
     // cells at the natural size, for the next build's capacity
     double want = 1.0;
@@ -643,6 +644,7 @@ __device__ void setGrid(const Member& M) {
     if (ncells <= maxCells) break;
     cell *= 1.26;
   }
+  for (int a = 0; a < 3; ++a) covered = covered && dim[a] < (1 << 20);
   double* s = M.scal + SC_GRID;
   s[0] = lo[0]; s[1] = lo[1]; s[2] = lo[2];
   s[3] = cell;
@@ -651,10 +653,12 @@ __device__ void setGrid(const Member& M) {
   // and the cells' edge over the kernel reach where the capacity enlarged them:
   // the FP32 pre-test's relative error is below 2e-6 times their product (the
   // offsets are rounded at the size of a cell).  The band is ten times that,
-  // 1e-3 at most, and the pre-test is off beyond a product of 100.
+  // 1e-3 at most, and the pre-test is off beyond a product of 100, and where
+  // the grid ends before the box does (the offsets in its last cells have any
+  // size).
   const double natural = M.prm.kernelExtent*hmaxAll*1.001/sub;
   const double spread = hmaxAll*M.scal[SC_LMAXALL]*fmax(1.0, cell/natural);
-  s[7] = (M.grid.filterTol > 0.0f && spread > 0.0 && spread <= 100.0)
+  s[7] = (M.grid.filterTol > 0.0f && covered && spread > 0.0 && spread <= 100.0)
              ? fmin((double)M.grid.filterTol, kFilterTolPerSpread*fmax(spread, 1.0)) : 0.0;
   // the largest kernel reach in cells (<= sub), for the walks' pruning
   M.scal[SC_REACH] = M.prm.kernelExtent*hmaxAll/cell;
@@ -912,6 +916,10 @@ __global__ void __launch_bounds__(kGhostThreads) cell_index_kernel(const Member*
 //                               pre-test band): beyond that r^2 the node's own
 //                               eta^2 lies above the band
 //   lmax    [candcap] float:    FP32 max eig(H)
+// Both are in units of the cell edge, as every length of the FP32 tests is: r^2
+// and its bounds are then of order one, and no FP32 square overflows or
+// vanishes whatever the problem's unit of length (a centimetre with kernels of
+// 1e20 cm, say).
 // and sortedIdx[slot], the node of each slot.  The walks read only `pre` for
 // most candidates; `lmax` when the i-side test alone does not decide, and
 // the FP64 position and H of the node (state, ghost positions) for the
@@ -936,8 +944,9 @@ __device__ __forceinline__ float symEta2F(const float* h, float x, float y, floa
   return __fmaf_rn(ex, ex, __fmaf_rn(ey, ey, ez*ez));
 }
 
-// The walking node: FP32 H and cell offsets for the pre-test, its cell, its
-// sorted slot and node index (the exact test re-reads its FP64 state).
+// The walking node: FP32 H and cell offsets for the pre-test (in cell edges),
+// its cell, its sorted slot and node index (the exact test re-reads its FP64
+// state).
 struct Walker {
   float hf[6];
   float lam2;          // isotropic H = lam I: lam^2 (then eta_i^2 = lam^2 |r|^2)
@@ -957,8 +966,8 @@ __device__ __forceinline__ Walker makeWalker(const Member& M, const NbrArrays& a
   if (w.idx >= M.n) return w;
   const V3 r = nodePos(M, w.idx);
   const Sym H = nodeH(M, w.idx);
-  w.hf[0] = (float)H.xx; w.hf[1] = (float)H.xy; w.hf[2] = (float)H.xz;
-  w.hf[3] = (float)H.yy; w.hf[4] = (float)H.yz; w.hf[5] = (float)H.zz;
+  w.hf[0] = (float)(H.xx*g.cell); w.hf[1] = (float)(H.xy*g.cell); w.hf[2] = (float)(H.xz*g.cell);
+  w.hf[3] = (float)(H.yy*g.cell); w.hf[4] = (float)(H.yz*g.cell); w.hf[5] = (float)(H.zz*g.cell);
   w.iso = H.xy == 0.0 && H.xz == 0.0 && H.yz == 0.0 && H.xx == H.yy && H.xx == H.zz;
   w.lam2 = w.hf[0]*w.hf[0];
   const float4 p = __ldg(a.pre + s);
@@ -968,6 +977,15 @@ __device__ __forceinline__ Walker makeWalker(const Member& M, const NbrArrays& a
   w.cy = cellCoord(r.y, g.lo[1], g.cell, g.dim[1]);
   w.cz = cellCoord(r.z, g.lo[2], g.cell, g.dim[2]);
   return w;
+}
+
+// Square of the distance, in cells, beyond which a walk leaves candidates out:
+// the largest kernel reach, a relative margin, and `slack` for the rounding of
+// the FP32 offsets (which counts where the cells' capacity made them many times
+// a reach).
+__device__ __forceinline__ float reachBound2(float reach, float slack) {
+  const float r = reach*1.00005f + slack;
+  return r*r;
 }
 
 // Distance, in cells, from a walker at fraction f of its cell to the cell d
@@ -1010,11 +1028,11 @@ __device__ __forceinline__ Row<SUB> loadRow(const Member& M, const Grid& g, cons
 }
 
 template<int SUB>
-__device__ __forceinline__ float rowDxc(const Row<SUB>& r, const Walker& w, int32_t k, float cellf) {
+__device__ __forceinline__ float rowDxc(const Row<SUB>& r, const Walker& w, int32_t k) {
   int xc = r.x0 - w.cx;
 #pragma unroll
   for (int c = 0; c < 2*SUB; ++c) xc += (k >= r.e[c]);
-  return (float)xc*cellf;
+  return (float)xc;
 }
 
 // The exact FP64 predicate for nodes i and j (the walks reach it for the
@@ -1032,7 +1050,7 @@ __device__ __forceinline__ bool exactTest(const Member& M, int32_t i, int32_t j,
 
 // ConnectivityMap predicate |H_i r_ij|^2 <= kappa^2 || |H_j r_ij|^2 <= kappa^2
 // (src/Neighbor/ConnectivityMapInline.hh:169-186) for candidate slot k, whose
-// cell corner lies at (dxc, dyc, dzc) from the walker's (FP32).
+// cell corner lies at (dxc, dyc, dzc) from the walker's, in cells.
 // With tol > 0 a FP32 pre-test decides every pair whose eta^2 lies clearly
 // outside the band kappa^2 (1 -+ tol): eta_i^2 from the FP32 H_i, eta_j^2
 // bounded by min/max eig(H_j)^2 |r_ij|^2, r_ij from the cell offsets.  The
@@ -1074,6 +1092,7 @@ __global__ void __launch_bounds__(kGhostThreads) cell_scatter_kernel(const Membe
   // the pre-test's upper band edge, as the walks form it
   const float k2f = (float)(M.prm.kernelExtent*M.prm.kernelExtent);
   const double k2hi = (double)(k2f*(1.0f + g.filterTol));
+  const double inv = 1.0/g.cell;
   FOR_ITEMS(k, allNodes(M)) {
     const int c = M.cidx[k];
     const int64_t slot = M.cellStart[c] + atomicAdd(M.cellFill + c, 1);
@@ -1083,10 +1102,10 @@ __global__ void __launch_bounds__(kGhostThreads) cell_scatter_kernel(const Membe
     const int cy = cellCoord(r.y, g.lo[1], g.cell, g.dim[1]);
     const int cz = cellCoord(r.z, g.lo[2], g.cell, g.dim[2]);
     const int64_t root = k < M.n ? k : M.groot[k - M.n];
-    const double hm = M.hmaxi[root];
-    pre[slot] = make_float4((float)(r.x - (g.lo[0] + cx*g.cell)), (float)(r.y - (g.lo[1] + cy*g.cell)),
-                            (float)(r.z - (g.lo[2] + cz*g.cell)), (float)(k2hi*hm*hm));
-    lmax[slot] = (float)M.hmaxi[M.n + root];
+    const double hm = M.hmaxi[root]*inv;
+    pre[slot] = make_float4((float)((r.x - (g.lo[0] + cx*g.cell))*inv), (float)((r.y - (g.lo[1] + cy*g.cell))*inv),
+                            (float)((r.z - (g.lo[2] + cz*g.cell))*inv), (float)(k2hi*hm*hm));
+    lmax[slot] = (float)(M.hmaxi[M.n + root]*g.cell);
   }
 }
 
@@ -1128,11 +1147,10 @@ __global__ void __launch_bounds__(256, SUB == 1 ? NBR_THREAD_MIN_BLOCKS : 1) nbr
     const float k2f = (float)k2;
     const bool pretest = g.filterTol > 0.0f;
     const float k2lo = k2f*(1.0f - g.filterTol), k2hi = k2f*(1.0f + g.filterTol);
-    const float cellf = (float)g.cell;
     const int32_t i = me.idx;
     // window of +-SUB cells; with SUB > 1 the rows and cells farther than the
     // largest kernel reach (in cells, with a margin) are skipped
-    const float rc2 = g.reach*g.reach*1.0001f;
+    const float rc2 = reachBound2(g.reach, 1.0e-6f);
     auto accept = [&](int32_t k) {
       if (collect) {
         const int32_t j = __ldg(M.sortedIdx + k);
@@ -1151,22 +1169,22 @@ __global__ void __launch_bounds__(256, SUB == 1 ? NBR_THREAD_MIN_BLOCKS : 1) nbr
       ++count;
     };
     {
-      const float fx = me.ox/cellf, fy = me.oy/cellf, fz = me.oz/cellf;
+      const float fx = me.ox, fy = me.oy, fz = me.oz;
       for (int dz = -SUB; dz <= SUB; ++dz) {
         const int z = me.cz + dz;
         if (z < 0 || z >= g.dim[2]) continue;
         const float gz = axisGap(dz, fz);
-        const float dzc = (float)dz*cellf;
+        const float dzc = (float)dz;
         for (int dy = -SUB; dy <= SUB; ++dy) {
           const int y = me.cy + dy;
           if (y < 0 || y >= g.dim[1]) continue;
           const float gy = axisGap(dy, fy);
           const float gyz = gy*gy + gz*gz;
           if (SUB > 1 && gyz > rc2) continue;
-          const float dyc = (float)dy*cellf;
+          const float dyc = (float)dy;
           const Row<SUB> row = loadRow<SUB>(M, g, me, y, z, fx, gyz, rc2);
           for (int32_t k = row.start; k < row.end; ++k) {
-            if (k != s && candTest(M, a, me, k, rowDxc<SUB>(row, me, k, cellf), dyc, dzc, k2, k2lo, k2hi, pretest))
+            if (k != s && candTest(M, a, me, k, rowDxc<SUB>(row, me, k), dyc, dzc, k2, k2lo, k2hi, pretest))
               accept(k);
           }
         }
@@ -1295,9 +1313,8 @@ __device__ __noinline__ void walkWarp(const Member& M, const Grid& g, int64_t s,
   const float k2f = (float)k2;
   const bool pretest = g.filterTol > 0.0f;
   const float k2lo = k2f*(1.0f - g.filterTol), k2hi = k2f*(1.0f + g.filterTol);
-  const float cellf = (float)g.cell;
-  const float rc2 = g.reach*g.reach*1.0001f;
-  const float fx = me.ox/cellf, fy = me.oy/cellf, fz = me.oz/cellf;
+  const float rc2 = reachBound2(g.reach, 1.0e-6f);
+  const float fx = me.ox, fy = me.oy, fz = me.oz;
   // The window's rows, one per lane (rows outside the grid or, with SUB > 1,
   // beyond the kernel reach are empty), their candidates numbered in one
   // sequence by a warp scan: the lanes then take 32 consecutive candidates at
@@ -1344,8 +1361,8 @@ __device__ __noinline__ void walkWarp(const Member& M, const Grid& g, int64_t s,
         int xc = row[2] - me.cx;
 #pragma unroll
         for (int c = 0; c < 2*SUB; ++c) xc += (k >= row[3 + c]);
-        const float dyc = (float)(r % (2*SUB + 1) - SUB)*cellf, dzc = (float)(r/(2*SUB + 1) - SUB)*cellf;
-        pass = candTest(M, a, me, k, (float)xc*cellf, dyc, dzc, k2, k2lo, k2hi, pretest);
+        const float dyc = (float)(r % (2*SUB + 1) - SUB), dzc = (float)(r/(2*SUB + 1) - SUB);
+        pass = candTest(M, a, me, k, (float)xc, dyc, dzc, k2, k2lo, k2hi, pretest);
       }
     }
     const unsigned ballot = __ballot_sync(0xffffffffu, pass);
@@ -1541,7 +1558,7 @@ __device__ __forceinline__ void mergeRuns(const int32_t* key, const uint16_t* sr
   }
 }
 
-// The walker's side of the test.
+// The walker's side of the test (lengths in cells).
 struct CellWalker {
   float x, y, z;
   float T;             // r^2 above both nodes' T: not neighbors
@@ -1550,11 +1567,12 @@ struct CellWalker {
 };
 
 // A pair between the bounds: the FP32 form of H_i, then the exact test.
-__device__ __noinline__ bool cellUndecided(const Member& M, int32_t i, int32_t j, float fx, float fy, float fz,
-                                           float cT, double k2, float k2lo, float k2hi, bool pretest) {
+__device__ __noinline__ bool cellUndecided(const Member& M, int32_t i, int32_t j, double cell, float fx, float fy,
+                                           float fz, float cT, double k2, float k2lo, float k2hi, bool pretest) {
   if (pretest) {
     const Sym H = nodeH(M, i);
-    const float hf[6] = {(float)H.xx, (float)H.xy, (float)H.xz, (float)H.yy, (float)H.yz, (float)H.zz};
+    const float hf[6] = {(float)(H.xx*cell), (float)(H.xy*cell), (float)(H.xz*cell),
+                         (float)(H.yy*cell), (float)(H.yz*cell), (float)(H.zz*cell)};
     const float r2 = __fmaf_rn(fx, fx, __fmaf_rn(fy, fy, fz*fz));
     const float e2i = symEta2F(hf, fx, fy, fz);
     if (e2i <= k2lo) return true;
@@ -1591,13 +1609,12 @@ __global__ void __launch_bounds__(kCellThreads, 4) nbr_cell_kernel(const Member*
   const float k2f = (float)k2;
   const bool pretest = filterTol > 0.0f;
   const float k2lo = k2f*(1.0f - filterTol), k2hi = k2f*(1.0f + filterTol);
-  const float cellf = (float)M.scal[SC_GRID + 3];
+  const double cell = M.scal[SC_GRID + 3];
   const int dim0 = (int)scalI(M.scal, SC_GRID + 4), dim1 = (int)scalI(M.scal, SC_GRID + 5),
             dim2 = (int)scalI(M.scal, SC_GRID + 6);
-  // no candidate farther than the largest kernel reach can pass (the margin
-  // covers the FP32 offsets)
-  const float reach = (float)M.scal[SC_REACH]*cellf;
-  const float reach2 = reach*reach*1.0001f;
+  // no candidate farther than the largest kernel reach can pass (the slack
+  // covers the FP32 offsets and a walker at the tolerance of `outside`)
+  const float reach2 = reachBound2((float)M.scal[SC_REACH], 1.2e-5f);
   int most = 0;
   unsigned above = 0;
   for (int c = (int)mb.block; c < ncells; c += mb.blocks) {
@@ -1609,12 +1626,12 @@ __global__ void __launch_bounds__(kCellThreads, 4) nbr_cell_kernel(const Member*
       any = true;
       // a node clamped into the grid's outermost cells may lie outside its cell
       const float4 p = a.pre[s];
-      const float lo = -1.0e-5f*cellf, hi = 1.00001f*cellf;
+      const float lo = -1.0e-5f, hi = 1.00001f;
       outside = outside || fminf(p.x, fminf(p.y, p.z)) < lo || fmaxf(p.x, fmaxf(p.y, p.z)) > hi;
     }
     if (!__syncthreads_or(any)) continue;
     if (tid == 0) crowded = 0;
-    const float rc2 = __syncthreads_or(outside) ? FLT_MAX : reach2;
+    const float rc2 = __syncthreads_or(outside) ? CUDART_INF_F : reach2;
     const int cyz = c/dim0, cx = c - cyz*dim0, cz = cyz/dim1, cy = cyz - cz*dim1;
     if (wib == 0) {
       // the 27 cells, x fastest: first slot and nodes, and an upper bound of each run's position
@@ -1656,7 +1673,7 @@ __global__ void __launch_bounds__(kCellThreads, 4) nbr_cell_kernel(const Member*
     for (int q = wib; q < 27; q += kCellWarps) {
       const int len = cellLen[q], at = cellAt[q];
       const int32_t first = cellS0[q];
-      const float ox = (float)(q % 3 - 1)*cellf, oy = (float)((q/3) % 3 - 1)*cellf, oz = (float)(q/9 - 1)*cellf;
+      const float ox = (float)(q % 3 - 1), oy = (float)((q/3) % 3 - 1), oz = (float)(q/9 - 1);
       int kept = 0;
       for (int base = 0; base < len; base += 32) {
         const int t = base + lane;
@@ -1665,8 +1682,8 @@ __global__ void __launch_bounds__(kCellThreads, 4) nbr_cell_kernel(const Member*
         if (t < len) {
           p = a.pre[first + t];
           p.x += ox; p.y += oy; p.z += oz;
-          const float gx = fmaxf(fmaxf(-p.x, p.x - cellf), 0.0f), gy = fmaxf(fmaxf(-p.y, p.y - cellf), 0.0f),
-                      gz = fmaxf(fmaxf(-p.z, p.z - cellf), 0.0f);
+          const float gx = fmaxf(fmaxf(-p.x, p.x - 1.0f), 0.0f), gy = fmaxf(fmaxf(-p.y, p.y - 1.0f), 0.0f),
+                      gz = fmaxf(fmaxf(-p.z, p.z - 1.0f), 0.0f);
           keep = q == 13 || gx*gx + gy*gy + gz*gz <= rc2;   // (the own nodes' places follow their slots)
         }
         const unsigned bal = __ballot_sync(0xffffffffu, keep);
@@ -1722,11 +1739,14 @@ __global__ void __launch_bounds__(kCellThreads, 4) nbr_cell_kernel(const Member*
         some = some || on;
         const float4 p = a.pre[on ? s + q : s0];
         const float lm = a.lmax[on ? s + q : s0];
-        // an empty place tests like any other and is not stored
-        w[q] = CellWalker{p.x, p.y, p.z, pretest ? p.w : FLT_MAX, pretest ? __fdividef(k2lo, lm*lm) : -1.0f, on ? i : -1};
+        // an empty place tests like any other and is not stored; without the
+        // pre-test every candidate is left to the exact test
+        w[q] = CellWalker{p.x, p.y, p.z, pretest ? p.w : CUDART_INF_F, pretest ? __fdividef(k2lo, lm*lm) : -1.0f, on ? i : -1};
       }
       if (!some) continue;
       const int batches = (count + 31) >> 5;              // at most 32
+      // the last batch's places that hold a candidate
+      const unsigned filled = 0xffffffffu >> (32*batches - count);
       // the batch's ballots, kept by the lane of the batch's number
       unsigned sure[kWalkers], open[kWalkers];
 #pragma unroll
@@ -1735,11 +1755,10 @@ __global__ void __launch_bounds__(kCellThreads, 4) nbr_cell_kernel(const Member*
         const int t = 32*b + lane;
         const int at = src[t < count ? t : count - 1];
         const float4 cnd = sh.pre[at];
-        const float cA = t < count ? sh.acc[at] : -FLT_MAX;
-        const float x = t < count ? cnd.x : FLT_MAX;        // past the end: infinitely far
+        const float cA = sh.acc[at];
 #pragma unroll
         for (int q = 0; q < kWalkers; ++q) {
-          const float fx = w[q].x - x, fy = w[q].y - cnd.y, fz = w[q].z - cnd.z;
+          const float fx = w[q].x - cnd.x, fy = w[q].y - cnd.y, fz = w[q].z - cnd.z;
           const float r2 = __fmaf_rn(fx, fx, __fmaf_rn(fy, fy, fz*fz));
           const unsigned in = __ballot_sync(0xffffffffu, r2 <= fmaxf(w[q].A, cA));
           const unsigned near = __ballot_sync(0xffffffffu, r2 <= fmaxf(w[q].T, cnd.w));
@@ -1750,6 +1769,7 @@ __global__ void __launch_bounds__(kCellThreads, 4) nbr_cell_kernel(const Member*
       for (int q = 0; q < kWalkers; ++q) {
         const int32_t i = w[q].idx;
         if (i < 0) continue;
+        if (lane == batches - 1) { sure[q] &= filled; open[q] &= filled; }
         // the walker itself is no neighbor
         const int self = sh.own[s + q - s0];
         if (self >> 5 == lane) { sure[q] &= ~(1u << (self & 31)); open[q] &= ~(1u << (self & 31)); }
@@ -1758,7 +1778,7 @@ __global__ void __launch_bounds__(kCellThreads, 4) nbr_cell_kernel(const Member*
           const int bit = __ffs(open[q]) - 1;
           open[q] &= open[q] - 1;
           const int t = 32*lane + bit, at = src[t];
-          if (cellUndecided(M, i, key[t], w[q].x - sh.pre[at].x, w[q].y - sh.pre[at].y, w[q].z - sh.pre[at].z,
+          if (cellUndecided(M, i, key[t], cell, w[q].x - sh.pre[at].x, w[q].y - sh.pre[at].y, w[q].z - sh.pre[at].z,
                             sh.pre[at].w, k2, k2lo, k2hi, pretest))
             sure[q] |= 1u << bit;
         }

@@ -43,3 +43,65 @@ def test_clumped_cells(gpu_lib, pkg, oracle_mod, clump, passes, periodic, vary):
         go, gn, gr = g.connectivity()
         assert np.array_equal(go, oo) and np.array_equal(gn, on) and np.array_equal(gr, orr)
         assert g.num_pairs() == o.num_pairs()
+
+
+def _same_connectivity(g, o):
+    oo, on, orr = o.connectivity()
+    go, gn, gr = g.connectivity()
+    assert np.array_equal(go, oo) and np.array_equal(gn, on) and np.array_equal(gr, orr)
+    assert g.num_pairs() == o.num_pairs()
+
+
+# 1e-24 and 1e21: squares of lengths vanish or overflow in FP32; 1e19: some of them do
+@pytest.mark.parametrize("unit", [1.0e-24, 1.0, 1.0e19, 1.0e21])
+@pytest.mark.parametrize("form", ["pre-test", "exact", "spread"])
+@pytest.mark.parametrize("walk,cells", [(2, 1), (2, 2), (1, 1), (1, 2)])
+def test_units_of_length(gpu_lib, pkg, oracle_mod, unit, form, walk, cells):
+    """The FP32 tests of the walks decide nothing wrongly in any unit of length,
+    with the pre-test, without it, and with smoothing scales more than 100 apart
+    (where it is off)."""
+    gen, abi = pkg.generators, pkg.abi
+    ns, _ = _clump(pkg, 50, 3, (1, 0, 1), True)
+    if form == "spread":
+        ns.H[::3, [0, 3, 5]] *= 150.0
+    big = gen.NodeSet(ns.pos * unit, ns.vel, ns.mass, ns.rho, ns.eps, ns.H / unit, ns.dx * unit)
+    cfg = gen.kh_config(abi, kernel=abi.KERNEL_BSPLINE, periodic=(1, 0, 1), max_neighbors=2048, xmax=(unit,) * 3)
+    g, o = pkg.SPHHydro(cfg, big), oracle_mod.OracleProblem(cfg, big)
+    g.set_schedule("neighbor walk", walk)
+    g.set_schedule("neighbor cells", cells)
+    g.set_schedule("neighbor filter", 0 if form == "exact" else 1)
+    g.build_neighbors()
+    o.build_neighbors()
+    assert o.num_pairs() > ns.n
+    _same_connectivity(g, o)
+
+
+def test_pairs_across_large_cells(gpu_lib, pkg):
+    """A few nodes in a box of many reaches: the first build's cells are thousands
+    of reaches wide, and pairs just within reach lie across a cell's face."""
+    gen, abi = pkg.generators, pkg.abi
+    pairs, h = 400, 1.0055e-6
+    n = 2 * pairs + 2
+    # the first build's cell edge (plan_capacities, setGrid)
+    ghosts = n // 2 + 4096
+    cells = (n + ghosts + ghosts // 2 + 1024) // 2 + 65
+    cell = 2.0 * h * 1.001
+    while int(1.0 / cell + 1.0) ** 3 > cells:
+        cell *= 1.26
+    rng = np.random.default_rng(5)
+    first = rng.uniform(0.05, 0.95, (pairs, 3))
+    first[:, 0] = cell * rng.integers(1, int(1.0 / cell), pairs) - rng.uniform(0.0, 3.0e-3, pairs) * 2.0 * h
+    second = first + np.array([0.99995 * 2.0 * h, 0.0, 0.0])
+    pos = np.concatenate([[[0.0, 0.0, 0.0], [1.0, 1.0, 1.0]], first, second])
+    H = np.zeros((n, 6))
+    H[:, [0, 3, 5]] = 1.0 / h
+    ns = gen.NodeSet(pos, np.zeros((n, 3)), np.full(n, 1.0 / n), np.ones(n), np.ones(n), H, cell)
+    g = pkg.SPHHydro(gen.kh_config(abi, kernel=abi.KERNEL_BSPLINE, periodic=(0, 0, 0)), ns)
+    g.set_schedule("neighbor walk", 2)
+    g.build_neighbors()
+    off, nbr, _ = g.connectivity()
+    # every node of a pair has the other one (none of the random pairs meet), the corners nobody
+    near = np.sqrt(((pos[:, None] - pos[None]) ** 2).sum(2)) <= 2.0 * h
+    np.fill_diagonal(near, False)
+    assert near.sum() == 2 * pairs and not near[:2].any()
+    assert np.array_equal(np.diff(off), near.sum(1)) and np.array_equal(nbr, np.nonzero(near)[1])
