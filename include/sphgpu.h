@@ -319,9 +319,11 @@ int sphgpu_kernel_launches(sphgpu_problem* p, int64_t* launches);
  * are walked once; used when the problem evolves energy compatibly (it has
  * that buffer) and the lists fit in it, otherwise 2 = a counting walk, then
  * a filling walk.  Both give the same ConnectivityMap.  stage "neighbor
- * cells": cells per kernel reach of the walk's grid, 0 = automatic (1),
- * 1 = cells of one reach (27-cell window), 2 = cells of half a reach
- * (125-cell window, rows and cells beyond the reach skipped).  Same
+ * cells": cells per kernel reach of the walk's grid, 0 = automatic (1, or 2
+ * once a walk of large candidate sets has found a quarter of its nodes in cells
+ * too crowded to share their candidates), 1 = cells of one reach (27-cell
+ * window), 2 = cells of half a reach (125-cell window, rows and cells beyond
+ * the reach skipped).  Same
  * ConnectivityMap either way.  stage "ghost passes": the six periodic
  * boundary passes of the ghost build, 0 = automatic (while every member has
  * at most 32,768 nodes: one launch with a thread-block cluster per member;

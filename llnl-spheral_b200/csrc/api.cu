@@ -498,7 +498,7 @@ uint64_t graph_key(const Batch& b) {
     // sizes and plans that set launch shapes, kernel variants and shared memory
     const int64_t sizes[] = {p->n, p->gcap, p->ecap, p->candcap, p->cellcap, p->reccap, p->creccap,
                              p->mreccap, p->blockSumsCap, p->redcap, p->maxNbr, p->fillCap, p->fillSchedule,
-                             p->grid.sub, p->grid.stashCap, p->grid.stashStride};
+                             p->grid.sub, p->grid.stashCap, p->grid.stashStride, p->grid.crowdList, p->crowd > 0, p->denseSet > 0.0};
     for (int64_t v : sizes) mix((uint64_t)v);
   }
   return h;
@@ -730,10 +730,10 @@ int run_graph_steps(Batch& b, int64_t count, int64_t* done) {
   for (int64_t s = 0; s < count; ++s) SPH_CHECK(cudaGraphLaunch(b.graphExec, b.stream));
   b.memDirty = true;     // the next eager call uploads to the rotating slots again
   const int s1[8] = {SC_STEPS, -1, SC_TIME, SC_DT, SC_G, SC_TOTAL, SC_MAXCOUNT, SC_PAIRS};
-  const int s2[3] = {SC_NCELLS, SC_CELLSWANTED, SC_PAIRSUM};
+  const int s2[4] = {SC_NCELLS, SC_CELLSWANTED, SC_PAIRSUM, SC_CROWDED};
   std::vector<double> r1, r2;
   SPH_TRY(batch_gather(b, s1, 8, r1));
-  SPH_TRY(batch_gather(b, s2, 3, r2));
+  SPH_TRY(batch_gather(b, s2, 4, r2));
   int64_t ran = count;
   for (int m = 0; m < nm; ++m) ran = asI64(r1[8*m]) < ran ? asI64(r1[8*m]) : ran;
   // kernels run: every completed replay; the open kernel of each one that
@@ -759,9 +759,10 @@ int run_graph_steps(Batch& b, int64_t count, int64_t* done) {
     p.E = asI64(a[5]);
     p.maxCount = asI32(a[6]);
     p.pairs = asI64(a[7]);
-    p.ncells = asI64(r2[3*m]);
-    p.cellsWanted = asI64(r2[3*m + 1]);
-    p.pairsEvaluated += asI64(r2[3*m + 2]);
+    p.ncells = asI64(r2[4*m]);
+    p.cellsWanted = asI64(r2[4*m + 1]);
+    p.pairsEvaluated += asI64(r2[4*m + 2]);
+    note_crowd(p, asI64(r2[4*m + 3]));
     if (herr & (DERR_GHOST_CAPACITY | DERR_ENTRY_CAPACITY | DERR_LIST_CAPACITY | DERR_NBR_CAPACITY)) overflow = true;
     else if (herr) return batch_check_errors(b, "step_rk2");
   }

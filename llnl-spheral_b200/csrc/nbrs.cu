@@ -32,8 +32,10 @@
 //   nbr_cell<COUNT|FILL>                     block per cell, for large
 //                                            candidate sets: the window
 //                                            staged and ordered once per cell
+//   nbr_crowded<COUNT|FILL>                  ... warp per node of the cells too
+//                                            crowded for it
 //   nbr_walk<COUNT|FILL>                     warp per node over cells of half
-//                                            a reach, for large sets
+//                                            a reach, for denser sets
 #include <cstdio>
 #include <cstring>
 #include <climits>
@@ -665,6 +667,7 @@ __device__ void setGrid(const Member& M) {
   setScalI(M.scal, SC_NCELLS, ncells);
   setScalI(M.scal, SC_MAXCOUNT, 0);
   setScalI(M.scal, SC_PAIRS, 0);
+  setScalI(M.scal, SC_CROWDED, 0);
 }
 
 __global__ void grid_kernel(const Member* mem, int nmem) {
@@ -1300,7 +1303,7 @@ struct RowTable {
 };
 
 template<bool FILL, int SUB>
-__device__ __noinline__ void walkWarp(const Member& M, const Grid& g, int64_t s, int32_t* sbuf, int cap, int maxNbr,
+__device__ __forceinline__ void walkWarp(const Member& M, const Grid& g, int64_t s, int32_t* sbuf, int cap, int maxNbr,
                                       int32_t* R) {
   const int lane = threadIdx.x & 31;
   const int scap = FILL ? 0 : M.grid.stashCap;
@@ -1419,6 +1422,13 @@ __device__ __noinline__ void walkWarp(const Member& M, const Grid& g, int64_t s,
     atomicAdd(reinterpret_cast<unsigned long long*>(M.scal + SC_PAIRS), (unsigned long long)above);
 }
 
+// (a call of its own where a kernel's registers are meant for other work)
+template<bool FILL>
+__device__ __noinline__ void walkWarpCall(const Member& M, const Grid& g, int64_t s, int32_t* sbuf, int cap, int maxNbr,
+                                          int32_t* R) {
+  walkWarp<FILL, 1>(M, g, s, sbuf, cap, maxNbr, R);
+}
+
 // A warp per sorted slot (walkWarp), cells of half a kernel reach.
 template<bool FILL>
 __global__ void __launch_bounds__(256) nbr_walk_kernel(const Member* mem, BlockMap bm, int cap, int maxNbr) {
@@ -1462,9 +1472,9 @@ __global__ void __launch_bounds__(256) nbr_walk_kernel(const Member* mem, BlockM
 // scan of its words' counts instead of one after the other: 702 us.
 constexpr int kCellThreads = 256;
 constexpr int kCellWarps = kCellThreads/32;
-constexpr int kCellCand = 1536;                        // nodes of the 27 cells that can be staged (more: walkWarp)
+constexpr int kCellCand = 1536;                        // nodes of the 27 cells that can be staged (more: crowded)
 constexpr int kCellTest = 1024;                        // of them within the reach of the cell: a ballot word per lane
-constexpr int kCellSort = 128;                         // nodes of a cell kept in node order (more: walkWarp)
+constexpr int kCellSort = 128;                         // nodes of a cell kept in node order (more: crowded)
 constexpr int kWalkers = 4;                            // walkers a warp tests at a time
 constexpr int64_t kCellBlocks = 148*16;                // blocks of a member, at most
 
@@ -1596,7 +1606,7 @@ __global__ void __launch_bounds__(kCellThreads, 4) nbr_cell_kernel(const Member*
   __shared__ int32_t cellS0[27];
   __shared__ int cellLen[27], cellAt[28];       // staged nodes of each cell, their first position
   __shared__ int rowAt[10], planeAt[4];
-  __shared__ int crowded;
+  __shared__ int crowded, listAt;
   const MemberBlock mb = memberBlock(bm);
   const Member& M = mem[mb.m];
   const int tid = threadIdx.x, lane = tid & 31, wib = tid >> 5;
@@ -1659,11 +1669,19 @@ __global__ void __launch_bounds__(kCellThreads, 4) nbr_cell_kernel(const Member*
     }
     __syncthreads();
     // too many to stage or to merge: a warp per walker, its list sorted by itself
+    // (nbr_crowded_kernel; the fill pass has the counting pass's list)
     auto walkAlone = [&]() {
+      if (!FILL) {
+        if (tid == 0) listAt = (int)atomicAdd(reinterpret_cast<unsigned long long*>(M.scal + SC_CROWDED),
+                                              (unsigned long long)(s1 - s0));
+        __syncthreads();
+        if (M.grid.crowdList) for (int32_t s = s0 + tid; s < s1; s += kCellThreads) M.cidx[listAt + (s - s0)] = s;
+      }
+      if (M.grid.crowdList) return;
       int32_t* rows = reinterpret_cast<int32_t*>(cellSmem) + wib*(cap + RowTable<1>::NR*RowTable<1>::RW);
       const Grid g = loadGrid(M);
       for (int32_t s = s0 + wib; s < s1; s += kCellWarps) {
-        walkWarp<FILL, 1>(M, g, s, rows + RowTable<1>::NR*RowTable<1>::RW, cap, maxNbr, rows);
+        walkWarpCall<FILL>(M, g, s, rows + RowTable<1>::NR*RowTable<1>::RW, cap, maxNbr, rows);
         __syncwarp();
       }
     };
@@ -1834,7 +1852,37 @@ __global__ void __launch_bounds__(kCellThreads, 4) nbr_cell_kernel(const Member*
   }
 }
 
+// The slots of the cell walk's crowded cells (listed in cidx, which is free
+// after the counting sort), a warp each over the whole grid.
+//
+// Why: the cell's own block has eight warps for them, so a problem whose nodes
+// lie in a few cells, or in one clump, would leave most of the chip idle behind
+// chains of dozens of walks.  The launch is left out while no build has seen a
+// crowded cell (Problem::crowd).  One slot a warp: in a loop over the list on a
+// fixed grid the walk is 20% slower (64^3 nodes at 216 a cell 20.2 against 16.8 ms).
+// Measured (B200, whole build, the cell's block -> the list): 16^3 nodes at nPerh 3
+// 6.1 -> 0.7 ms, 64^3 nodes with 4,000 of them in a clump 12.0 -> 2.4 ms.
+template<bool FILL>
+__global__ void __launch_bounds__(256, 3) nbr_crowded_kernel(const Member* mem, BlockMap bm, int cap, int maxNbr) {
+  extern __shared__ int32_t sbuf_all[];
+  __shared__ RowTable<1> rows[256/32];
+  const MemberBlock mb = memberBlock(bm);
+  const Member& M = mem[mb.m];
+  const int wib = threadIdx.x >> 5;
+  const bool collect = FILL || M.grid.stashCap > 0;
+  const int64_t w = (mb.block*(int64_t)blockDim.x + threadIdx.x) >> 5;
+  if (w >= scalI(M.scal, SC_CROWDED)) return;
+  walkWarp<FILL, 1>(M, loadGrid(M), M.cidx[w], sbuf_all + (collect ? wib*cap : 0), cap, maxNbr, rows[wib].v);
+}
+
+
 int64_t grow(int64_t v) { return v + v/4 + 1024; }
+
+// Cells of one kernel reach of the last build's grid (0: no build yet).
+double reach_cells(const Problem& p) {
+  const int sub = p.lastNbrCells > 0 ? p.lastNbrCells : 1;
+  return p.cellsWanted > 0 ? (double)p.cellsWanted/(double)(sub*sub*sub) : 0.0;
+}
 
 // Capacities for the next build, from the previous one (or first estimates).
 int plan_capacities(Batch& b) {
@@ -1845,20 +1893,25 @@ int plan_capacities(Batch& b) {
     const int64_t G = p.G > 0 ? p.G : p.hintG;
     const int64_t E = p.E > 0 ? p.E : p.hintE;
     if (G > 0) SPH_TRY(ensure_capacity_ghosts(p, grow(G)));
-    // schedule: a warp per node once the 27-cell candidate set of the last
-    // build kept 32 lanes busy, or once a thread's list would not fit in
+    // schedule: the cell walk (half-reach cells: a warp per node) once the
+    // 27-cell candidate set of the last build kept 32 lanes busy, or once a thread's list would not fit in
     // shared memory
-    const int lastSub = p.lastNbrCells > 0 ? p.lastNbrCells : 1;
-    const double cells1 = p.cellsWanted > 0 ? (double)p.cellsWanted/(double)(lastSub*lastSub*lastSub) : 0.0;
+    const double cells1 = reach_cells(p);
     const double candPerNode = cells1 > 0.0 ? 27.0*(double)(p.n + p.G)/cells1 : 0.0;
     const int req = p.nbrSchedule != NBR_SCHEDULE_AUTO ? p.nbrSchedule : b.nbrSchedule;
     p.fillSchedule = (req == NBR_SCHEDULE_WARP || (req == NBR_SCHEDULE_AUTO && candPerNode > 384.0) ||
                       sizeof(int32_t)*32*(size_t)(p.fillCap > 8 ? p.fillCap : 64) > kMaxListSmem)
                          ? NBR_SCHEDULE_WARP : NBR_SCHEDULE_THREAD;
     // cells per kernel reach: one unless requested (half-reach cells test
-    // fewer candidates but walk more rows; the autotuner measures both)
+    // fewer candidates but walk more rows; the autotuner measures both) or a
+    // quarter of the slots lay in cells too crowded for the cell walk: half-reach
+    // cells have no such limit.  Measured (B200, lattice 64^3, build): nPerh 1.8
+    // (47 nodes a cell) cell walk 1.25 ms, half-reach cells 2.79; 1.85 (51) 4.41 with the
+    // crowded cells' list, 2.82; nPerh 3 (216) 24.0, 14.3
     const int reqCells = p.nbrCells != 0 ? p.nbrCells : b.nbrCells;
-    p.grid.sub = reqCells != 0 ? reqCells : 1;
+    if (candPerNode < 0.8*p.denseSet) p.denseSet = 0.0;
+    p.grid.sub = reqCells != 0 ? reqCells : (p.fillSchedule == NBR_SCHEDULE_WARP && p.denseSet > 0.0 ? 2 : 1);
+    p.grid.crowdList = p.crowd != 0 ? 1 : 0;
     const int sub = p.grid.sub;
     // cells the grid wants at this subdivision (the last build's, rescaled), else the hint
     const int64_t cells = cells1 > 0.0 ? (int64_t)(cells1*sub*sub*sub) + 1 : p.hintCells;
@@ -2045,12 +2098,13 @@ int launch_build(Batch& b) {
   cell_scatter_kernel<<<capGrid, kGhostThreads, 0, st>>>(b.d_mem, cap); batch_count_launch(b);
   // ---- neighbor counts, offsets, lists
   int maxNbr = 0, tcap = 1, wmax = 0;
-  bool tstash = false, wstash = false;
+  bool tstash = false, wstash = false, alone = false;
   for (Problem* p : b.mem) {
     maxNbr = p->maxNbr > maxNbr ? p->maxNbr : maxNbr;
     if (p->fillSchedule == NBR_SCHEDULE_WARP) {
       wmax = p->fillCap > wmax ? p->fillCap : wmax;
       wstash = wstash || p->grid.stashCap > 0;
+      alone = alone || p->grid.crowdList == 0;
     } else {
       tcap = p->fillCap > tcap ? p->fillCap : tcap;
       tstash = tstash || p->grid.stashCap > 0;
@@ -2072,9 +2126,10 @@ int launch_build(Batch& b) {
   const size_t tsmem = sizeof(int32_t)*(size_t)fthreads*tcap;
   const size_t wsmem = sizeof(int32_t)*(wthreads/32)*(size_t)wcap;
   // the cell walk's staging area, at least a list and a row table per warp
+  // where a block may walk a crowded cell itself
   const size_t clists = sizeof(int32_t)*kCellWarps*(size_t)(wcap + RowTable<1>::NR*RowTable<1>::RW);
   const size_t cstage = sizeof(CellShared);
-  const size_t csmem = clists > cstage ? clists : cstage;
+  const size_t csmem = alone && clists > cstage ? clists : cstage;
   auto smemAttr = [](auto* kernel, size_t bytes) -> int {
     if (bytes <= 48*1024) return SPHGPU_OK;
     return cuda_status(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes),
@@ -2084,6 +2139,7 @@ int launch_build(Batch& b) {
   SPH_TRY(smemAttr(nbr_thread_kernel<false, 2>, tsmem)); SPH_TRY(smemAttr(nbr_thread_kernel<true, 2>, tsmem));
   SPH_TRY(smemAttr(nbr_cell_kernel<false>, csmem)); SPH_TRY(smemAttr(nbr_cell_kernel<true>, csmem));
   SPH_TRY(smemAttr(nbr_walk_kernel<false>, wsmem)); SPH_TRY(smemAttr(nbr_walk_kernel<true>, wsmem));
+  SPH_TRY(smemAttr(nbr_crowded_kernel<false>, wsmem)); SPH_TRY(smemAttr(nbr_crowded_kernel<true>, wsmem));
   // One walk launch per (schedule, cell subdivision) present.  pass 0: count
   // (and the lists of members with a stash); pass 1: fill (members without).
   auto walk = [&](bool threadSched, int sub, bool fill) -> int {
@@ -2120,6 +2176,15 @@ int launch_build(Batch& b) {
         else nbr_walk_kernel<false><<<grid, threads, smem, st>>>(b.d_mem, map, c, maxNbr);
       }
     }
+    batch_count_launch(b);
+    if (threadSched || sub != 1) return SPHGPU_OK;
+    SPH_TRY(batch_map_items(b, [&](const Problem& p) {
+      if (thread(p) || p.grid.sub != 1 || !p.grid.crowdList || (fill && p.grid.stashCap)) return (int64_t)0;
+      return 32*p.candcap; }, wthreads, &map, &grid));
+    if (!grid) return SPHGPU_OK;
+    const size_t smem = fill || wstash ? wsmem : 0;
+    if (fill) nbr_crowded_kernel<true><<<grid, wthreads, smem, st>>>(b.d_mem, map, wcap, maxNbr);
+    else nbr_crowded_kernel<false><<<grid, wthreads, smem, st>>>(b.d_mem, map, wcap, maxNbr);
     batch_count_launch(b);
     return SPHGPU_OK;
   };
@@ -2160,6 +2225,17 @@ int launch_build(Batch& b) {
 int plan_build(Batch& b) { return plan_capacities(b); }
 int launch_build_captured(Batch& b) { return launch_build(b); }
 
+// After a build: whether the cell walk has met crowded cells, and whether they
+// hold so much of the problem that it had better not be used.  Once it has, the
+// problem keeps the list (a run whose clump comes and goes is not captured
+// anew each time).
+void note_crowd(Problem& p, int64_t crowdedSlots) {
+  if (p.fillSchedule != NBR_SCHEDULE_WARP || p.grid.sub != 1) return;
+  if (crowdedSlots > 0) p.crowd = 1;
+  else if (p.crowd < 0) p.crowd = 0;
+  if (4*crowdedSlots > p.n + p.G && reach_cells(p) > 0.0) p.denseSet = 27.0*(double)(p.n + p.G)/reach_cells(p);
+}
+
 // Ghosts and ConnectivityMap of every member: all stages launched with the
 // sizes kept on the device, then one read-back of the sizes; a capacity
 // overflow grows the buffers and repeats the build.
@@ -2176,21 +2252,22 @@ int build_connectivity(Batch& b) {
       b.afterBuildLaunch = nullptr;
       SPH_TRY(f());
     }
-    const int slots[7] = {SC_G, SC_TOTAL, SC_MAXCOUNT, SC_PAIRS, SC_NCELLS, SC_CELLSWANTED, -1};
+    const int slots[8] = {SC_G, SC_TOTAL, SC_MAXCOUNT, SC_PAIRS, SC_NCELLS, SC_CELLSWANTED, -1, SC_CROWDED};
     std::vector<double> r;
-    SPH_TRY(batch_gather(b, slots, 7, r));
+    SPH_TRY(batch_gather(b, slots, 8, r));
     bool redo = false;
     for (int m = 0; m < nm; ++m) {
       Problem& p = *b.mem[m];
-      const int herr = (int)r[m*7 + 6];
-      p.G = asI64(r[m*7]);
+      const int herr = (int)r[m*8 + 6];
+      p.G = asI64(r[m*8]);
       p.ntot = p.n + p.G;
-      p.E = asI64(r[m*7 + 1]);
-      p.maxCount = asI32(r[m*7 + 2]);
-      p.pairs = asI64(r[m*7 + 3]);
-      p.ncells = asI64(r[m*7 + 4]);
-      p.cellsWanted = asI64(r[m*7 + 5]);
+      p.E = asI64(r[m*8 + 1]);
+      p.maxCount = asI32(r[m*8 + 2]);
+      p.pairs = asI64(r[m*8 + 3]);
+      p.ncells = asI64(r[m*8 + 4]);
+      p.cellsWanted = asI64(r[m*8 + 5]);
       p.lastNbrCells = p.grid.sub;
+      note_crowd(p, asI64(r[m*8 + 7]));
       if (herr) cudaMemsetAsync(p.d_err, 0, sizeof(int), b.stream);
       if ((herr & DERR_NBR_CAPACITY) || p.maxCount > p.maxNbr) {
         set_error("a node has more neighbors than max_neighbors");

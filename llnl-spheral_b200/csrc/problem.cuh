@@ -268,6 +268,8 @@ struct Grid {
                        // pair-acceleration buffer until compacted (0: separate fill pass)
   int64_t stashStride; // thread schedule: element c of sorted slot s at c*stashStride + s
   int sub;             // cells per kernel reach (1: 27-cell walk, 2: 125-cell walk with pruning)
+  int crowdList;       // cell walk: 1 = the slots of crowded cells are listed for a warp each, 0 = the
+                       // cell's block walks them
   float reach;         // kernel reach kappa*max(1/min(eig(H))) in cells (device-side, per build)
 };
 
@@ -295,6 +297,8 @@ struct Problem {
   int lastNbrPasses = 0;    // walks over the candidates the last build made (1 or 2)
   int fillCap = 0;          // neighbor-list capacity planned for the fill pass
   int fillSchedule = 0;     // schedule planned for this build (NBR_SCHEDULE_THREAD/WARP)
+  int crowd = -1;           // crowded cells seen by the cell walk: -1 not known, 0 none so far, 1 some
+  double denseSet = 0.0;    // candidates per node when a quarter of the slots was crowded (0: never)
   // sizes the first neighbor build plans its buffers from (0: built-in guesses)
   int64_t hintG = 0, hintE = 0, hintCells = 0;
 
@@ -442,7 +446,8 @@ enum ScalSlot {
   SC_STEPS = 41,       // completed steps since the host last reset it (i64)
   SC_PAIRSUM = 42,     // pair interactions evaluated by all completed steps (i64)
   SC_PHMAX = 43,       // 6 ghost hmax words, one per boundary pass (fused ghost passes, double bits)
-  NSCAL = 49
+  SC_CROWDED = 49,     // slots of the cell walk's crowded cells (i64)
+  NSCAL = 50
 };
 
 // Sizes and grid of the current connectivity (device side).
@@ -609,6 +614,7 @@ int batch_scan(Batch& b, int which);
 // ---- stages (ghosts/neighbors: nbrs.cu; SPH: sph.cu; mixed: sph_mixed.cu; CRKSPH: crk.cu)
 int build_connectivity(Batch& b);     // ghosts + ConnectivityMap, device-sized
 int plan_build(Batch& b);             // capacities and schedules of the next build
+void note_crowd(Problem& p, int64_t crowdedSlots);
 int launch_build_captured(Batch& b);  // the build's launches, sized on the device, no read-back
 // FP64 pair records of the members that read them next (PACK_ALL: every member)
 enum PackNeed { PACK_ALL = 0, PACK_FOR_EVAL = 1, PACK_FOR_FINALIZE = 2 };

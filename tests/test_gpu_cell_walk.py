@@ -105,3 +105,53 @@ def test_pairs_across_large_cells(gpu_lib, pkg):
     np.fill_diagonal(near, False)
     assert near.sum() == 2 * pairs and not near[:2].any()
     assert np.array_equal(np.diff(off), near.sum(1)) and np.array_equal(nbr, np.nonzero(near)[1])
+
+
+@pytest.mark.parametrize("passes", [1, 2])
+def test_crowded_cells_appear(gpu_lib, pkg, oracle_mod, passes):
+    """Crowded cells that no earlier build of the problem had (their block walks
+    them), then the builds after it (their slots are listed), then none again."""
+    ns, cfg = _clump(pkg, 300, 11, (1, 1, 1), True)
+    rng = np.random.default_rng(3)
+    spread = pkg.generators.NodeSet(rng.uniform(0.0, 1.0, (ns.n, 3)), ns.vel, ns.mass, ns.rho, ns.eps, ns.H, ns.dx)
+    g = pkg.SPHHydro(cfg, spread)
+    g.set_schedule("neighbor walk", 2)
+    g.set_schedule("neighbor passes", passes)
+    for nodes in (spread, ns, spread):
+        g.set_state(nodes)
+        o = oracle_mod.OracleProblem(cfg, nodes)
+        o.build_neighbors()
+        for _ in range(2):
+            g.build_neighbors()
+            _same_connectivity(g, o)
+
+
+@pytest.mark.parametrize("nPerh", [2.0, 3.0])
+def test_dense_sets(gpu_lib, pkg, oracle_mod, nPerh):
+    """64 and 216 nodes per cell in the automatic schedule: the thread walk, the
+    cell walk with every cell crowded, half-reach cells, then the steps' rebuilds,
+    in a batch with a set that keeps the cell walk."""
+    gen, abi = pkg.generators, pkg.abi
+    ns = gen.kelvin_helmholtz(nx=15, ny=15, nz=15, nPerh=nPerh, jitter=0.1)
+    cfg = gen.kh_config(abi, kernel=abi.KERNEL_BSPLINE, nPerh=nPerh, max_neighbors=2048, dtMin=1.0e-4, dtMax=1.0e-4)
+    g = pkg.SPHHydro(cfg, ns)
+    o = oracle_mod.OracleProblem(cfg, ns)
+    o.build_neighbors()
+    cells = []
+    for _ in range(4):
+        g.build_neighbors()
+        _same_connectivity(g, o)
+        cells.append(g.schedule("neighbor cells"))
+    assert cells[0] == 1 and cells[-1] == 2
+    box = ((0.0, 0.0, 0.0), (1.0, 0.25, 0.25))
+    tube = gen.sod(nx=32, ny=8, nz=8, box=box)
+    tcfg = gen.sod_config(abi, ns_box=box)
+    pair = [pkg.SPHHydro(cfg, ns), pkg.SPHHydro(tcfg, tube)]
+    alone = [g, pkg.SPHHydro(tcfg, tube)]
+    g.set_state(ns)
+    for h in alone:
+        h.step(3)
+    pkg.SPHBatch(pair).step(3)
+    for a, b in zip(alone, pair):
+        for k in ("position", "velocity", "mass density", "specific thermal energy", "H"):
+            assert np.array_equal(a.field(k), b.field(k)), k
