@@ -1218,7 +1218,7 @@ int sphgpu_create(const sphgpu_config* cfg, int64_t n_internal, sphgpu_problem**
     if ((rc = ensure_capacity_ghosts(*p, n/2 + 4096)) != SPHGPU_OK) break;
     p->solo = new (std::nothrow) Batch();
     if (p->solo == nullptr) { set_error("host allocation failed"); rc = SPHGPU_ERR_NOMEM; break; }
-    if ((rc = batch_init(solo(p), p->stream)) != SPHGPU_OK) break;
+    if ((rc = batch_init(solo(p), p->stream, false)) != SPHGPU_OK) break;
     p->solo->mem.push_back(p);
     if ((rc = cuda_status(cudaDeviceSynchronize(), "create")) != SPHGPU_OK) break;
   } while (false);
@@ -1735,7 +1735,7 @@ int sphgpu_batch_create(sphgpu_problem* const* members, int32_t count, sphgpu_ba
   int rc = cuda_status(cudaStreamCreateWithFlags(&st, cudaStreamNonBlocking), "batch stream");
   if (rc == SPHGPU_OK) {
     b->ownStream = true;
-    rc = batch_init(*b, st);
+    rc = batch_init(*b, st, count > 1);
     b->ownStream = true;
   }
   if (rc != SPHGPU_OK) {

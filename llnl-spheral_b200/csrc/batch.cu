@@ -244,11 +244,19 @@ int64_t scan_items(const Problem& p, int which) { return scanCapacity(p.n, p.can
 
 Member describe_member(const Problem& p) { return member_of(p); }
 
-int batch_init(Batch& b, cudaStream_t stream) {
+int batch_init(Batch& b, cudaStream_t stream, bool maps) {
   b.stream = stream;
   for (int k = 0; k < Batch::kMemSlots; ++k)
     if (cudaEventCreateWithFlags(&b.memEvents[k], cudaEventDisableTiming) != cudaSuccess)
       return cuda_status(cudaGetLastError(), "batch event");
+  if (!maps) return SPHGPU_OK;
+  if (dev_alloc(reinterpret_cast<void**>(&b.d_maps), sizeof(int32_t)*kMapRing) != cudaSuccess ||
+      cudaMallocHost(&b.h_maps, sizeof(int32_t)*kMapRing) != cudaSuccess) {
+    set_error("batch block-map ring allocation failed");
+    return SPHGPU_ERR_NOMEM;
+  }
+  b.mapcap = kMapRing;
+  b.mappos = 0;
   return SPHGPU_OK;
 }
 
@@ -335,20 +343,6 @@ int batch_map(Batch& b, const std::vector<int64_t>& blocks, BlockMap* bm, unsign
     bm->nmem = nm;
     *grid = (unsigned)total;
     return SPHGPU_OK;
-  }
-  // the ring is made when a batch of several members first maps a launch (a
-  // single problem never does: 4 MB of pinned memory each)
-  if (b.d_maps == nullptr) {
-    if (dev_alloc(reinterpret_cast<void**>(&b.d_maps), sizeof(int32_t)*kMapRing) != cudaSuccess ||
-        cudaMallocHost(&b.h_maps, sizeof(int32_t)*kMapRing) != cudaSuccess) {
-      dev_free(b.d_maps);
-      b.d_maps = nullptr;
-      b.h_maps = nullptr;
-      set_error("batch block-map ring allocation failed");
-      return SPHGPU_ERR_NOMEM;
-    }
-    b.mapcap = kMapRing;
-    b.mappos = 0;
   }
   const int64_t need = ((int64_t)nm + 1 + 31) & ~(int64_t)31;
   if (need > b.mapcap) { set_error("batch too large for the block-map ring"); return SPHGPU_ERR_CAPACITY; }

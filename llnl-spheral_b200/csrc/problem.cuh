@@ -571,7 +571,9 @@ struct Batch {
 };
 
 // batch.cu
-int batch_init(Batch& b, cudaStream_t stream);
+// maps: with the block-map ring that a batch of several members needs (4 MB of
+// pinned and of device memory; a single problem never maps a launch)
+int batch_init(Batch& b, cudaStream_t stream, bool maps);
 
 // Device buffers of problems and batches come from one stream-ordered memory
 // pool per device that keeps freed blocks (release threshold unlimited), so

@@ -125,7 +125,7 @@ int server_device(sphgpu_server& s) {
   cudaStream_t st = nullptr;
   int rc = cuda_status(cudaStreamCreateWithFlags(&st, cudaStreamNonBlocking), "server stream");
   if (rc != SPHGPU_OK) return rc;
-  rc = batch_init(s.batch, st);
+  rc = batch_init(s.batch, st, true);
   s.batch.ownStream = true;
   if (rc != SPHGPU_OK) {
     batch_free(s.batch);

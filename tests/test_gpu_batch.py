@@ -287,3 +287,22 @@ def test_batch_rejects_duplicates(gpu_lib, pkg):
     a = pkg.SPHHydro(cfg, ns)
     with pytest.raises(RuntimeError):
         pkg.SPHBatch([a, a])
+
+
+def test_first_build_makes_no_block_map_ring(gpu_lib, pkg):
+    """The 4 MB block-map ring of a batch is made with the batch; its first build
+    pins only the small descriptor ring and the gather buffer."""
+    import torch
+    from torch.profiler import ProfilerActivity, profile
+
+    mem = [pkg.SPHHydro(cfg, ns) for ns, cfg in _specs(pkg)[:2]]
+
+    def pinned(work):
+        with profile(activities=[ProfilerActivity.CPU, ProfilerActivity.CUDA]) as prof:
+            out = work()
+            torch.cuda.synchronize()
+        return out, sum(e.name in ("cudaMallocHost", "cudaHostAlloc") for e in prof.events())
+
+    batch, made = pinned(lambda: pkg.SPHBatch(mem))
+    _, first = pinned(batch.build_neighbors)
+    assert made >= 1 and first <= 2
