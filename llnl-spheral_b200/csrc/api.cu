@@ -498,7 +498,7 @@ uint64_t graph_key(const Batch& b) {
     // sizes and plans that set launch shapes, kernel variants and shared memory
     const int64_t sizes[] = {p->n, p->gcap, p->ecap, p->candcap, p->cellcap, p->reccap, p->creccap,
                              p->mreccap, p->blockSumsCap, p->redcap, p->maxNbr, p->fillCap, p->fillSchedule,
-                             p->grid.sub, p->grid.stashCap, p->grid.stashStride, p->grid.crowdList, p->crowd > 0, p->denseSet > 0.0};
+                             p->grid.sub, p->grid.stashCap, p->grid.stashStride, p->grid.crowdList, p->crowd > 0, p->denseSet > 0.0, longRows(*p)};
     for (int64_t v : sizes) mix((uint64_t)v);
   }
   return h;
@@ -757,6 +757,7 @@ int run_graph_steps(Batch& b, int64_t count, int64_t* done) {
     p.G = asI64(a[4]);
     p.ntot = p.n + p.G;
     p.E = asI64(a[5]);
+    note_rows(p);
     p.maxCount = asI32(a[6]);
     p.pairs = asI64(a[7]);
     p.ncells = asI64(r2[4*m]);

@@ -2262,6 +2262,7 @@ int build_connectivity(Batch& b) {
       p.G = asI64(r[m*8]);
       p.ntot = p.n + p.G;
       p.E = asI64(r[m*8 + 1]);
+      note_rows(p);
       p.maxCount = asI32(r[m*8 + 2]);
       p.pairs = asI64(r[m*8 + 3]);
       p.ncells = asI64(r[m*8 + 4]);

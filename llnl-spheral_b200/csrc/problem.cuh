@@ -284,6 +284,7 @@ struct Problem {
   int64_t G = 0;            // ghosts
   int64_t gcap = 0;
   int64_t E = 0, ecap = 0;  // CSR entries
+  bool longRow = false;     // rows long enough for a group of lanes per node (longRows)
   int64_t pairs = 0;        // unordered pairs (ncalc)
   int64_t pairsEvaluated = 0;  // pair interactions of every evaluation in the RK2 steps so far
   int maxNbr = 1024;
@@ -723,7 +724,13 @@ int cuda_status(cudaError_t e, const char* where);
 // on average, and below that the thread-per-node kernels' full lanes win (the
 // 7.8 entries of Kelvin-Helmholtz leave half of two batches empty).
 constexpr int64_t kLongRow = 32;
-inline bool longRows(const Problem& p) { return p.E >= kLongRow*p.n; }
+inline bool longRows(const Problem& p) { return p.longRow; }
+// After a build.  Back to the thread-per-node kernels a little below the line, so
+// that a run whose mean lies on it is not captured anew with every change.
+inline void note_rows(Problem& p) {
+  if (p.E >= kLongRow*p.n) p.longRow = true;
+  else if (p.E < (kLongRow - 2)*p.n) p.longRow = false;
+}
 constexpr int kRowMaxNodes = 2;       // nodes per group of a block, at most
 // Nodes per group: as many as leave two waves of blocks of 8 groups.
 inline int rowNodes(int64_t nodes) {

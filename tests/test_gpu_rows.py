@@ -127,3 +127,33 @@ def test_paired_planes_of_large_problems(gpu_lib, pkg, precision):
     small.step(1)
     for k in ("position", "velocity", "mass density", "specific thermal energy", "H"):
         assert np.array_equal(large.field(k)[sel][inner], small.field(k)[inner]), k
+
+
+@pytest.mark.parametrize("first,then", [(0.17, 0.1), (0.1, 0.17)])
+def test_captured_step_follows_the_row_length(gpu_lib, pkg, first, then):
+    """A new state in the same buffers with long rows in place of short ones, or
+    the other way round: the steps after it run the kernels that a new problem
+    of that state runs (the captured step of the old rows is right, but slow)."""
+    gen, abi = pkg.generators, pkg.abi
+
+    def state(h):
+        ns = gen.kelvin_helmholtz(nx=8, ny=8, nz=8, jitter=0.1)
+        ns.H[:, [0, 3, 5]] = 1.0 / h
+        return ns
+
+    # H follows the density, not the ideal neighbor count: the rows keep their length
+    cfg = gen.kh_config(abi, kernel=abi.KERNEL_BSPLINE, HUpdate=abi.H_INTEGRATE, dtMin=1.0e-4, dtMax=1.0e-4)
+    launches = []
+    for states in ((first, then), (then,)):
+        g = pkg.SPHHydro(cfg, state(max(first, then)))
+        g.build_neighbors()                    # (both problems' buffers hold the long rows)
+        for h in states:
+            g.set_state(state(h))
+            g.step(6)
+            g.step(6)
+        before = g.kernel_launches()
+        g.step(6)
+        launches.append(g.kernel_launches() - before)
+        rows = np.diff(g.connectivity()[0]).mean()
+        assert (rows >= 32) == (then > 0.15)
+    assert launches[0] == launches[1]
