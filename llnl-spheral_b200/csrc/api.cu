@@ -978,6 +978,7 @@ int autotune_impl(Batch& b, double* report) {
     int bestS = NBR_SCHEDULE_AUTO;
     for (int k = 0; k < 2 && rc == SPHGPU_OK; ++k) {
       b.nbrSchedule = schedules[k];
+      b.nbrCells = 1;
       double ms = 0.0;
       rc = timeit([&]() { return build_neighbors_impl(b); }, &ms);
       out[1 + k] = ms;
