@@ -298,7 +298,9 @@ int sphgpu_kernel_launches(sphgpu_problem* p, int64_t* launches);
  * candidate sets: a block per cell that shares its candidates (cells of one
  * kernel reach), a warp per node (half a reach).  Every schedule yields the
  * same ConnectivityMap.
- * stage "pair loop": threads per block of the derivative kernels, 64 or 128.
+ * stage "pair loop": threads per block of the derivative kernels with a thread
+ * per node, 64 or 128 (SPH members with 32 neighbors per node and more have a
+ * group of lanes per node, always in blocks of 128).
  * stage "neighbor filter": 1 (default) = an FP32 pre-test decides the pairs
  * clearly inside or outside the kernel support and the exact FP64 test the
  * rest (used only while every H has condition number <= 100, where the FP32
@@ -340,9 +342,10 @@ int sphgpu_get_schedule(sphgpu_problem* p, const char* stage, int32_t* schedule)
  * fastest.  Results do not depend on the schedule; the call leaves the
  * connectivity rebuilt and the derivatives evaluated at the current state (as
  * sphgpu_build_neighbors, sphgpu_initialize and sphgpu_evaluate_derivatives
- * do).  report (may be NULL) = {neighbor schedule, ms thread, ms warp,
- * pair-loop threads, ms 64, ms 128, cells per kernel reach, ms with
- * half-reach cells}. */
+ * do).  report (may be NULL) = {neighbor schedule, ms of schedule 1, ms of
+ * schedule 2, pair-loop threads, ms 64, ms 128, cells per kernel reach, ms with
+ * half-reach cells}; where the pair loop's threads reach no member they are not
+ * compared and both times are the one measured. */
 int sphgpu_autotune(sphgpu_problem* p, double report[8]);
 /* ---- batches (no counterpart in the reference, which advances one problem
  * at a time).  A batch advances many independent problems together: each

@@ -998,16 +998,19 @@ int autotune_impl(Batch& b, double* report) {
     if ((rc = pack_records(b)) != SPHGPU_OK) break;
     if ((rc = initialize_impl(b)) != SPHGPU_OK) break;
     if ((rc = hold_restart_state(b)) != SPHGPU_OK) break;
-    // pair loop: threads per block
+    // pair loop: threads per block (timed once, and left as it is, where no
+    // member has a kernel that it reaches)
     const int widths[2] = {64, 128};
     best = 1e300;
-    int bestW = 128;
-    for (int k = 0; k < 2 && rc == SPHGPU_OK; ++k) {
-      b.evalThreads = widths[k];
+    int bestW = b.evalThreads;
+    const bool reached = anyMember(b, [](const Problem& p) { return isCrkP(p) || !longRows(p); });
+    for (int k = 0; k < (reached ? 2 : 1) && rc == SPHGPU_OK; ++k) {
+      if (reached) b.evalThreads = widths[k];
       double ms = 0.0;
       rc = timeit([&]() { return launch_eval(b); }, &ms);
       out[4 + k] = ms;
-      if (ms < best) { best = ms; bestW = widths[k]; }
+      if (!reached) out[5] = ms;
+      else if (ms < best) { best = ms; bestW = widths[k]; }
     }
     b.evalThreads = bestW;
     out[3] = bestW;

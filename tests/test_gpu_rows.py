@@ -157,3 +157,17 @@ def test_captured_step_follows_the_row_length(gpu_lib, pkg, first, then):
         rows = np.diff(g.connectivity()[0]).mean()
         assert (rows >= 32) == (then > 0.15)
     assert launches[0] == launches[1]
+
+
+@pytest.mark.parametrize("threads", [64, 128])
+def test_autotune_leaves_the_pair_loop_of_long_rows(gpu_lib, pkg, threads):
+    """The kernels with a group of lanes per node have no choice of threads: the
+    autotuner reports one time and keeps the caller's value."""
+    gen, abi = pkg.generators, pkg.abi
+    box = ((0.0, 0.0, 0.0), (1.0, 0.25, 0.25))
+    g = pkg.SPHHydro(gen.sod_config(abi, ns_box=box), gen.sod(nx=32, ny=8, nz=8, box=box))
+    g.set_schedule("pair loop", threads)
+    g.build_neighbors()
+    rep = g.autotune()
+    assert rep["pair loop"] == threads and g.schedule("pair loop") == threads
+    assert rep["pair loop ms"][64] == rep["pair loop ms"][128] > 0
