@@ -1,8 +1,9 @@
 """The cell walk (neighbor walk 2 over cells of one kernel reach) where its
 staging changes form: cells with more nodes than one, two and four registers
 per lane hold, cells it leaves unordered, windows beyond the staging area and
-beyond the tested candidates, nodes in no order.  The ConnectivityMap is
-integer work: every entry equals the oracle's."""
+beyond the tested candidates, nodes in no order, any unit of length, crowded
+cells that come and go.  The ConnectivityMap is integer work: every entry equals
+the oracle's."""
 import numpy as np
 import pytest
 
@@ -25,8 +26,8 @@ def _clump(pkg, clump, seed, periodic, vary):
     return full, cfg
 
 
-# 20: one register per lane; 50, 100: two and four; 140: a cell left unordered; 800: the 27 cells still fit the
-# staging area, 1100: more than a ballot word per lane; 1700: more than the staging area
+# 20: one register per lane in the cells' ordering; 50, 100: two and four; 140 and more: cells left unordered, whose
+# windows are all crowded (test_full_windows has the windows that fill the staging area and the ballots)
 @pytest.mark.parametrize("clump", [20, 50, 100, 140, 800, 1100, 1700])
 @pytest.mark.parametrize("passes", [1, 2])
 @pytest.mark.parametrize("periodic,vary", [((1, 1, 1), False), ((1, 0, 1), True)])
@@ -169,3 +170,61 @@ def test_autotune_of_a_dense_set(gpu_lib, pkg):
     assert g.schedule("neighbor cells") == 2
     rep = g.autotune()
     assert rep["neighbor cells"] == 2 and rep["neighbor cells ms"][2] < 0.9 * rep["neighbor cells ms"][1]
+
+
+def _windows(o, ns, reach, periodic):
+    """Nodes of each cell, and for every cell with an internal node the nodes of its 27-cell window and those of
+    them within reach of the cell (setGrid, nbr_cell_kernel)."""
+    pos = np.concatenate([ns.pos, o.ghost_positions()])
+    lo, hi = ns.pos.min(0), ns.pos.max(0)
+    for a in range(3):
+        if periodic[a]:
+            lo[a], hi[a] = min(lo[a], -1.001 * reach), max(hi[a], 1.0 + 1.001 * reach)
+    edge = 1.001 * reach
+    dim = ((hi - lo) / edge).astype(int) + 1
+    at = np.clip(((pos - lo) / edge).astype(int), 0, dim - 1)
+    cells = {}
+    for k, c in enumerate(map(tuple, at)):
+        cells.setdefault(c, []).append(k)
+    staged, tested = [], []
+    for c in set(map(tuple, at[:ns.n])):
+        window = [k for dz in (-1, 0, 1) for dy in (-1, 0, 1) for dx in (-1, 0, 1)
+                  for k in cells.get((c[0] + dx, c[1] + dy, c[2] + dz), [])]
+        corner = lo + np.array(c) * edge
+        gap = np.maximum(np.maximum(corner - pos[window], pos[window] - corner - edge), 0.0)
+        staged.append(len(window))
+        tested.append(int(((gap ** 2).sum(1) <= reach ** 2).sum()))
+    return max(map(len, cells.values())), np.array(staged), np.array(tested)
+
+
+# windows whose candidates need up to 32 ballot words; more candidates than ballot words hold; more nodes than the
+# staging area holds: all with every cell in node order
+@pytest.mark.parametrize("per_cell,branch", [(47.5, "words"), (54.0, "tested"), (63.0, "staged")])
+@pytest.mark.parametrize("passes", [1, 2])
+@pytest.mark.parametrize("periodic", [(1, 1, 1), (1, 0, 0)])
+def test_full_windows(gpu_lib, pkg, oracle_mod, per_cell, branch, passes, periodic):
+    gen, abi = pkg.generators, pkg.abi
+    n = 3000
+    rng = np.random.default_rng(17)
+    h = 0.5 * (per_cell / n) ** (1.0 / 3.0) / 1.001
+    H = np.zeros((n, 6))
+    H[:, [0, 3, 5]] = 1.0 / h
+    ns = gen.NodeSet(rng.uniform(0.0, 1.0, (n, 3)), np.zeros((n, 3)), np.full(n, 1.0 / n), np.ones(n), np.ones(n), H, h)
+    cfg = gen.kh_config(abi, kernel=abi.KERNEL_BSPLINE, periodic=periodic, max_neighbors=2048)
+    o = oracle_mod.OracleProblem(cfg, ns)
+    o.build_neighbors()
+    largest, staged, tested = _windows(o, ns, 2.0 * h, periodic)
+    assert largest <= 128
+    if branch == "words":
+        assert ((staged <= 1536) & (tested > 992) & (tested <= 1024)).any()
+    elif branch == "tested":
+        assert ((staged <= 1536) & (tested > 1024)).any() and (tested <= 1024).any()
+    else:
+        assert (staged > 1536).any() and (staged <= 1536).any()
+    g = pkg.SPHHydro(cfg, ns)
+    g.set_schedule("neighbor walk", 2)
+    g.set_schedule("neighbor cells", 1)
+    g.set_schedule("neighbor passes", passes)
+    for _ in range(2):
+        g.build_neighbors()
+        _same_connectivity(g, o)

@@ -119,6 +119,69 @@ def test_ghost_passes_every_schedule(gpu_lib, pkg, oracle_mod, case, passes):
     assert np.array_equal(g.connectivity()[1], o.connectivity()[1])
 
 
+def _ghosts(g):
+    g.build_neighbors()
+    off, nbr, root = g.connectivity()
+    return root, g.ghost_positions(), off, nbr
+
+
+# 32,768 nodes: the most that the automatic schedule builds with a cluster of blocks per problem
+@pytest.mark.parametrize("n", [32767, 32768, 32769])
+def test_ghost_schedules_at_the_cluster_limit(gpu_lib, pkg, n):
+    """The automatic schedule and the two others make the same ghosts in the same
+    order, the same positions and lists."""
+    gen, abi = pkg.generators, pkg.abi
+    ns = gen.kelvin_helmholtz(nx=33, ny=32, nz=32, jitter=0.2)
+    sel = np.sort(np.random.default_rng(n).permutation(ns.n)[:n])
+    ns = gen.NodeSet(ns.pos[sel], ns.vel[sel], ns.mass[sel], ns.rho[sel], ns.eps[sel], ns.H[sel], ns.dx)
+    g = pkg.SPHHydro(gen.kh_config(abi), ns)
+    want = None
+    for passes in (1, 0, 2):
+        g.set_schedule("ghost passes", passes)
+        got = _ghosts(g)
+        want = want or got
+        assert got[0].size > 1000 and all(np.array_equal(a, b) for a, b in zip(got, want))
+
+
+@pytest.mark.parametrize("periodic", [(1, 1, 1), (0, 1, 0)])
+def test_ghosts_without_nodes_near_the_planes(gpu_lib, pkg, oracle_mod, periodic):
+    """No node near a periodic plane, every schedule: no ghosts."""
+    gen, abi = pkg.generators, pkg.abi
+    ns = gen.kelvin_helmholtz(nx=10, ny=10, nz=10, box=((0.3, 0.3, 0.3), (0.7, 0.7, 0.7)))
+    cfg = gen.kh_config(abi, periodic=periodic)
+    o = oracle_mod.OracleProblem(cfg, ns)
+    o.build_neighbors()
+    assert o.num_ghosts() == 0
+    g = pkg.SPHHydro(cfg, ns)
+    for passes in (0, 1, 2):
+        g.set_schedule("ghost passes", passes)
+        root, _, off, nbr = _ghosts(g)
+        assert root.size == 0 and np.array_equal(off, o.connectivity()[0]) and np.array_equal(nbr, o.connectivity()[1])
+
+
+def test_ghosts_of_a_batch_with_and_without_periodic_planes(gpu_lib, pkg):
+    """A batch of a periodic, a non-periodic and a partly periodic member, every
+    schedule: each as alone."""
+    gen, abi = pkg.generators, pkg.abi
+    sets = [((1, 1, 1), 12), ((0, 0, 0), 9), ((0, 1, 0), 15)]
+
+    def members():
+        return [pkg.SPHHydro(gen.kh_config(abi, periodic=p), gen.kelvin_helmholtz(nx=m, ny=m, nz=m, jitter=0.2))
+                for p, m in sets]
+
+    alone = [_ghosts(g) for g in members()]
+    assert alone[0][0].size > 0 and alone[1][0].size == 0 and alone[2][0].size > 0
+    for passes in (0, 1, 2):
+        together = members()
+        batch = pkg.SPHBatch(together)
+        batch.set_schedule("ghost passes", passes)
+        batch.build_neighbors()
+        for g, want in zip(together, alone):
+            off, nbr, root = g.connectivity()
+            got = (root, g.ghost_positions(), off, nbr)
+            assert all(np.array_equal(a, b) for a, b in zip(got, want))
+
+
 @pytest.mark.parametrize("case", list(CASES))
 def test_evaluate_derivatives_parity(gpu_lib, pkg, oracle_mod, case):
     g, o, ns = _pair(pkg, oracle_mod, case)

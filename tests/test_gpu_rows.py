@@ -1,8 +1,9 @@
-"""The group-of-lanes FP64 pair kernel (rows of 32 entries and more) at the edges
-of its batches of 16 entries and its blocks of 8 and 16 nodes.  It forms the
-same terms and adds them in the same order as the oracle, so every derivative
-is bit-equal except the cube root of the ideal-H moment (CUDA pow against
-glibc pow, 2 ulp: 1e-12 is the specification's tolerance)."""
+"""The group-of-lanes kernels (rows of 32 entries and more) at the edges of their
+batches of 16 entries and their blocks of 8 nodes, and of 16 from 18,944 nodes
+on.  The FP64 pair kernel forms the same terms and adds them in the same order
+as the oracle, so every derivative is bit-equal except the cube root of the
+ideal-H moment (CUDA pow against glibc pow, 2 ulp: 1e-12 is the specification's
+tolerance)."""
 import numpy as np
 import pytest
 
@@ -16,7 +17,7 @@ KEYS = ["delta velocity hydro", "delta specific thermal energy", "delta mass den
         "XSPH delta vi"]
 
 
-# nodes: one block short of its last group, odd counts, one node more than a block of 8 and of 16
+# nodes: full blocks of 8, one node more than a full block (449, 497, 505)
 @pytest.mark.parametrize("keep", [512, 505, 497, 449])
 @pytest.mark.parametrize("options", [{}, {"XSPH": 1}, {"epsTensile": 0.3, "compatibleEnergyEvolution": 0},
                                      {"balsaraShearCorrection": 1}])
@@ -171,3 +172,130 @@ def test_autotune_leaves_the_pair_loop_of_long_rows(gpu_lib, pkg, threads):
     rep = g.autotune()
     assert rep["pair loop"] == threads and g.schedule("pair loop") == threads
     assert rep["pair loop ms"][64] == rep["pair loop ms"][128] > 0
+
+
+def _ragged(pkg, n, seed):
+    """n nodes of a jittered 27^3 lattice in the unit cube, rows of about 40 entries."""
+    gen = pkg.generators
+    ns = gen.kelvin_helmholtz(nx=27, ny=27, nz=27, nPerh=1.1, jitter=0.1, seed=seed)
+    sel = np.sort(np.random.default_rng(seed).permutation(ns.n)[:n])
+    return gen.NodeSet(ns.pos[sel], ns.vel[sel], ns.mass[sel], ns.rho[sel], ns.eps[sel], ns.H[sel], ns.dx)
+
+
+# from 18,944 nodes the blocks have two nodes per group of lanes, 16 in all: every kind of last block (its first pass
+# full or not, its second empty, with one node, with seven, all but one)
+@pytest.mark.parametrize("n,options", [(18944, {}), (19009, {"XSPH": 1}), (19015, {"XSPH": 1}), (19016, {}),
+                                       (19017, {"epsTensile": 0.3, "compatibleEnergyEvolution": 0}),
+                                       (19023, {"XSPH": 1, "balsaraShearCorrection": 1})])
+def test_rows_of_large_problems(gpu_lib, pkg, oracle_mod, n, options):
+    """FP64 bit for bit with the oracle; the mixed form within its 1e-5 of FP64."""
+    gen, abi = pkg.generators, pkg.abi
+    ns = _ragged(pkg, n, n)
+    cfg = gen.kh_config(abi, kernel=abi.KERNEL_BSPLINE, nPerh=1.1, **options)
+    g, o = pkg.SPHHydro(cfg, ns), oracle_mod.OracleProblem(cfg, ns)
+    for p in (g, o):
+        p.build_neighbors()
+    assert np.diff(g.connectivity()[0]).mean() >= 32
+    if options.get("balsaraShearCorrection"):
+        g.initialize(), o.initialize()
+    g.evaluateDerivatives()
+    o.evaluate_derivatives()
+    for k in KEYS:
+        assert np.array_equal(g.field(k), o.field(k)), k
+    assert normwise(g.field("new H"), o.field("new H")) <= 1e-12
+    m = pkg.SPHHydro(gen.kh_config(abi, kernel=abi.KERNEL_BSPLINE, nPerh=1.1, precision=abi.PRECISION_MIXED, **options), ns)
+    m.build_neighbors()
+    if options.get("balsaraShearCorrection"):
+        m.initialize()
+    m.evaluateDerivatives()
+    for k in KEYS + ["new H"]:
+        assert normwise(m.field(k), g.field(k)) <= 1e-5, k
+
+
+@pytest.mark.parametrize("n", [19009, 19015])
+def test_ragged_steps_of_large_problems(gpu_lib, pkg, oracle_mod, n):
+    """A step with the compatible energy of long rows at such sizes: the oracle's
+    state within the specification's 1e-12."""
+    gen, abi = pkg.generators, pkg.abi
+    ns = _ragged(pkg, n, n)
+    cfg = gen.kh_config(abi, kernel=abi.KERNEL_BSPLINE, nPerh=1.1)
+    g, o = pkg.SPHHydro(cfg, ns), oracle_mod.OracleProblem(cfg, ns)
+    g.step(1)
+    o.step(1)
+    for k in ("position", "velocity", "mass density", "specific thermal energy", "H"):
+        assert normwise(g.field(k), o.field(k)) <= 1e-12, k
+
+
+@pytest.mark.parametrize("precision", ["PRECISION_FP64", "PRECISION_MIXED"])
+def test_uneven_batch_with_two_nodes_per_group(gpu_lib, pkg, precision):
+    """Members of one node per group of lanes alone and of two in the batch (19,001
+    nodes in all): bit for bit the same."""
+    gen, abi = pkg.generators, pkg.abi
+    cfg = gen.kh_config(abi, kernel=abi.KERNEL_BSPLINE, nPerh=1.1, XSPH=1, precision=getattr(abi, precision))
+
+    def members():
+        out = []
+        for n in (7001, 6993, 5007):
+            ns = _ragged(pkg, n, n)
+            ns.H[:] *= (n / 19683.0) ** (1.0 / 3.0)          # (thinned: the rows keep their length)
+            out.append(pkg.SPHHydro(cfg, ns))
+        return out
+
+    alone, together = members(), members()
+    for h in alone:
+        h.build_neighbors()
+        assert np.diff(h.connectivity()[0]).mean() >= 32
+        h.evaluateDerivatives()
+    batch = pkg.SPHBatch(together)
+    batch.build_neighbors()
+    batch.evaluateDerivatives()
+    for a, b in zip(alone, together):
+        for k in KEYS + ["new H"]:
+            assert np.array_equal(a.field(k), b.field(k)), k
+    for h in alone:
+        h.step(2)
+    batch.step(2)
+    for a, b in zip(alone, together):
+        for k in ("position", "velocity", "mass density", "specific thermal energy", "H"):
+            assert np.array_equal(a.field(k), b.field(k)), k
+
+
+@pytest.mark.parametrize("precision", ["PRECISION_FP64", "PRECISION_MIXED"])
+@pytest.mark.parametrize("options", [{}, {"XSPH": 1}, {"epsTensile": 0.3, "compatibleEnergyEvolution": 0},
+                                     {"balsaraShearCorrection": 1}])
+def test_rows_and_thread_kernels_give_the_same_bits(gpu_lib, pkg, precision, options):
+    """The same rows with a group of lanes per node (a set alone: rows of 32 entries
+    and more on average) and with a thread per node (the set with many isolated
+    nodes behind it, which shorten the mean row): derivatives and steps are the same
+    bits, summed density, compatible energy and update included."""
+    gen, abi = pkg.generators, pkg.abi
+    keep = 505
+    ns = gen.kelvin_helmholtz(nx=8, ny=8, nz=8, jitter=0.2, seed=2)
+    h = np.random.default_rng(4).uniform(0.13, 0.2, keep)
+    H = np.zeros((keep, 6))
+    H[:, [0, 3, 5]] = 1.0 / h[:, None]
+    dense = gen.NodeSet(ns.pos[:keep], ns.vel[:keep], ns.mass[:keep], ns.rho[:keep], ns.eps[:keep], H, ns.dx)
+    side = np.arange(22) + 2.0
+    far = np.stack(np.meshgrid(side, side, side), -1).reshape(-1, 3)
+    m = far.shape[0]
+
+    def joined(a, fill):
+        return np.concatenate([a, np.broadcast_to(fill, (m,) + a.shape[1:])])
+
+    both = gen.NodeSet(np.concatenate([dense.pos, far]), joined(dense.vel, 0.0), joined(dense.mass, dense.mass[0]),
+                       joined(dense.rho, 1.0), joined(dense.eps, 1.0), joined(dense.H, dense.H[0]), dense.dx)
+    cfg = gen.kh_config(abi, kernel=abi.KERNEL_BSPLINE, periodic=(0, 0, 0), precision=getattr(abi, precision),
+                        HUpdate=abi.H_INTEGRATE, dtMin=1.0e-4, dtMax=1.0e-4, **options)
+    rows, threads = pkg.SPHHydro(cfg, dense), pkg.SPHHydro(cfg, both)
+    for p, long in ((rows, True), (threads, False)):
+        p.build_neighbors()
+        entries = np.diff(p.connectivity()[0])
+        assert (entries.mean() >= 32) == long and entries[:keep].mean() >= 32 and not entries[keep:].any()
+        p.initialize()
+        p.evaluateDerivatives()
+    for k in KEYS + ["new H"]:
+        assert np.array_equal(rows.field(k), threads.field(k)[:keep]), k
+    for p in (rows, threads):
+        p.step(3)
+    for k in ("position", "velocity", "mass density", "specific thermal energy", "H"):
+        assert np.array_equal(rows.field(k), threads.field(k)[:keep]), k
