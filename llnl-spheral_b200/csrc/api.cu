@@ -356,6 +356,9 @@ bool isCrkP(const Problem& p) { return p.prm.hydro == SPHGPU_HYDRO_CRKSPH; }
 bool needsStartupVolume(const Problem& p) { return isCrkP(p) && !p.crkVolumeReady; }
 bool isMixedSph(const Problem& p) { return !isCrkP(p) && p.cfg.precision == SPHGPU_PRECISION_MIXED; }
 bool isMixedCrk(const Problem& p) { return isCrkP(p) && p.cfg.precision == SPHGPU_PRECISION_MIXED; }
+bool firstCellWalk(const Problem& p) {
+  return p.crowd < 0 && p.fillSchedule == NBR_SCHEDULE_WARP && p.grid.sub == 1;
+}
 bool hasGradh(const Problem& p) { return !isCrkP(p) && p.prm.gradh; }
 
 // CRKSPH volume (CRKSumVolume or mass/density) of the CRKSPH members;
@@ -616,7 +619,7 @@ int capture_full_step(Batch& b) {
   // everything the replay touches must exist before the capture
   if (anyMember(b, isCrkP)) SPH_TRY(crk_prepare(b));
   if (anyMember(b, isMixedSph) || anyMember(b, isMixedCrk)) SPH_TRY(prepare_mixed(b));
-  SPH_TRY(plan_build(b));
+  SPH_TRY(plan_build(b, true));
   SPH_TRY(enable_graph(b));
   SPH_TRY(upload_graph_descriptors(b));
   b.mapArenaPos = 0;
@@ -797,7 +800,8 @@ int steps_impl(Batch& b, int64_t nsteps) {
       }
       SPH_TRY(capture_full_step(b));
     }
-    const int64_t want = nsteps - done;
+    // (a first cell walk is replayed once, to learn of crowded cells)
+    const int64_t want = anyMember(b, firstCellWalk) ? 1 : nsteps - done;
     int64_t ran = 0;
     SPH_TRY(run_graph_steps(b, want, &ran));
     done += ran;

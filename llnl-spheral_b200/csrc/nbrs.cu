@@ -1461,15 +1461,15 @@ __global__ void __launch_bounds__(256) nbr_walk_kernel(const Member* mem, BlockM
 // along x, then y, then z, each element finding its rank by bisection in the
 // two other runs.
 //
-// Measured (B200): Sod 256x32x32 (262,144 nodes, 115 neighbors) 786 us against
-// 1,939 us with a warp per node; 24 tubes of the ensemble together 2.83 against
+// Measured (B200): Sod 256x32x32 (262,144 nodes, 115 neighbors) 680 us against
+// 1,939 us with a warp per node; 24 tubes of the ensemble together 2.81 against
 // 8.92 ms.  Bound by the latency of its steps between barriers (32 warps per
 // SM, about half of the cycles issue): the merges' bisections, then the tests
-// and the lists' stores.  With the bisections in the two other runs one after
-// the other and a warp per 32 elements of one run the merges took 23,000 of a
-// cell's 60,000 cycles, and the walk 786 us.  Loading the 27 cells ahead of
-// the first test: 786 us again (the registers spill); a list's places from a
-// scan of its words' counts instead of one after the other: 702 us.
+// and the lists' stores.  Other forms, against 699 us at the time: the bisections
+// in the two other runs one after the other and a warp per 32 elements of one
+// run, 786 (the merges took 23,000 of a cell's 60,000 cycles); the 27 cells'
+// loads ahead of the first test, 786 (the registers spill); a list's places from
+// a scan of its words' counts instead of one after the other, 702.
 constexpr int kCellThreads = 256;
 constexpr int kCellWarps = kCellThreads/32;
 constexpr int kCellCand = 1536;                        // nodes of the 27 cells that can be staged (more: crowded)
@@ -1885,7 +1885,8 @@ double reach_cells(const Problem& p) {
 }
 
 // Capacities for the next build, from the previous one (or first estimates).
-int plan_capacities(Batch& b) {
+// captured: for a graph that replays the build.
+int plan_capacities(Batch& b, bool captured = false) {
   for (Problem* pp : b.mem) {
     Problem& p = *pp;
     const int64_t oldg = p.gcap, oldc = p.candcap, olde = p.ecap, oldcells = p.cellcap;
@@ -1911,7 +1912,9 @@ int plan_capacities(Batch& b) {
     const int reqCells = p.nbrCells != 0 ? p.nbrCells : b.nbrCells;
     if (candPerNode < 0.8*p.denseSet) p.denseSet = 0.0;
     p.grid.sub = reqCells != 0 ? reqCells : (p.fillSchedule == NBR_SCHEDULE_WARP && p.denseSet > 0.0 ? 2 : 1);
-    p.grid.crowdList = p.crowd != 0 ? 1 : 0;
+    // (before the first cell walk an eager build lists what it finds; a captured
+    // one would launch the empty list in every replay: its first replay tells)
+    p.grid.crowdList = p.crowd > 0 || (p.crowd < 0 && !captured) ? 1 : 0;
     const int sub = p.grid.sub;
     // cells the grid wants at this subdivision (the last build's, rescaled), else the hint
     const int64_t cells = cells1 > 0.0 ? (int64_t)(cells1*sub*sub*sub) + 1 : p.hintCells;
@@ -2222,7 +2225,7 @@ int launch_build(Batch& b) {
 // The build's launches alone, for a CUDA-graph capture of the whole step:
 // capacities planned beforehand (plan_build), no read-back; a capacity
 // overflow sets the member's error flag on the device instead.
-int plan_build(Batch& b) { return plan_capacities(b); }
+int plan_build(Batch& b, bool captured) { return plan_capacities(b, captured); }
 int launch_build_captured(Batch& b) { return launch_build(b); }
 
 // After a build: whether the cell walk has met crowded cells, and whether they

@@ -142,10 +142,11 @@ enum RecField {
 // one.  A pair loop's lanes visit nodes that are mostly consecutive, so one
 // 32-byte load of a warp covers 8 to 12 cache lines; with whole records side
 // by side every lane's load is a line of its own (32 lines for each of the
-// ten 16-byte loads), and those line accesses bound the pair kernels.  Measured (B200, Kelvin-Helmholtz 128^3,
-// whole records -> planes): FP64 pair kernel 807 -> 688 us, summed density
-// 268 -> 184, mid-point update 229 -> 183; mixed 511 -> 488, 203 -> 137,
-// 195 -> 168; CRKSPH 1M volumes and density 202 -> 119.
+// ten 16-byte loads), and those line accesses bound the pair kernels.  Measured
+// (B200, Kelvin-Helmholtz 128^3, whole records / planes / paired planes, which
+// that size takes, see planeAt): FP64 pair kernel 807 / 688 / 724 us, summed
+// density 268 / 184 / 184, mid-point update 229 / 183 / 189; mixed 511 / 488 /
+// 521, 203 / 137 / 157, 195 / 168 / 171; CRKSPH 1M volumes and density 202 -> 119.
 struct D4 {
   double a, b, c, d;
 };
@@ -168,13 +169,12 @@ __device__ __forceinline__ void stPlane(double* p, double a, double b, double c,
 // has no locality every 32-byte piece fetched from HBM brings its 64-byte
 // neighborhood with it.  Measured (B200, Kelvin-Helmholtz in a random node order,
 // one step; whole records / planes / paired planes): 128^3 FP64 4.54 / 4.92 /
-// 4.46 ms, mixed 4.06 / 4.38 / 4.12; 112^3 2.88 / 2.97 / 2.76, 2.50 / 2.58 /
-// 2.48; 96^3 1.78 / 1.74 / 1.65, 1.56 / 1.54 / 1.50.  In lattice order a pair
-// covers twice the lines of a plane (128^3 FP64 pair kernel 687 -> 724 us, mixed
-// 510 -> 522, Sod 1,817 -> 1,860), so problems whose single planes are no slower
+// 4.44 ms, mixed 4.05 / 4.38 / 4.06; 112^3 2.88 / 2.97 / 2.76, 2.50 / 2.58 /
+// 2.47; 96^3 1.78 / 1.74 / 1.65, 1.56 / 1.54 / 1.50.  In lattice order a pair
+// covers twice the lines of a plane (the pair kernels above, Sod 2% more), so problems whose single planes are no slower
 // than whole records in either order keep them.  CRKSPH's longer records (PAIRED
 // false) gain from planes in either order (96^3 random 3.21 / 2.86 / 2.89 ms; 1M
-// in order, pair kernel 520 against 548 us).
+// in order, pair kernel 520 us against 548 paired).
 constexpr int64_t kPairedPlanes = 1900000;
 template<bool PAIRED = true>
 __host__ __device__ __forceinline__ int64_t planeAt(int64_t cap, int64_t k, int q) {
@@ -616,7 +616,7 @@ int batch_scan(Batch& b, int which);
 
 // ---- stages (ghosts/neighbors: nbrs.cu; SPH: sph.cu; mixed: sph_mixed.cu; CRKSPH: crk.cu)
 int build_connectivity(Batch& b);     // ghosts + ConnectivityMap, device-sized
-int plan_build(Batch& b);             // capacities and schedules of the next build
+int plan_build(Batch& b, bool captured = false);  // capacities and schedules of the next build
 void note_crowd(Problem& p, int64_t crowdedSlots);
 int launch_build_captured(Batch& b);  // the build's launches, sized on the device, no read-back
 // FP64 pair records of the members that read them next (PACK_ALL: every member)

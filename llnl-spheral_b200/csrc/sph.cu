@@ -430,8 +430,8 @@ __global__ void __launch_bounds__(128, SPH_FP64_MIN_BLOCKS) sph_eval_fp64_kernel
 // independent pairs, the entries and the stored pair accelerations are read
 // and written coalesced, and the sums take three registers a lane.  Lanes past
 // the end of a row add zeros, which leave every sum's bits (no sum is -0).
-// Measured (B200, Sod, 115 neighbors): 2,048 nodes 298 -> 31 us, 262,144 nodes
-// 1,977 -> 1,833 us; bound by L1 line accesses (63% of their rate) and the
+// Measured (B200, Sod, 115 neighbors; the thread-per-node kernel over whole
+// records -> this one): 2,048 nodes 297 -> 31 us, 262,144 nodes 1,973 -> 1,836 us; bound by L1 line accesses (63% of their rate) and the
 // latency of the divisions, the FP64 pipe 38% busy.
 constexpr int kRowLanes = 16;
 constexpr int kRowPad = kRowLanes + 1;
