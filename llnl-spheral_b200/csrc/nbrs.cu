@@ -1914,7 +1914,8 @@ int plan_capacities(Batch& b, bool captured = false) {
     p.grid.sub = reqCells != 0 ? reqCells : (p.fillSchedule == NBR_SCHEDULE_WARP && p.denseSet > 0.0 ? 2 : 1);
     // (before the first cell walk an eager build lists what it finds; a captured
     // one would launch the empty list in every replay: its first replay tells)
-    p.grid.crowdList = p.crowd > 0 || (p.crowd < 0 && !captured) ? 1 : 0;
+    const bool cellWalk = p.fillSchedule == NBR_SCHEDULE_WARP && p.grid.sub == 1;
+    p.grid.crowdList = cellWalk && (p.crowd > 0 || (p.crowd < 0 && !captured)) ? 1 : 0;
     const int sub = p.grid.sub;
     // cells the grid wants at this subdivision (the last build's, rescaled), else the hint
     const int64_t cells = cells1 > 0.0 ? (int64_t)(cells1*sub*sub*sub) + 1 : p.hintCells;

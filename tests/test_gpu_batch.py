@@ -306,3 +306,33 @@ def test_first_build_makes_no_block_map_ring(gpu_lib, pkg):
     batch, made = pinned(lambda: pkg.SPHBatch(mem))
     _, first = pinned(batch.build_neighbors)
     assert made >= 1 and first <= 2
+
+
+@pytest.mark.parametrize("kind", ["thread walk", "cell walk", "dense"])
+def test_runs_of_new_states_replay_the_captured_step(gpu_lib, pkg, kind):
+    """A program that runs state after state in one problem (new state, build, steps)
+    replays the step it has captured: no eager step from the third run on.  (Eager
+    steps gather the sizes of their build and the dt, four launches that a replay
+    has not.)"""
+    gen, abi = pkg.generators, pkg.abi
+    if kind == "cell walk":
+        box = ((0.0, 0.0, 0.0), (1.0, 0.25, 0.25))
+        ns, cfg = gen.sod(nx=32, ny=8, nz=8, box=box), gen.sod_config(abi, ns_box=box)
+    else:
+        nPerh = 1.35 if kind == "thread walk" else 3.0
+        kernel = abi.KERNEL_WENDLANDC4 if kind == "thread walk" else abi.KERNEL_BSPLINE
+        ns = gen.kelvin_helmholtz(nx=14, ny=14, nz=14, nPerh=nPerh, jitter=0.05)
+        cfg = gen.kh_config(abi, kernel=kernel, nPerh=nPerh, max_neighbors=2048, dtMin=1.0e-5, dtMax=1.0e-5)
+    g = pkg.SPHHydro(cfg, ns)
+    launches = []
+    for _ in range(6):
+        g.set_state(ns)
+        g.build_neighbors()
+        g.initialize()
+        g.evaluateDerivatives()
+        before = g.kernel_launches()
+        g.step(3)
+        first = g.kernel_launches() - before
+        g.step(3)
+        launches.append((first, g.kernel_launches() - before - first))
+    assert all(a == b == launches[-1][1] for a, b in launches[3:]), launches
