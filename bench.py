@@ -89,13 +89,13 @@ def eval_alg_bytes_mixed(nodes, ghosts, entries):
     return nodes * 136 + 2 * (nodes + ghosts) * 112 + nodes * 432 + 16 * entries
 
 
-# DRAM traffic (read + write) measured by ncu on Kelvin-Helmholtz 96^3
-# (884,736 nodes, 56,456 ghosts, 5,363,712 entries) for the record pack and
-# the pair kernel of each form; scaled to other sizes by the algorithmic
-# bytes (all three units grow together).
-EVAL_TRAFFIC_96 = {"fp64": 155681536 + 107269376 + 180020480 + 449962752,
-                   "mixed": 150498816 + 67565056 + 190594816 + 386470912}
-EVAL_UNITS_96 = (884736, 56456, 5363712)
+# DRAM traffic (read + write) measured by ncu on Kelvin-Helmholtz 112^3
+# (1,404,928 nodes, 76,616 ghosts, 8,429,568 entries), which has the record
+# layout of 128^3, for the record pack and the pair kernel of each form; scaled
+# to other sizes by the algorithmic bytes (all three units grow together).
+EVAL_TRAFFIC_112 = {"fp64": 245091584 + 204587008 + 313802752 + 784777984,
+                    "mixed": 243307008 + 137284608 + 302858240 + 648876800}
+EVAL_UNITS_112 = (1404928, 76616, 8429568)
 
 
 def kh_problem(pkg, nx, nz=None, seed=20261203):
@@ -643,7 +643,7 @@ def time_batch(pkg, probs, steps, warmup, world, graph):
     batch.close()
     return {"value": pairs / t, "unit": METRIC, "ms_per_step": 1e3 * t / steps,
             "kernel_launches_per_step": launches / steps, "step_graph": bool(graph),
-            "autotuned": {"neighbor walk": ["auto", "thread per node", "warp per node"][tune["neighbor walk"]],
+            "autotuned": {"neighbor walk": ["auto", "thread per node", "block per cell or warp per node"][tune["neighbor walk"]],
                           "neighbor cells per kernel reach": tune["neighbor cells"],
                           "pair loop threads": tune["pair loop"]}}
 
@@ -940,14 +940,14 @@ def run_ours(args):
 
     def roofline(form, alg, t_eval, kernel):
         achieved = alg / (t_eval / 1e3) / 1e9
-        measured = EVAL_TRAFFIC_96[form]
-        units96 = eval_alg_bytes_fp64(*EVAL_UNITS_96) if form == "fp64" else eval_alg_bytes_mixed(*EVAL_UNITS_96)
+        measured = EVAL_TRAFFIC_112[form]
+        units112 = eval_alg_bytes_fp64(*EVAL_UNITS_112) if form == "fp64" else eval_alg_bytes_mixed(*EVAL_UNITS_112)
         return {"bound": "hbm", "kernel": kernel, "achieved": achieved, "peak": peak,
                 "peak_kind": peak_kind + " (MEASURED_PEAKS hbm_gbs)" if peak_kind == "measured" else peak_kind,
                 "unit": "GB/s", "frac": achieved / peak,
-                "traffic": None if measured is None else measured * alg / units96,
+                "traffic": None if measured is None else measured * alg / units112,
                 "traffic_source": None if measured is None else
-                "ncu dram__bytes_read.sum + dram__bytes_write.sum of the two kernels on Kelvin-Helmholtz 96^3, "
+                "ncu dram__bytes_read.sum + dram__bytes_write.sum of the two kernels on Kelvin-Helmholtz 112^3, "
                 "scaled by the algorithmic bytes",
                 "algorithmic_bytes": alg, "eval_ms": t_eval}
 

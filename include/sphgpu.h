@@ -333,7 +333,8 @@ int sphgpu_kernel_launches(sphgpu_problem* p, int64_t* launches);
  * four launches and a prefix sum per pass, 2 = all six passes in one
  * cooperative launch with grid barriers.  Same ghosts in the same order
  * either way.
- * sphgpu_get_schedule reports what the last call used. */
+ * sphgpu_get_schedule reports what the last call used (stage "ghost passes": 2
+ * for the cluster launch, too). */
 int sphgpu_set_schedule(sphgpu_problem* p, const char* stage, int32_t schedule);
 int sphgpu_get_schedule(sphgpu_problem* p, const char* stage, int32_t* schedule);
 /* Autotuner: times every schedule of the neighbor walk (thread per node, or 2

@@ -897,7 +897,7 @@ int set_schedule_impl(Batch& b, int* nbrSchedule, int* nbrCells, const char* sta
   }
   if (std::strcmp(stage, "neighbor walk") == 0) {
     if (schedule < NBR_SCHEDULE_AUTO || schedule > NBR_SCHEDULE_WARP) {
-      set_error("neighbor walk schedule must be 0 (auto), 1 (thread per node) or 2 (warp per node)");
+      set_error("neighbor walk schedule must be 0 (auto), 1 (thread per node) or 2 (block per cell, or warp per node)");
       return SPHGPU_ERR_ARG;
     }
     *nbrSchedule = schedule;
@@ -951,7 +951,7 @@ int set_schedule_impl(Batch& b, int* nbrSchedule, int* nbrCells, const char* sta
 // data and timed with CUDA events on the batch stream (one warm run, then the
 // median of three); the fastest is kept.  All schedules give bit-identical
 // results, so tuning changes speed only.  report = {neighbor schedule,
-// ms thread, ms warp, pair-loop threads, ms 64, ms 128, cells per kernel
+// ms of schedule 1, of schedule 2, pair-loop threads, ms 64, ms 128, cells per kernel
 // reach, ms with half-reach cells}.
 int autotune_impl(Batch& b, double* report) {
   cudaEvent_t e0 = nullptr, e1 = nullptr;
@@ -976,7 +976,7 @@ int autotune_impl(Batch& b, double* report) {
   double out[8] = {0, 0, 0, 0, 0, 0, 0, 0};
   int rc = SPHGPU_OK;
   do {
-    // neighbor walk: thread per node vs warp per node
+    // neighbor walk: thread per node vs the cell walk
     const int schedules[2] = {NBR_SCHEDULE_THREAD, NBR_SCHEDULE_WARP};
     double best = 1e300;
     int bestS = NBR_SCHEDULE_AUTO;
