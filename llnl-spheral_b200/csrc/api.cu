@@ -765,6 +765,7 @@ int run_graph_steps(Batch& b, int64_t count, int64_t* done) {
     p.pairs = asI64(a[7]);
     p.ncells = asI64(r2[4*m]);
     p.cellsWanted = asI64(r2[4*m + 1]);
+    p.lastNbrCells = p.grid.sub;           // (the captured plan's: it may have changed them)
     p.pairsEvaluated += asI64(r2[4*m + 2]);
     note_crowd(p, asI64(r2[4*m + 3]));
     if (herr & (DERR_GHOST_CAPACITY | DERR_ENTRY_CAPACITY | DERR_LIST_CAPACITY | DERR_NBR_CAPACITY)) overflow = true;

@@ -228,3 +228,28 @@ def test_full_windows(gpu_lib, pkg, oracle_mod, per_cell, branch, passes, period
     for _ in range(2):
         g.build_neighbors()
         _same_connectivity(g, o)
+
+
+# (h 0.22: 85 nodes per cell, windows of 2,300)
+@pytest.mark.parametrize("clump,h", [(300, 0.08), (0, 0.22)])
+def test_crowded_cells_in_captured_steps(gpu_lib, pkg, clump, h):
+    """Steps straight from a new state, whose first cell walk is in a captured step:
+    a clump (the list joins the second capture) and a set that is crowded all over
+    (half-reach cells from then on) take the states of eager steps."""
+    gen, abi = pkg.generators, pkg.abi
+    ns, _ = _clump(pkg, clump, 5, (1, 1, 1), False)
+    ns.H[:, [0, 3, 5]] = 1.0 / h
+    ns.pos[:] += np.random.default_rng(9).uniform(-1.0e-3, 1.0e-3, ns.pos.shape)
+    cfg = gen.kh_config(abi, kernel=abi.KERNEL_BSPLINE, max_neighbors=2048, HUpdate=abi.H_INTEGRATE,
+                        dtMin=1.0e-6, dtMax=1.0e-6)
+    out = []
+    for graph in (0, 1):
+        g = pkg.SPHHydro(cfg, ns)
+        g.set_schedule("neighbor walk", 0 if clump == 0 else 2)
+        g.set_schedule("step graph", graph)
+        g.step(9)
+        out.append(g)
+    assert out[0].schedule("neighbor cells") == out[1].schedule("neighbor cells") == (2 if clump == 0 else 1)
+    assert np.array_equal(out[0].connectivity()[1], out[1].connectivity()[1])
+    for k in ("position", "velocity", "mass density", "specific thermal energy", "H"):
+        assert np.array_equal(out[0].field(k), out[1].field(k)), k
